@@ -244,8 +244,9 @@ int hs2_altcorr_forward_packed(const void* packed1, const void* packed2, int dty
  *   -> fmap1_grad [b,n1,c,h,w], fmap2_grad [b,n2,c,h2,w2] of `dtype`, fully written.
  *   `scale` multiplies every product: 1 reproduces the reference operator (which
  *   leaves out the forward's 1/16), 1/16 gives the exact adjoint of the forward.
- *   workspace: f32 accumulators, hs2_altcorr_backward_workspace_size() bytes
- *   (0 when dtype is f32).
+ *   workspace: hs2_altcorr_backward_workspace_size() bytes (channel-last f32 features and
+ *   accumulators of the tiled kernel for c == 128).  With fewer bytes, down to the f32
+ *   accumulators alone (none when dtype is f32), the pixel-by-pixel kernel runs instead.
  */
 int hs2_altcorr_backward_workspace_size(int dtype, int b, int n1, int n2, int c, int h, int w, int h2,
                                         int w2, size_t* bytes);
