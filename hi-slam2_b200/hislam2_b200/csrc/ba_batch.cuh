@@ -3,22 +3,23 @@
 // iteration.  Included at the end of ba.cu: the work units run the same device
 // bodies as the single-window kernels.
 //
-// Work units, handed out phase-major by an atomic counter (every unit of phase k of
-// every window before any unit of phase k+1):
+// Work units, handed out in a fixed order by an atomic counter (a window's phases in
+// order; see batch_plan for the interleaving of the windows):
 //   0  edge table (ba_edge_setup) in 256-edge-thread units, + one unit zeroing the
 //      window's per-edge sums and FP64 system;
 //   1  linearisation, one unit per (depth frame, 1024 pixels) (ba_linearize body,
 //      256 threads);
 //   2  assembly (256 edge threads per unit) and the SIMT Schur Gram, one unit per
-//      (depth frame, pixel split) (ba_schur body);
+//      (depth frame, pixel split) (batch_gram, or the ba_schur body for frames of more
+//      than kGramRows rows);
 //   3  the damped FP64 Cholesky solve of the window's reduced system, one unit
 //      (single CTA: 32-column panels in shared memory for systems up to 256 wide,
 //      column by column in global memory above that, up to 6 * kBatchMaxPoses);
 //   4  back-substitution per (depth frame, 1024 pixels) and the pose retraction.
 // A unit of phase k > 0 waits (acquire, bounded) until the window's phase k-1
 // counter reaches its unit count; units count themselves done with a release add.
-// Every unit of an earlier phase was handed to a resident CTA before the wait
-// begins (cooperative launch: all CTAs co-resident), so no wait can cycle.  A wait
+// Every unit of its window's earlier phases was handed to a resident CTA before the
+// wait begins (cooperative launch: all CTAs co-resident), so no wait can cycle.  A wait
 // that runs out sets HS2_DEV_TIMEOUT in the window's info and the launch drains.
 // The keys (depth slots, edge groups, E-row lists) do not change between
 // iterations and are built once by hs2_ba_batch_prepare.
@@ -57,8 +58,12 @@ struct BatchWin {
 struct BatchHdr {
   int nwin;
   int total;                          // units of all phases
-  int cum[kBatchPhases + 1];          // first unit of each phase
   int grid;                           // CTAs of the persistent launch
+};
+
+// One run of consecutive units: phase `phase` of window `win`, units start ..
+struct BatchSeg {
+  int start, phase, win;
 };
 
 // Damped FP64 Cholesky of the lower triangle of A (n x n, row-major) and the solve
@@ -258,6 +263,181 @@ __device__ void batch_cholesky_blocked(int n, float lm, float ep, BaPtrs w, floa
   }
 }
 
+// Schur Gram of one (depth frame s, pixel split) for the small frames of a batch: FP32,
+// S = (Q F) F^T and v = (Q F) w over the frame's 6 nr rows, with w appended as one more row.
+// Stages of 32 to 128 pixels (more for smaller frames, whose tiles are few: the pixels then
+// occupy the threads) arrive by cp.async, as many in flight as fit; rows end in four spare
+// floats, so the 16-byte reads of eight neighbouring rows hit different banks.  With nb = rows / 8,
+// a thread owns the 64 products of rows {bi + nb k} and {bj + nb l}, bi <= bj: every
+// unordered pair of rows falls in exactly one such tile, neighbouring threads read
+// neighbouring rows, and 16 row reads feed 256 FMAs.  The CTA's threads are split over
+// tiles and pixel slices; the slices are summed in shared memory, so one FP64 atomic per
+// entry leaves the CTA.
+// The general ba_schur body (22-block tiles, one thread per 6x6 block) leaves two thirds
+// of a CTA idle on frames of 5 to 14 blocks, stages 132 rows whatever the frame holds and
+// waits for every stage: 420 us per unit against 55 to 70 us here (64 windows of 8 to 40
+// keyframes, two units per frame, two CTAs per SM; one LM iteration 6.4 ms against 2.26 ms).
+constexpr int kGramRows = 256;        // rows with w's: 42 blocks
+constexpr int kGramTiles = (kGramRows / 8) * (kGramRows / 8 + 1) / 2;
+constexpr int kGramStages = 4;
+
+__device__ __forceinline__ void cp_async4_zfill(uint32_t dst, const void* src, uint32_t bytes) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+
+__device__ void batch_gram(int s, int split, int HW, int chunk, const BaPtrs& w, int P, const int32_t* __restrict__ info,
+                           float* __restrict__ sm) {
+  if (info[0] || s >= info[1]) return;
+  const int nr = w.sptr[s + 1] - w.sptr[s];
+  if (nr == 0) return;
+  const int nd = 6 * nr, rows = nd + 1;
+  if (rows > kGramRows) {
+    ba_schur_body(s, split, HW, chunk, w, P, 1, 0, info);
+    return;
+  }
+  const int c0 = split * chunk, c1 = min(HW, c0 + chunk);
+  if (c0 >= c1) return;
+  __shared__ uint16_t tile_of[kGramTiles];   // bi << 8 | bj
+  const int tid = threadIdx.x;
+  const int nb = (rows + 7) >> 3, ntile = nb * (nb + 1) / 2;
+  // pixels per stage (a power of two), floats per staged row
+  const int sh = rows <= 32 ? 7 : rows <= 96 ? 6 : 5, TP = 1 << sh, ld = TP + 4;
+  const int slices = min(TP / 4, max(1, kBatchThreads / ntile));
+  // a stage: 8 nb rows (rows.. stay zero), then Q
+  const int stage = (8 * nb + 1) * ld;
+  const int nst = min(kGramStages, (int)(kBatchDynSmem / sizeof(float)) / stage);
+  const int nchunk = (c1 - c0 + TP - 1) / TP;
+  const int HWs = row_stride(HW);
+  const float* Er = w.erows + (int64_t)w.rptr[s] * 6 * HWs;
+  const float* Q = w.qbuf + (int64_t)s * HW;
+  const float* W = w.wbuf + (int64_t)s * HW;
+  const int* spose = w.spose + w.sptr[s];
+  const int64_t n = 6 * (int64_t)P;
+  const uint32_t smb = smem_u32(sm);
+  auto load = [&](int c) {
+    if (c < nchunk) {
+      const uint32_t dst = smb + (uint32_t)(c % nst) * stage * 4u;
+      const int p0 = c0 + c * TP;
+      for (int idx = tid; idx < nd * (TP / 4); idx += kBatchThreads) {
+        const int r = idx >> (sh - 2), q = (idx & (TP / 4 - 1)) * 4;
+        const int live = min(4, max(0, c1 - p0 - q));
+        cp_async16(dst + (uint32_t)(r * ld + q) * 4u, Er + (int64_t)r * HWs + p0 + (live ? q : 0), 4u * live);
+      }
+      if (tid < 2 * TP) {
+        const int q = tid & (TP - 1), p = p0 + q;
+        const float* src = (tid < TP ? W : Q) + min(p, c1 - 1);
+        cp_async4_zfill(dst + (uint32_t)((tid < TP ? nd : 8 * nb) * ld + q) * 4u, src, p < c1 ? 4u : 0u);
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  for (int t0 = 0; t0 < ntile; t0 += kBatchThreads) {
+    const int nt = min(kBatchThreads, ntile - t0);
+    const int t = tid % nt, slice = tid / nt;
+    const bool live = slice < slices;
+    __syncthreads();                          // the previous round's (or unit's) readers of sm
+    if (t0 == 0)
+      for (int bi = tid; bi < nb; bi += kBatchThreads)
+        for (int bj = bi, at = bi * nb - bi * (bi - 1) / 2; bj < nb; ++bj, ++at) tile_of[at] = (uint16_t)(bi << 8 | bj);
+    for (int idx = tid; idx < nst * (8 * nb - rows) * ld; idx += kBatchThreads) {   // padding rows
+      const int st = idx / ((8 * nb - rows) * ld);
+      sm[st * stage + rows * ld + idx - st * (8 * nb - rows) * ld] = 0.f;
+    }
+    for (int c = 0; c < nst - 1; ++c) load(c);
+    __syncthreads();
+    const int bi = tile_of[t0 + t] >> 8, bj = tile_of[t0 + t] & 255;
+    float acc[8][8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+#pragma unroll
+      for (int l = 0; l < 8; ++l) acc[k][l] = 0.f;
+    for (int c = 0; c < nchunk; ++c) {
+      if (nst == 1) load(c);
+      else load(c + nst - 1);                 // the stage its last readers left at the end of pass c - 1
+      if (nst >= 4) asm volatile("cp.async.wait_group 3;" ::: "memory");
+      else if (nst == 3) asm volatile("cp.async.wait_group 2;" ::: "memory");
+      else if (nst == 2) asm volatile("cp.async.wait_group 1;" ::: "memory");
+      else asm volatile("cp.async.wait_group 0;" ::: "memory");
+      __syncthreads();
+      if (live) {
+        const float* st = sm + (c % nst) * stage;
+        for (int q = slice; q < TP / 4; q += slices) {
+          const float4* a = reinterpret_cast<const float4*>(st + bi * ld) + q;
+          const float4* b = reinterpret_cast<const float4*>(st + bj * ld) + q;
+          const float4 qv = *(reinterpret_cast<const float4*>(st + 8 * nb * ld) + q);
+          float4 bv[8];
+#pragma unroll
+          for (int l = 0; l < 8; ++l) bv[l] = b[l * nb * (ld / 4)];
+#pragma unroll
+          for (int k = 0; k < 8; ++k) {
+            float4 av = a[k * nb * (ld / 4)];
+            av.x *= qv.x;
+            av.y *= qv.y;
+            av.z *= qv.z;
+            av.w *= qv.w;
+#pragma unroll
+            for (int l = 0; l < 8; ++l) {
+              acc[k][l] = fmaf(av.x, bv[l].x, acc[k][l]);
+              acc[k][l] = fmaf(av.y, bv[l].y, acc[k][l]);
+              acc[k][l] = fmaf(av.z, bv[l].z, acc[k][l]);
+              acc[k][l] = fmaf(av.w, bv[l].w, acc[k][l]);
+            }
+          }
+        }
+      }
+      __syncthreads();
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    // sum of the slices, the upper half onto the lower half (entry-major: neighbouring threads
+    // hit neighbouring banks)
+    for (int left = slices; left > 1;) {
+      const int h = (left + 1) >> 1;
+      __syncthreads();
+      if (slice >= h && slice < left) {
+#pragma unroll
+        for (int k = 0; k < 64; ++k) sm[k * h * nt + tid - h * nt] = acc[k >> 3][k & 7];
+      }
+      __syncthreads();
+      if (slice < left - h) {
+#pragma unroll
+        for (int k = 0; k < 64; ++k) acc[k >> 3][k & 7] += sm[k * h * nt + tid];
+      }
+      left = h;
+    }
+    __syncthreads();
+    if (slice == 0) {
+#pragma unroll
+      for (int k = 0; k < 64; ++k) sm[k * nt + t] = acc[k >> 3][k & 7];
+    }
+    __syncthreads();
+    for (int idx = tid; idx < 64 * nt; idx += kBatchThreads) {
+      const int kl = idx / nt, tt = idx - kl * nt;
+      const int ti = tile_of[t0 + tt] >> 8, tj = tile_of[t0 + tt] & 255;
+      int r = ti + nb * (kl >> 3), c = tj + nb * (kl & 7);
+      if (r >= rows || c >= rows || (ti == tj && r > c)) continue;
+      if (r > c) {
+        const int x = r;
+        r = c;
+        c = x;
+      }
+      if (r == nd) continue;                  // w . w
+      const double v = -(double)sm[idx];
+      const int a = r / 6, x = r - 6 * a, pa = spose[a];
+      if (c == nd) {
+        atomicAdd(&w.b[pa * 6 + x], v);
+        continue;
+      }
+      const int b = c / 6, y = c - 6 * b, pb = spose[b];
+      if (pa > pb) atomicAdd(&w.A[(pa * 6 + x) * n + pb * 6 + y], v);
+      else if (pa < pb) atomicAdd(&w.A[(pb * 6 + y) * n + pa * 6 + x], v);
+      else {
+        atomicAdd(&w.A[(pa * 6 + x) * n + pa * 6 + y], v);
+        if (r != c) atomicAdd(&w.A[(pa * 6 + y) * n + pa * 6 + x], v);
+      }
+    }
+  }
+}
+
 __device__ void batch_unit(const BatchWin& W, int ph, int idx, float lm, float ep, double* pv) {
   const int tid = threadIdx.x;
   const BaPtrs& w = W.w;
@@ -282,7 +462,7 @@ __device__ void batch_unit(const BatchWin& W, int ph, int idx, float lm, float e
         ba_assemble_body(idx * kBatchThreads + tid, W.ii, W.jj, (int)W.E, W.t0, W.P, w, W.info);
       } else {
         const int g = idx - W.nasm;
-        ba_schur_body(g / W.gsplit, g % W.gsplit, W.HW, W.gchunk, w, W.P, 1, 0, W.info);
+        batch_gram(g / W.gsplit, g % W.gsplit, W.HW, W.gchunk, w, W.P, W.info, reinterpret_cast<float*>(pv));
       }
       break;
     case 3:
@@ -303,7 +483,7 @@ __device__ void batch_unit(const BatchWin& W, int ph, int idx, float lm, float e
 }
 
 __global__ void __launch_bounds__(kBatchThreads, 2)
-ba_batch_kernel(const BatchHdr* __restrict__ hdr, const BatchWin* __restrict__ wins, const int* __restrict__ prefix,
+ba_batch_kernel(const BatchHdr* __restrict__ hdr, const BatchWin* __restrict__ wins, const BatchSeg* __restrict__ segs,
                 unsigned* __restrict__ done, unsigned* __restrict__ next, int* __restrict__ abort_flag, float lm,
                 float ep) {
   __shared__ int s_u, s_ph, s_w, s_idx, s_go;
@@ -314,24 +494,21 @@ ba_batch_kernel(const BatchHdr* __restrict__ hdr, const BatchWin* __restrict__ w
       const int u = (int)atomicAdd(next, 1u);
       s_u = u;
       if (u < total) {
-        int ph = 0;
-        while (u >= hdr->cum[ph + 1]) ++ph;
-        const int local = u - hdr->cum[ph];
-        const int* pre = prefix + ph * (nwin + 1);
-        int lo = 0, hi = nwin - 1;          // last window with pre[w] <= local
+        int lo = 0, hi = kBatchPhases * nwin - 1;   // last segment that starts at or before u
         while (lo < hi) {
           const int mid = (lo + hi + 1) >> 1;
-          if (pre[mid] <= local) lo = mid;
+          if (segs[mid].start <= u) lo = mid;
           else hi = mid - 1;
         }
+        const int ph = segs[lo].phase, win = segs[lo].win;
         s_ph = ph;
-        s_w = lo;
-        s_idx = local - pre[lo];
+        s_w = win;
+        s_idx = u - segs[lo].start;
         int go = 1;
         if (ph > 0) {
-          const unsigned need = (unsigned)wins[lo].units[ph - 1] + g_batch_unsatisfiable;
+          const unsigned need = (unsigned)wins[win].units[ph - 1] + g_batch_unsatisfiable;
           const unsigned limit = g_batch_spin;
-          const unsigned* c = done + lo * kBatchPhases + ph - 1;
+          const unsigned* c = done + win * kBatchPhases + ph - 1;
           unsigned i = 0;
           while (ld_acquire_gpu(c) < need) {
             if (++i > limit || *(volatile int*)abort_flag) {
@@ -368,8 +545,8 @@ __global__ void ba_batch_flag_kernel(const BatchWin* __restrict__ wins, int nwin
 struct BatchPlanHost {
   BatchHdr hdr;
   std::vector<BatchWin> wins;
-  std::vector<int> prefix;
-  size_t off_hdr, off_wins, off_prefix, off_ctl, ctl_bytes, off_ws, total;
+  std::vector<BatchSeg> segs;
+  size_t off_hdr, off_wins, off_segs, off_ctl, ctl_bytes, total;
   std::vector<size_t> ws_off;
 };
 
@@ -388,7 +565,7 @@ static int batch_plan(const hs2_ba_window* in, int nwin, int gsplit, BatchPlanHo
   auto take = [&](size_t bytes) { size_t at = o; o = align256(o + bytes); return at; };
   pl.off_hdr = take(sizeof(BatchHdr));
   pl.off_wins = take(sizeof(BatchWin) * nwin);
-  pl.off_prefix = take(sizeof(int) * kBatchPhases * (nwin + 1));
+  pl.off_segs = take(sizeof(BatchSeg) * kBatchPhases * nwin);
   pl.ctl_bytes = sizeof(unsigned) * (kBatchPhases * (size_t)nwin + 2);
   pl.off_ctl = take(pl.ctl_bytes);
   for (int k = 0; k < nwin; ++k) {
@@ -444,21 +621,35 @@ static int batch_plan(const hs2_ba_window* in, int nwin, int gsplit, BatchPlanHo
     W.units[3] = 1;
     W.units[4] = W.nback + 1;
   }
-  pl.off_ws = pl.ws_off.empty() ? o : pl.ws_off[0];
   pl.total = o;
-  pl.prefix.assign(kBatchPhases * (nwin + 1), 0);
-  pl.hdr.nwin = nwin;
-  pl.hdr.cum[0] = 0;
-  for (int ph = 0; ph < kBatchPhases; ++ph) {
-    int acc = 0;
-    for (int k = 0; k < nwin; ++k) {
-      pl.prefix[ph * (nwin + 1) + k] = acc;
-      acc += pl.wins[k].units[ph];
-    }
-    pl.prefix[ph * (nwin + 1) + nwin] = acc;
-    pl.hdr.cum[ph + 1] = pl.hdr.cum[ph] + acc;
+  // Order of the units.  Windows go by falling number of poses, phases 0 and 1 of all of
+  // them first.  A window's solve is one unit on one CTA and its length grows with the cube
+  // of the poses, so it follows its Gram as soon as one grid of later units lies between
+  // them (by then the Gram's units are done or nearly so): the long solves run under the
+  // other windows' Grams.  64 windows: 2.70 ms per iteration with every phase of all
+  // windows before the next phase, 2.24 ms so.
+  std::vector<int> order(nwin);
+  for (int k = 0; k < nwin; ++k) order[k] = k;
+  std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return pl.wins[a].P > pl.wins[b].P; });
+  pl.segs.clear();
+  int at = 0;
+  auto put = [&](int ph, int k) {
+    pl.segs.push_back(BatchSeg{at, ph, k});
+    at += pl.wins[k].units[ph];
+  };
+  for (int ph = 0; ph < 2; ++ph)
+    for (int k : order) put(ph, k);
+  std::vector<int> end(nwin);
+  int solved = 0;
+  for (int i = 0; i < nwin; ++i) {
+    put(2, order[i]);
+    end[i] = at;
+    for (; solved < i && at - end[solved] >= 2 * kNumSMs; ++solved) put(3, order[solved]);
   }
-  pl.hdr.total = pl.hdr.cum[kBatchPhases];
+  for (; solved < nwin; ++solved) put(3, order[solved]);
+  for (int k : order) put(4, k);
+  pl.hdr.nwin = nwin;
+  pl.hdr.total = at;
   return HS2_OK;
 }
 
@@ -511,7 +702,7 @@ extern "C" int hs2_ba_batch_prepare(const hs2_ba_window* windows, int num_window
   HS2_CUDA(cudaMemcpyAsync(base + pl.off_hdr, &pl.hdr, sizeof(BatchHdr), cudaMemcpyHostToDevice, s));
   HS2_CUDA(cudaMemcpyAsync(base + pl.off_wins, pl.wins.data(), sizeof(BatchWin) * num_windows,
                            cudaMemcpyHostToDevice, s));
-  HS2_CUDA(cudaMemcpyAsync(base + pl.off_prefix, pl.prefix.data(), sizeof(int) * pl.prefix.size(),
+  HS2_CUDA(cudaMemcpyAsync(base + pl.off_segs, pl.segs.data(), sizeof(BatchSeg) * pl.segs.size(),
                            cudaMemcpyHostToDevice, s));
   for (int k = 0; k < num_windows; ++k) {
     const hs2_ba_window& a = windows[k];
@@ -542,12 +733,12 @@ extern "C" int hs2_ba_batch_run(void* workspace, int num_windows, int grid, int 
   auto take = [&](size_t bytes) { size_t at = o; o = align256(o + bytes); return at; };
   const size_t off_hdr = take(sizeof(BatchHdr));
   const size_t off_wins = take(sizeof(BatchWin) * nwin);
-  const size_t off_prefix = take(sizeof(int) * kBatchPhases * (nwin + 1));
+  const size_t off_segs = take(sizeof(BatchSeg) * kBatchPhases * nwin);
   const size_t ctl_bytes = sizeof(unsigned) * (kBatchPhases * (size_t)nwin + 2);
   const size_t off_ctl = take(ctl_bytes);
   const BatchHdr* dh = reinterpret_cast<const BatchHdr*>(base + off_hdr);
   const BatchWin* dw = reinterpret_cast<const BatchWin*>(base + off_wins);
-  const int* dp = reinterpret_cast<const int*>(base + off_prefix);
+  const BatchSeg* dp = reinterpret_cast<const BatchSeg*>(base + off_segs);
   unsigned* done = reinterpret_cast<unsigned*>(base + off_ctl);
   unsigned* next = done + kBatchPhases * nwin;
   int* abort_flag = reinterpret_cast<int*>(next + 1);
