@@ -31,6 +31,7 @@ SIGNATURES = {
     "hs2_version": [],
     "hs2_frame_distance": [_p, _i64, _p, _i64, _i32, _i32, _p, _p, _p, _i64, _f32, _p, _p, _p],
     "hs2_corr_index_forward": [_p, _i32, _i64, _i32, _i32, _i32, _i32, _p, _i32, _p, _p],
+    "hs2_corr_pyramid_forward": [_p, _i32, _i32, _i64, _i32, _i32, _p, _i32, _p, _p],
     "hs2_corr_index_backward": [_p, _p, _i32, _i64, _i32, _i32, _i32, _i32, _i32, _p, _p],
     "hs2_corr_volume_workspace_size": [_i64, _i64, _i32, _i32, _i32, _i32, _i32, ctypes.POINTER(_sz)],
     "hs2_corr_volume": [_p, _i64, _p, _i64, _i32, _i32, _i32, _i32, _p, _p, _i64, _i32, _i32, _p, _p, _p, _sz,

@@ -557,6 +557,34 @@ def corr_index_forward(volume, coords, radius):
     return [corr]
 
 
+def corr_pyramid_fits(volumes, coords, radius):
+    """Whether :func:`corr_pyramid_forward` takes these levels (else one corr_index_forward per level)."""
+    if radius not in (3, 4) or not 1 <= len(volumes) <= 4 or coords.dim() != 4 or coords.dtype != torch.float32 \
+            or not coords.is_cuda:
+        return False
+    n, h, w, two = coords.shape
+    v0 = volumes[0]
+    return two == 2 and 0 < n <= 65535 and v0.dtype in (torch.float32, torch.float16, torch.bfloat16) \
+        and all(v.dtype == v0.dtype and v.device == coords.device and v.is_contiguous()
+                and tuple(v.shape) == (n, h, w, h >> l, w >> l) and v.numel() for l, v in enumerate(volumes))
+
+
+def corr_pyramid_forward(volumes, coords, radius):
+    """``corr_index_forward`` of every pyramid level at ``coords / 2^level``, concatenated.
+
+    ``volumes[l]`` [N,H,W,H>>l,W>>l], ``coords`` [N,H,W,2] contiguous; returns [N, L*(2r+1)^2, H, W].
+    For inputs that pass :func:`corr_pyramid_fits`.
+    """
+    _contig("coords", coords)
+    n, h, w, _ = coords.shape
+    L, r, dev = len(volumes), int(radius), coords.device
+    corr = torch.empty(n, L * (2 * r + 1) ** 2, h, w, dtype=volumes[0].dtype, device=dev)
+    ptrs = (ctypes.c_void_p * 4)(*[v.data_ptr() for v in volumes])
+    _lib.check(_lib.load().hs2_corr_pyramid_forward(ptrs, L, _DTYPES[volumes[0].dtype], n, h, w, _ptr(coords), r,
+                                                    _ptr(corr), _stream(dev)), "corr_pyramid_forward")
+    return corr
+
+
 def corr_index_backward(volume, coords, corr_grad, radius):
     """``droid_backends.corr_index_backward`` (reference ``src/droid.cpp:266-275``) -> [volume_grad]."""
     _contig("volume", volume)

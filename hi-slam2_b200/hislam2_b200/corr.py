@@ -8,7 +8,8 @@
 * :class:`AltCorrBlock` keeps ``AltCorrBlock(fmaps, num_levels=4, radius=3)`` and
   ``__call__(coords, ii, jj)`` (reference ``:90-117``) on ``altcorr_forward``.
 * :class:`CorrSampler` / :class:`CorrLayer` are the two ``torch.autograd.Function``
-  wrappers.  ``CorrSampler`` is the reference's (``:6-20``).  ``CorrLayer``'s
+  wrappers.  ``CorrSampler`` is the reference's (``:6-20``); :class:`PyramidSampler` samples
+  all levels of a CorrBlock at once.  ``CorrLayer``'s
   backward is the exact adjoint of the forward (``altcorr_backward`` with
   ``scale=1/16``): the reference's ``CorrLayer.backward`` cannot run as written
   (``:83-87`` unpacks three of five saved tensors and returns the wrong number of
@@ -44,6 +45,32 @@ class CorrSampler(torch.autograd.Function):
         return grad_volume, None, None
 
 
+class PyramidSampler(torch.autograd.Function):
+    """:class:`CorrSampler` of every pyramid level at coords / 2^level in one launch, concatenated;
+    coords [N, H, W, 2]; gradients w.r.t. the volumes."""
+
+    @staticmethod
+    def forward(ctx, coords, radius, *volumes):
+        ctx.save_for_backward(coords, *volumes)
+        ctx.radius = radius
+        return backends.corr_pyramid_forward(volumes, coords, radius)
+
+    @staticmethod
+    def backward(ctx, grad_output):
+        coords, *volumes = ctx.saved_tensors
+        rd = 2 * ctx.radius + 1
+        n, _, ht, wd = grad_output.shape
+        planar = coords.permute(0, 3, 1, 2).contiguous()
+        grads = []
+        for i, volume in enumerate(volumes):
+            if not ctx.needs_input_grad[2 + i]:
+                grads.append(None)
+                continue
+            g = grad_output[:, i * rd * rd:(i + 1) * rd * rd].contiguous().view(n, rd, rd, ht, wd)
+            grads.append(backends.corr_index_backward(volume, planar / 2 ** i, g, ctx.radius)[0])
+        return (None, None, *grads)
+
+
 class CorrBlock:
     """All-pairs correlation pyramid of HI-SLAM2's frontend (reference ``modules/corr.py:23-71``)."""
 
@@ -57,8 +84,12 @@ class CorrBlock:
         self.corr_pyramid = [v.view(batch * num, ht, wd, ht // 2 ** i, wd // 2 ** i) for i, v in enumerate(levels)]
 
     def __call__(self, coords):
-        out_pyramid = []
         batch, num, ht, wd, _ = coords.shape
+        levels = self.corr_pyramid[:self.num_levels]
+        pixels = coords.reshape(batch * num, ht, wd, -1)
+        if len(levels) == self.num_levels and backends.corr_pyramid_fits(levels, pixels, self.radius):
+            return PyramidSampler.apply(pixels.contiguous(), self.radius, *levels).view(batch, num, -1, ht, wd)
+        out_pyramid = []
         coords = coords.permute(0, 1, 4, 2, 3).contiguous().view(batch * num, 2, ht, wd)
         for i in range(self.num_levels):
             corr = CorrSampler.apply(self.corr_pyramid[i], (coords / 2 ** i).contiguous(), self.radius)

@@ -69,6 +69,15 @@ int hs2_frame_distance(const float* poses, int64_t num_poses, const float* disps
 int hs2_corr_index_forward(const void* volume, int dtype, int64_t n, int h1, int w1, int h2, int w2,
                            const float* coords, int radius, void* corr, hs2_stream_t stream);
 
+/* corr_pyramid_forward  (reference: hislam2/modules/corr.py:40-51, CorrBlock's lookup)
+ *   corr_index_forward of every pyramid level at coords / 2^level in one launch:
+ *   volumes[l] [n,h1,w1,h1>>l,w1>>l] of `dtype` (f32, f16, bf16) for 1 to 4 levels,
+ *   coords [n,h1,w1,2] f32 (x, y), radius 3 or 4
+ *   -> corr [n, levels*(2r+1)^2, h1, w1], the levels' channels one after the other.
+ */
+int hs2_corr_pyramid_forward(const void* const* volumes, int levels, int dtype, int64_t n, int h1, int w1,
+                             const float* coords, int radius, void* corr, hs2_stream_t stream);
+
 /* corr_index_backward  (reference: src/droid.cpp:266-275, src/correlation_kernels.cu:73-124,156-184)
  *   coords [n,2,h1,w1] f32, corr_grad [n,2r+1,2r+1,h1,w1] of `dtype`
  *   -> volume_grad [n,h1,w1,h2,w2] of `dtype`, fully written (zeros outside the windows).
