@@ -564,7 +564,7 @@ def corr_pyramid_fits(volumes, coords, radius):
         return False
     n, h, w, two = coords.shape
     v0 = volumes[0]
-    return two == 2 and 0 < n <= 65535 and v0.dtype in (torch.float32, torch.float16, torch.bfloat16) \
+    return two == 2 and 0 < n <= 65535 and h * w <= 1 << 24 and v0.dtype in (torch.float32, torch.float16, torch.bfloat16) \
         and all(v.dtype == v0.dtype and v.device == coords.device and v.is_contiguous()
                 and tuple(v.shape) == (n, h, w, h >> l, w >> l) and v.numel() for l, v in enumerate(volumes))
 

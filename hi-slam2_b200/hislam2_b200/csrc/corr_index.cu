@@ -112,8 +112,10 @@ corr_index_fwd_kernel(const T* __restrict__ volume, const float* __restrict__ co
 // target are read.  Output: a warp owns one x offset and 32 pixels and walks the window
 // rows: u = (1 - fx) w[a] + fx w[a+1] once per row, two rows per output.
 // Bound by the window rows' DRAM sectors (about 4x the taps' bytes at levels 0 and 1).
-// 258 edges at 43x77, radius 4, four FP16 levels: 0.64 ms (1950 GB/s of taps and outputs),
+// 258 edges at 43x77, radius 4, four FP16 levels: 0.58 ms (DRAM at 4.2 TB/s, 2.4 GB moved),
 // against 0.90 ms for four launches of 2-byte gathers plus 0.64 ms of copies to concatenate them.
+constexpr int kCiMaxPlane = 1 << 24;   // elements of a target plane this kernel takes (64 of them stay below 2^31)
+
 struct CiLevels {
   const void* vol[4];
   int h2[4], w2[4];
@@ -143,7 +145,7 @@ corr_index_fwd_r_kernel(const __grid_constant__ CiLevels lv, const float* __rest
   const int n = blockIdx.y, lvl = blockIdx.z;
   const int h2 = lv.h2[lvl], w2 = lv.w2[lvl];
   const int HW1 = h1 * w1;
-  const int64_t HW2 = (int64_t)h2 * w2;
+  const unsigned HW2 = (unsigned)h2 * (unsigned)w2;   // at most kCiMaxPlane: offsets inside the tile fit 31 bits
   const int pix0 = blockIdx.x * TP;
   const int tid = threadIdx.x;
   if (tid < TP) {
@@ -157,7 +159,7 @@ corr_index_fwd_r_kernel(const __grid_constant__ CiLevels lv, const float* __rest
     org[tid] = make_int2(min(max((int)fx, -(1 << 20)), 1 << 20) - R, min(max((int)fy, -(1 << 20)), 1 << 20) - R);
   }
   __syncthreads();
-  const T* vol = static_cast<const T*>(lv.vol[lvl]) + ((int64_t)n * HW1 + pix0) * HW2;
+  const T* vol = static_cast<const T*>(lv.vol[lvl]) + ((int64_t)n * HW1 + pix0) * (int64_t)HW2;
   const int par0 = (int)(reinterpret_cast<uintptr_t>(vol) >> 1) & 1;   // 16-bit: element parity of the tile's planes
   {
     const int g = tid / S::SLOTS, slot = tid - g * S::SLOTS, jy = slot / S::WORDS, word = slot - jy * S::WORDS;
@@ -168,18 +170,17 @@ corr_index_fwd_r_kernel(const __grid_constant__ CiLevels lv, const float* __rest
       v[i] = 0u;
       if (g < S::GROUPS && p < TP && pix0 + p < HW1) {
         const int2 o = org[p];
-        const int y1 = o.y + jy;
-        const bool row = y1 >= 0 && y1 < h2;
-        const int64_t e0 = (int64_t)p * HW2 + (int64_t)y1 * w2 + o.x;          // first tap's element
+        const unsigned y1 = (unsigned)(o.y + jy);
+        // the first tap's element; a window row's column before or past the target is not read
+        const unsigned e0 = (unsigned)p * HW2 + y1 * (unsigned)w2 + (unsigned)o.x;
         if (S::kWords) {
-          const int par = (int)((e0 + par0) & 1);
+          const int par = (int)(e0 + par0) & 1;
           const int c = o.x - par + 2 * word;                                  // column of the word's first half
-          const int lo = max(o.x, 0), hi = min(o.x + D, w2);
-          if (row && c + 1 >= lo && c < hi)
-            v[i] = __ldg(reinterpret_cast<const uint32_t*>(vol + (e0 - par + 2 * word)));
+          if (y1 < (unsigned)h2 && (unsigned)(c + 1) <= (unsigned)w2)          // -1 <= c < w2: one half is a tap's
+            v[i] = __ldg(reinterpret_cast<const uint32_t*>(vol + (int)(e0 - par + 2 * word)));
         } else {
-          const int c = o.x + word;
-          if (row && c >= 0 && c < w2) v[i] = __float_as_uint(to_f(vol[e0 + word]));
+          if (y1 < (unsigned)h2 && (unsigned)(o.x + word) < (unsigned)w2)
+            v[i] = __float_as_uint(to_f(vol[(int)(e0 + word)]));
         }
       }
     }
@@ -197,14 +198,18 @@ corr_index_fwd_r_kernel(const __grid_constant__ CiLevels lv, const float* __rest
   const float gx = 1.f - f.x, gy = 1.f - f.y;
   const bool va = o.x + a >= 0 && o.x + a < w2, vb = o.x + a + 1 >= 0 && o.x + a + 1 < w2;
   T* out = corr + (((int64_t)n * gridDim.z + lvl) * RD * RD + a * RD) * HW1 + pix;
+  // 16-bit rows start at either half of a word: rows jy and jy + 2 alike
+  const int off0 = (par0 + p * (int)HW2 + o.y * w2 + o.x) & 1;
+  const T* hrow[2];
+  hrow[0] = reinterpret_cast<const T*>(win + p * S::LD) + off0 + a;
+  hrow[1] = reinterpret_cast<const T*>(win + p * S::LD) + ((off0 ^ w2) & 1) + a;
   float prev = 0.f;
 #pragma unroll
   for (int jy = 0; jy < D; ++jy) {
     float w0, w1v;
     if (S::kWords) {
       // words outside the target are 0; a word that straddles its edge is cut here
-      const int off = (par0 + p * (int)(HW2 & 1) + (o.y + jy) * w2 + o.x) & 1;
-      const T* row = reinterpret_cast<const T*>(win + p * S::LD + jy * S::WORDS) + off + a;
+      const T* row = hrow[jy & 1] + 2 * jy * S::WORDS;
       w0 = va ? to_f(row[0]) : 0.f;
       w1v = vb ? to_f(row[1]) : 0.f;
     } else {
@@ -305,7 +310,7 @@ template <typename T>
 static int launch_fwd(const void* volume, int64_t n, int h1, int w1, int h2, int w2, const float* coords,
                       int radius, void* corr, cudaStream_t stream) {
   const int HW1 = h1 * w1;
-  if (radius == 3 || radius == 4) {
+  if ((radius == 3 || radius == 4) && (int64_t)h2 * w2 <= kCiMaxPlane) {
     CiLevels lv{};
     lv.vol[0] = volume;
     lv.h2[0] = h2;
@@ -378,7 +383,8 @@ extern "C" int hs2_corr_pyramid_forward(const void* const* volumes, int levels, 
   using namespace hs2;
   int rc = check_dims("corr_pyramid_forward", n, h1, w1, h1, w1, radius);
   if (rc) return rc;
-  if (levels < 1 || levels > 4 || (radius != 3 && radius != 4) || (h1 >> (levels - 1)) < 1 || (w1 >> (levels - 1)) < 1) {
+  if (levels < 1 || levels > 4 || (radius != 3 && radius != 4) || (h1 >> (levels - 1)) < 1 || (w1 >> (levels - 1)) < 1 ||
+      (int64_t)h1 * w1 > kCiMaxPlane) {
     set_error("corr_pyramid_forward: 1 to 4 levels of a [%d, %d] target and radius 3 or 4 (got %d levels, radius %d)",
               h1, w1, levels, radius);
     return HS2_ERR_INVALID;
