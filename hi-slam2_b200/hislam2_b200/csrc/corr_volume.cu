@@ -14,24 +14,37 @@
 //   corr_pack      fmaps [K, 128, H, W] -> K-major operand rows [K, H*W, 128]
 //                  (x 0.25, which is exact; or, for the FP8 form, e4m3 values with one
 //                  scale per pixel: q = e4m3(f/4 / s), s = max_c |f/4| / 448);
-//   corr_volume    persistent (one CTA per SM), one work unit = (edge, 128 source
-//                  pixels).  Warp 0 streams the unit's A tile (128 source pixels x
-//                  128 channels) and, per N tile, the B tile of TWO target image
-//                  rows (each a box of RW = round_up(W, 16) pixels; pixels past the
-//                  frame read as zero) with 3-D TMA boxes (128B swizzle) into a
-//                  2-stage ring; warp 1 issues tcgen05.mma (kind::f16 for F16/BF16,
-//                  kind::f8f6f4 for E4M3; M = 128, N = 2 RW, accumulator F32) into
-//                  one of two 256-column TMEM buffers; warps 2-17 (four per TMEM
-//                  lane quarter, each half an image row of the tile) drain the
-//                  accumulator (tcgen05.ld), round to the volume type into a
-//                  shared staging tile, write level 0 in 16-byte chunks aligned in
-//                  global memory, pool level 1 from the two rows of the tile, and
-//                  levels 2 and 3 from two-row rings of the levels above.
+//   corr_volume    persistent (two CTAs per SM), one work unit = (edge, 128 source
+//                  pixels, a run of target image rows that starts at a multiple of 8).
+//                  Warp 0 streams the unit's A tile (128 source pixels x 128 channels)
+//                  and, per target image row, the B tile (a box of RW = round_up(W, 16)
+//                  pixels; pixels past the frame read as zero) with 3-D TMA boxes (128B
+//                  swizzle) into a 2-stage ring; warp 1 issues tcgen05.mma (kind::f16
+//                  for F16/BF16, kind::f8f6f4 for E4M3; M = 128, N = RW, accumulator
+//                  F32) into a ring of TMEM column ranges, one per image row; warps 2-5
+//                  (one per TMEM lane quarter, lane = source pixel) drain it for level
+//                  0, warps 6-9 for the pooled levels.
+// Epilogue: a lane owns a source pixel.  Each level of a source pixel is one contiguous run
+// of the output that grows with the image rows, so per image row and level a lane
+// appends its new elements, 16 accumulator columns at a time, to its row of a per-warp
+// staging buffer at the run's 16-byte phase in global memory; the warp then writes all
+// full 16-byte chunks (neighbouring lanes, neighbouring chunks) and each lane keeps its
+// partial chunk in registers for the next append.  Level 1 reads the two image rows'
+// accumulators again from TMEM and pools the rounded values; the rows above of levels 1
+// and 2 wait in shared memory.  No barrier spans the epilogue warps, single elements are
+// written only at the ends of a unit's runs, and everything runs in short loops: the
+// same epilogue unrolled over the columns missed the instruction cache and took 3.2 ms.
 // The volume is never re-read: the HBM traffic is the pyramid's writes plus the
 // operand reads (L2-resident: one frame's operand rows are 848 KB at 43x77).
+// Bound by instruction issue (IPC 1.8 per SM, 20% of the stalls on instruction fetch): the
+// DRAM floor is a third.  48 edges of 43x77, FP16, four levels: 0.68 ms, and 84 edges of
+// 48x64: 0.79 ms, against 1.40 and 1.94 ms for sixteen epilogue warps sharing a staging tile
+// between barriers (pooling from shared memory, element-wise run ends on every tile).
 //
 // Limits: 128 channels, W <= 96, H*W < 2^31 / 128.  Output element offsets are 64-bit.
 #include <cuda_fp8.h>
+
+#include <algorithm>
 
 #include "profile.cuh"
 #include "tc.cuh"
@@ -42,13 +55,11 @@ namespace {
 
 constexpr int kCvC = 128;          // feature channels (K of the contraction)
 constexpr int kCvMaxW = 96;        // widest image row a B box holds
-constexpr int kCvMaxRW = 96;       // round_up(kCvMaxW, 16): accumulator columns per image row
-constexpr int kCvEpiWarps = 16;    // four per TMEM lane quarter
+constexpr int kCvEpiWarps = 8;     // per TMEM lane quarter one for level 0, one for the pooled levels
 constexpr int kCvThreads = 32 * (2 + kCvEpiWarps);   // TMA, MMA, epilogue
-constexpr int kCvEpiThreads = 32 * kCvEpiWarps;
-constexpr int kCvRowsPerWarp = 128 / kCvEpiWarps;   // staging rows of a warp in phase B
-constexpr int kCvStages = 2;
-constexpr int kCvTmemCols = 512;   // two 256-column accumulators
+constexpr int kCvTmemCols = 256;
+constexpr int kCvMaxRegions = 4;   // image rows held in TMEM
+constexpr uint32_t kCvMinSmem = 77 * 1024, kCvPairSmem = 113 * 1024;   // two CTAs per SM (they fill TMEM)
 constexpr uint32_t kCvASub = 128 * 128;   // one 128-row x 128-byte swizzled sub-tile
 
 // operand forms: F16 / BF16 (kind::f16), E4M3 with per-pixel scales (kind::f8f6f4)
@@ -65,12 +76,16 @@ template <> struct Prec<kE4M3> {
 };
 
 struct CvGeom {
-  int H, W, HW, RW, SST;           // grid, row box, staging row stride (elements)
+  int H, W, HW, RW;
   int H1, W1, H2, W2, H3, W3;      // pooled level sizes
-  int levels, mtiles, ntiles;
+  int levels, mtiles, splits, split_rows;
   int64_t E;
-  uint32_t sub_b;                  // bytes of one B sub-tile (2 RW rows x 128 B)
-  uint32_t off_b, off_stg, off_r1, off_r2, off_bar, smem;
+  int stages, regions;             // B tiles in flight, accumulators in TMEM
+  // 16-byte chunks per lane (odd): staging rows of level 0 and of the pooled levels, level-1 and
+  // level-2 row above
+  int chunks, chunks_p, chunks1, chunks2;
+  uint32_t sub_b;                  // bytes of one B sub-tile (RW rows x 128 B)
+  uint32_t off_b, off_stg, off_stp, off_p1, off_p2, off_bar, smem;
 };
 
 CvGeom cv_geom(int H, int W, int64_t E, int levels, int esub) {
@@ -79,20 +94,36 @@ CvGeom cv_geom(int H, int W, int64_t E, int levels, int esub) {
   g.W = W;
   g.HW = H * W;
   g.RW = (W + 15) & ~15;
-  g.SST = 2 * g.RW + 2;                 // >= 2 W; SST / 2 odd
   g.H1 = H / 2, g.W1 = W / 2, g.H2 = g.H1 / 2, g.W2 = g.W1 / 2, g.H3 = g.H2 / 2, g.W3 = g.W2 / 2;
   g.levels = levels;
   g.mtiles = (g.HW + 127) / 128;
-  g.ntiles = (H + 1) / 2;
   g.E = E;
-  g.sub_b = (uint32_t)(2 * g.RW * 128);
-  const uint32_t a_bytes = 2 * kCvASub;
-  g.off_b = a_bytes;
-  g.off_stg = g.off_b + kCvStages * esub * g.sub_b;
-  g.off_r1 = g.off_stg + 128u * g.SST * 2;
-  g.off_r2 = g.off_r1 + 2u * 128 * (g.RW / 2) * 2;
-  g.off_bar = (g.off_r2 + 2u * 128 * (g.RW / 4) * 2 + 15) & ~15u;
-  g.smem = g.off_bar + 256 + 1024;   // barriers, flags, TMEM slot; 1 KB alignment slack
+  // image rows per unit: whole frames unless that leaves the last of few waves mostly empty;
+  // runs of a multiple of 8 rows keep the pooled levels inside a unit
+  const int groups = (H + 7) / 8;
+  const int64_t whole = std::max<int64_t>(1, E * g.mtiles);
+  const int want = (int)std::min<int64_t>(groups, std::max<int64_t>(1, (8 * 2 * kNumSMs + whole - 1) / whole));
+  g.split_rows = 8 * ((groups + want - 1) / want);
+  g.splits = (H + g.split_rows - 1) / g.split_rows;
+  g.sub_b = (uint32_t)(g.RW * 128);
+  g.regions = std::min(kCvMaxRegions, kCvTmemCols / g.RW);
+  g.chunks = (((7 + W) >> 3) + 1) | 1;
+  g.chunks_p = (((7 + g.W1) >> 3) + 1) | 1;
+  g.chunks1 = (g.RW / 16) | 1;
+  g.chunks2 = ((g.RW + 31) / 32) | 1;
+  g.off_b = (uint32_t)esub * kCvASub;
+  // two B tiles in flight and two CTAs per SM; at W > 64 one B tile (the ring of accumulators covers its
+  // load), at W > 80 two B tiles in one CTA
+  for (int n : {2, 1, 2}) {
+    g.stages = n;
+    g.off_stg = g.off_b + g.stages * esub * g.sub_b;
+    g.off_stp = g.off_stg + 4 * (32u * g.chunks * 16 + 64);
+    g.off_p1 = g.off_stp + 4 * (32u * g.chunks_p * 16 + 64);
+    g.off_p2 = g.off_p1 + 128u * 16 * g.chunks1;
+    g.off_bar = g.off_p2 + 128u * 16 * g.chunks2;
+    g.smem = std::max(kCvMinSmem, g.off_bar + 256 + 1024);   // barriers, flags, TMEM slot; 1 KB alignment slack
+    if (g.smem <= kCvPairSmem) break;
+  }
   return g;
 }
 
@@ -107,15 +138,6 @@ template <> __device__ __forceinline__ __nv_bfloat16 from_bits16<__nv_bfloat16>(
   return __ushort_as_bfloat16(b);
 }
 
-__device__ __forceinline__ void epi_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kCvEpiThreads) : "memory"); }
-// Barrier of the epilogue warps that also ANDs a predicate over them (a CTA-uniform decision).
-__device__ __forceinline__ bool epi_sync_and(bool v) {
-  uint32_t r;
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.and.pred q, 1, %2, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
-      : "=r"(r) : "r"((uint32_t)v), "n"(kCvEpiThreads) : "memory");
-  return r != 0;
-}
 // Bounded wait that ignores the abort flag: used on the way out to let copies and
 // MMAs that were already issued land before the CTA releases its memory.
 __device__ __forceinline__ void drain_wait(uint32_t bar, uint32_t parity) {
@@ -123,16 +145,119 @@ __device__ __forceinline__ void drain_wait(uint32_t bar, uint32_t parity) {
   }
 }
 
-// Rounded 2x2 average of four 16-bit values, in avg_pool2d's order.
-template <typename T>
-__device__ __forceinline__ uint16_t pool4(uint16_t a, uint16_t b, uint16_t c, uint16_t d) {
-  float s = 0.f;
-  s += to_f<T>(from_bits16<T>(a));
-  s += to_f<T>(from_bits16<T>(b));
-  s += to_f<T>(from_bits16<T>(c));
-  s += to_f<T>(from_bits16<T>(d));
-  return bits16<T>(from_f<T>(s / 4.0f));
+// Two floats rounded to T, the first in the low half.
+template <typename T> __device__ __forceinline__ uint32_t pack2(float lo, float hi);
+template <> __device__ __forceinline__ uint32_t pack2<__half>(float lo, float hi) {
+  const __half2 h = __floats2half2_rn(lo, hi);
+  return *reinterpret_cast<const uint32_t*>(&h);
 }
+template <> __device__ __forceinline__ uint32_t pack2<__nv_bfloat16>(float lo, float hi) {
+  const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
+template <typename T> __device__ __forceinline__ float2 unpack2(uint32_t w) {
+  return make_float2(to_f<T>(from_bits16<T>((uint16_t)w)), to_f<T>(from_bits16<T>((uint16_t)(w >> 16))));
+}
+
+// 2x2 average of the rounded pairs (y, x), (y, x+1) and (y+1, x), (y+1, x+1), in avg_pool2d's order.
+template <typename T>
+__device__ __forceinline__ float pool4(uint32_t top, uint32_t bottom) {
+  const float2 a = unpack2<T>(top), b = unpack2<T>(bottom);
+  // the + 0 turns a sum of negative zeros into the 0 that avg_pool2d's sum from 0 gives
+  return fmaf(a.x + a.y + b.x + b.y, 0.25f, 0.f);
+}
+
+// How the warp's lanes share a flush of up to `per` full chunks a row: lane = (row of a group,
+// chunk); the chunk stays, the rows step by whole groups.
+struct CvShare {
+  int group, r0, c;
+  __device__ explicit CvShare(int n) {
+    const int per = (7 + n) >> 3, lane = threadIdx.x & 31;
+    group = per > 0 ? 32 / per : 32;
+    r0 = per > 0 ? lane / per : 0;
+    c = lane - r0 * per;
+    if (per == 0 || r0 >= group) r0 = 32;             // idle
+  }
+};
+
+// Writes the warp's full chunks after an append of n elements.  Row r of the warp holds the
+// run of source pixel r; its new elements start at out[g0 + r * plane], `since` elements after
+// the unit's part of the run began.  rows: live rows of the warp; done: the unit's last append.
+// Returns the lane's partial chunk.
+// One copy for all levels: inlined everywhere, the epilogue's loops outgrow the instruction cache.
+__device__ __noinline__ uint4 run_flush(const CvShare sh, uint16_t* __restrict__ out, int64_t g0, int plane, int n,
+                                        int since, bool done, int rows, int chunks, const uint8_t* stg) {
+  const int lane = threadIdx.x & 31;
+  __syncwarp();
+  const int ph0 = (int)(g0 & 7);
+  uint16_t* base = out + (g0 - ph0);
+  // a chunk that also holds elements before the unit's part of the run (chunk 0 at a phase beyond
+  // `since`) is left to its lane
+  const int lim = sh.c == 0 ? since : 8, step = sh.group * plane;
+  int rel = ph0 + sh.r0 * plane;
+#pragma unroll 2
+  for (int r = sh.r0; r < rows; r += sh.group, rel += step) {
+    const int off = rel & 7;
+    if (8 * sh.c + 8 <= off + n && off <= lim) {
+      const uint4 v = *reinterpret_cast<const uint4*>(stg + 16 * (r * chunks + (r >> 3) + sh.c));
+      *reinterpret_cast<uint4*>(base + (rel - off + 8 * sh.c)) = v;
+    }
+  }
+  rel = ph0 + lane * plane;
+  const int off = rel & 7, total = off + n;
+  const uint8_t* row = stg + 16 * (lane * chunks + (lane >> 3));
+  if ((since < 8 || done) && lane < rows) {           // the ends of the unit's part of the run
+    const uint16_t* el = reinterpret_cast<const uint16_t*>(row);
+    uint16_t* dst = base + (rel - off);
+    const int head = off > since ? off - since : 0;   // elements of chunk 0 that are not the unit's
+    if (head && total >= 8)
+      for (int i = head; i < 8; ++i) dst[i] = el[i];
+    if (done)
+      for (int i = max(total & ~7, head); i < total; ++i) dst[i] = el[i];
+  }
+  const uint4 tail = *reinterpret_cast<const uint4*>(row + 16 * (total >> 3));
+  __syncwarp();
+  return tail;
+}
+
+// A lane's append to its staging row, word by word.  At an odd phase every stored word joins
+// the halves of neighbouring pairs: one byte permute, whose selector is the lane's.
+struct CvAppend {
+  uint32_t* dst;
+  uint32_t prev, sel;
+  int left;                                           // words to store
+  // n elements at phase off, after the run's partial chunk
+  __device__ CvAppend(uint8_t* row, const uint4& tail, int off, int n) {
+    *reinterpret_cast<uint4*>(row) = tail;
+    const int odd = off & 1;
+    prev = odd ? (uint32_t)reinterpret_cast<const uint16_t*>(row)[off - 1] << 16 : 0u;
+    sel = odd ? 0x5432u : 0x7654u;
+    dst = reinterpret_cast<uint32_t*>(row) + (off >> 1);
+    left = (n + odd + 1) >> 1;
+  }
+  template <int K>
+  __device__ __forceinline__ void put(const uint32_t (&w)[K]) {
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      if (k < left) dst[k] = __byte_perm(prev, w[k], sel);
+      prev = w[k];
+    }
+    dst += K;
+    left -= K;
+  }
+  // as put, for words that all belong to the run
+  template <int K>
+  __device__ __forceinline__ void put_full(const uint32_t (&w)[K]) {
+#pragma unroll
+    for (int k = 0; k < K; ++k) dst[k] = __byte_perm(k ? w[k - 1] : prev, w[k], sel);
+    prev = w[K - 1];
+    dst += K;
+    left -= K;
+  }
+  __device__ __forceinline__ void end() {             // an odd phase's last half word
+    if (left > 0) *dst = __byte_perm(prev, 0u, sel);
+  }
+};
 
 }  // namespace
 
@@ -191,10 +316,11 @@ struct CvOut {
 };
 
 template <int P, typename T>
-__global__ void __launch_bounds__(kCvThreads, 1)
+__global__ void __launch_bounds__(kCvThreads, 2)
 corr_volume_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant__ CUtensorMap bmap,
                    const int64_t* __restrict__ ii, const int64_t* __restrict__ jj, int64_t K1, int64_t K2,
-                   const float* __restrict__ s1, const float* __restrict__ s2, CvGeom g, CvOut out,
+                   const float* __restrict__ s1, const float* __restrict__ s2, const __grid_constant__ CvGeom g,
+                   const __grid_constant__ CvOut out,
                    int32_t* __restrict__ info) {
   using PR = Prec<P>;
   extern __shared__ uint8_t cv_raw[];
@@ -202,27 +328,23 @@ corr_volume_kernel(const __grid_constant__ CUtensorMap amap, const __grid_consta
   const uint32_t base = (raw + 1023u) & ~1023u;
   uint8_t* gb = cv_raw + (base - raw);
   uint64_t* bars = reinterpret_cast<uint64_t*>(gb + g.off_bar);
-  // a_full, a_empty, b_full[2], b_empty[2], t_full[2], t_empty[2], mma_done
+  // a_full, a_empty, b_full[2], b_empty[2], t_full[4], t_empty[4], mma_done
   const uint32_t bar0 = tc::smem_u32(bars);
   const uint32_t a_full = bar0, a_empty = bar0 + 8;
-  const uint32_t b_full = bar0 + 16, b_empty = bar0 + 32, t_full = bar0 + 48, t_empty = bar0 + 64;
-  const uint32_t mma_done = bar0 + 80;
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(gb + g.off_bar + 96);
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gb + g.off_bar + 104);
-  uint16_t* stg = reinterpret_cast<uint16_t*>(gb + g.off_stg);
-  uint16_t* ring1 = reinterpret_cast<uint16_t*>(gb + g.off_r1);
-  uint16_t* ring2 = reinterpret_cast<uint16_t*>(gb + g.off_r2);
-  const int R1 = g.RW / 2, R2 = g.RW / 4;   // ring row strides (elements)
+  const uint32_t b_full = bar0 + 16, b_empty = bar0 + 32, t_full = bar0 + 48, t_empty = bar0 + 80;
+  const uint32_t mma_done = bar0 + 112;
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(gb + g.off_bar + 128);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gb + g.off_bar + 136);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid == 0) {
     tc::mbar_init(a_full, 1);
     tc::mbar_init(a_empty, 1);
-    for (int s = 0; s < kCvStages; ++s) {
+    for (int s = 0; s < g.stages; ++s) {
       tc::mbar_init(b_full + 8 * s, 1);
       tc::mbar_init(b_empty + 8 * s, 1);
     }
-    for (int b = 0; b < 2; ++b) {
+    for (int b = 0; b < g.regions; ++b) {
       tc::mbar_init(t_full + 8 * b, 1);
       tc::mbar_init(t_empty + 8 * b, kCvEpiWarps);
     }
@@ -240,17 +362,26 @@ corr_volume_kernel(const __grid_constant__ CUtensorMap amap, const __grid_consta
   tc::fence_after();
   const uint32_t tmem = *tmem_slot;
 
-  const int64_t units = g.E * g.mtiles;
+  const int64_t units = g.E * g.mtiles * g.splits;
   const uint32_t b_stage = (uint32_t)PR::kSub * g.sub_b;
   const int kbox = 128 / PR::kEsize;                  // elements per 128-byte box row
+  // unit u -> edge, first source pixel, image rows [i0, i1)
+  auto unit_of = [&](int64_t u, int64_t& e, int& m0, int& i0, int& i1) {
+    const int64_t em = u / g.splits;
+    i0 = (int)(u - em * g.splits) * g.split_rows;
+    i1 = min(g.H, i0 + g.split_rows);
+    e = em / g.mtiles;
+    m0 = (int)(em - e * g.mtiles) * 128;
+  };
 
   if (warp == 0) {
     // ------------------------------------------------------------- TMA producer
     if (lane == 0) {
       uint32_t gt = 0, ul = 0;
       for (int64_t u = blockIdx.x; u < units; u += gridDim.x) {
-        const int64_t e = u / g.mtiles;
-        const int m0 = (int)(u - e * g.mtiles) * 128;
+        int64_t e;
+        int m0, i0, i1;
+        unit_of(u, e, m0, i0, i1);
         const int64_t fi = ii[e], fj = jj[e];
         if (fi < 0 || fi >= K1 || fj < 0 || fj >= K2) continue;   // every role skips the unit
         if (ul > 0 && !tc::mbar_wait(a_empty, (ul - 1) & 1, abort_flag)) break;
@@ -259,50 +390,48 @@ corr_volume_kernel(const __grid_constant__ CUtensorMap amap, const __grid_consta
         for (int kb = 0; kb < PR::kSub; ++kb)
           tc::tma_load_3d(base + kb * kCvASub, &amap, kb * kbox, m0, (int)fi, a_full);
         bool ok = true;
-        for (int j = 0; j < g.ntiles; ++j, ++gt) {
-          const int s = gt % kCvStages;
-          if (gt >= kCvStages && !tc::mbar_wait(b_empty + 8 * s, ((gt / kCvStages) - 1) & 1, abort_flag)) {
+        for (int i = i0; i < i1; ++i, ++gt) {
+          const int s = gt % g.stages;
+          if (gt >= g.stages && !tc::mbar_wait(b_empty + 8 * s, ((gt / g.stages) - 1) & 1, abort_flag)) {
             ok = false;
             break;
           }
-          const int nrow = (2 * j + 1 < g.H) ? 2 : 1;
-          tc::mbar_arrive_tx(b_full + 8 * s, (uint32_t)(nrow * PR::kSub * g.RW * 128));
+          tc::mbar_arrive_tx(b_full + 8 * s, (uint32_t)(PR::kSub * g.RW * 128));
           const uint32_t dst = base + g.off_b + s * b_stage;
-          for (int r = 0; r < nrow; ++r)
-            for (int kb = 0; kb < PR::kSub; ++kb)
-              tc::tma_load_3d(dst + kb * g.sub_b + r * g.RW * 128, &bmap, kb * kbox, (2 * j + r) * g.W, (int)fj,
-                              b_full + 8 * s);
+          for (int kb = 0; kb < PR::kSub; ++kb)
+            tc::tma_load_3d(dst + kb * g.sub_b, &bmap, kb * kbox, i * g.W, (int)fj, b_full + 8 * s);
         }
         if (!ok) break;
       }
       // let the copies already issued land before the CTA's shared memory is released
       if (ul > 0) drain_wait(a_full, (ul - 1) & 1);
-      for (uint32_t k = gt > kCvStages ? gt - kCvStages : 0; k < gt; ++k)
-        drain_wait(b_full + 8 * (k % kCvStages), (k / kCvStages) & 1);
+      for (uint32_t k = gt > (uint32_t)g.stages ? gt - g.stages : 0; k < gt; ++k)
+        drain_wait(b_full + 8 * (k % g.stages), (k / g.stages) & 1);
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------- MMA issuer
     if (lane == 0) {
       uint32_t gt = 0, ul = 0;
+      const uint32_t id = tc::idesc(128, g.RW, PR::kFmt);
       for (int64_t u = blockIdx.x; u < units; u += gridDim.x) {
-        const int64_t e = u / g.mtiles;
+        int64_t e;
+        int m0, i0, i1;
+        unit_of(u, e, m0, i0, i1);
         const int64_t fi = ii[e], fj = jj[e];
         if (fi < 0 || fi >= K1 || fj < 0 || fj >= K2) continue;
         if (!tc::mbar_wait(a_full, ul & 1, abort_flag)) break;
         ++ul;
         bool ok = true;
-        for (int j = 0; j < g.ntiles; ++j, ++gt) {
-          const int s = gt % kCvStages, b = gt & 1;
-          if (!tc::mbar_wait(b_full + 8 * s, (gt / kCvStages) & 1, abort_flag) ||
-              (gt >= 2 && !tc::mbar_wait(t_empty + 8 * b, ((gt >> 1) - 1) & 1, abort_flag))) {
+        for (int i = i0; i < i1; ++i, ++gt) {
+          const uint32_t s = gt % g.stages, b = gt % g.regions, used = gt / g.regions;
+          if (!tc::mbar_wait(b_full + 8 * s, (gt / g.stages) & 1, abort_flag) ||
+              (used > 0 && !tc::mbar_wait(t_empty + 8 * b, (used - 1) & 1, abort_flag))) {
             ok = false;
             break;
           }
           tc::fence_after();
-          const int nrow = (2 * j + 1 < g.H) ? 2 : 1;
-          const uint32_t id = tc::idesc(128, nrow * g.RW, PR::kFmt);
           const uint32_t bsrc = base + g.off_b + s * b_stage;
-          const uint32_t d = tmem + (uint32_t)(b * 256);
+          const uint32_t d = tmem + b * g.RW;
 #pragma unroll
           for (int kb = 0; kb < PR::kSub; ++kb)
 #pragma unroll
@@ -324,175 +453,180 @@ corr_volume_kernel(const __grid_constant__ CUtensorMap amap, const __grid_consta
     }
   } else {
     // ------------------------------------------------------------- epilogue
-    // Phase A (per tile): warp (quarter q, half h) reads its 32 accumulator rows' columns
-    // of image row h from TMEM, rounds them and stores them, 4 bytes at a time, into the
-    // staging row of each source pixel: segment layout, image row 0 at [0, W), row 1 at
-    // [W, 2W) (row stride SST, SST/2 odd: the 32 rows of a store hit 32 banks).
-    // Phase B: warp ew owns staging rows 16 ew .. 16 ew + 15.  Level 0: the row's
-    // segment is one contiguous run of the volume row; it is written in 16-byte chunks
-    // aligned in GLOBAL memory (lane = (row, chunk parity)), each gathered from 8 staged
-    // elements -- whole sectors per store; the two chunks that straddle the segment's
-    // ends go element by element.  Levels 1-3: lanes over x per row, each pooled value
-    // written to its ring and to global memory by the lane that forms it.
-    const int ew = warp - 2;                 // 0..15
     const int q = warp & 3;                  // TMEM lane quarter
-    const int h = (ew >> 2) >> 1;            // image row of the tile (phase A)
-    const int half = (ew >> 2) & 1;          // which half of the row's RW columns
-    const int hw = g.RW / 2;                 // columns per warp (a multiple of 8)
-    const int r = q * 32 + lane;             // accumulator row = source pixel within the unit
-    const int pa = lane % kCvRowsPerWarp, pb = lane / kCvRowsPerWarp;
-    const int prow = kCvRowsPerWarp * ew + pa;   // phase B staging row of this lane
-    constexpr int kChunkLanes = 32 / kCvRowsPerWarp;
-    const int64_t L1n = (int64_t)g.H1 * g.W1, L2n = (int64_t)g.H2 * g.W2, L3n = (int64_t)g.H3 * g.W3;
-    uint32_t gt = 0;
+    const bool pooled = warp >= 6;           // this warp's levels: 0, or 1 to 3
+    const int np = g.RW / 16;                // 16-column pieces of an image row
+    const int chunks = pooled ? g.chunks_p : g.chunks;
+    uint8_t* stg = gb + (pooled ? g.off_stp : g.off_stg) + q * (32 * chunks * 16 + 64);
+    // the skew of one chunk per eight rows spreads the rows of a store over the banks
+    uint8_t* row = stg + 16 * (lane * chunks + (lane >> 3));
+    const uint32_t tq = tmem + ((uint32_t)(q * 32) << 16);
+    uint32_t reg = 0, par = 0;               // the next accumulator row's TMEM range and barrier phase
+    const uint32_t last_reg = g.regions - 1;
+    auto next_row = [&]() {
+      if (reg == last_reg) {
+        reg = 0;
+        par ^= 1;
+      } else {
+        ++reg;
+      }
+    };
     for (int64_t u = blockIdx.x; u < units; u += gridDim.x) {
-      const int64_t e = u / g.mtiles;
-      const int m0 = (int)(u - e * g.mtiles) * 128;
+      int64_t e;
+      int m0, i0, i1;
+      unit_of(u, e, m0, i0, i1);
       const int64_t fi = ii[e], fj = jj[e];
       if (fi < 0 || fi >= K1 || fj < 0 || fj >= K2) {
         if (tid == 64 && m0 == 0) atomicOr(info, HS2_DEV_BAD_INDEX);
         continue;
       }
+      const int64_t px0 = e * g.HW + m0 + 32 * q;                 // the warp's first source pixel
+      const int rows = min(32, g.HW - m0 - 32 * q);               // live ones (may be <= 0)
       float sa = 1.f;
-      if (P == kE4M3) sa = (m0 + r < g.HW) ? s1[fi * g.HW + m0 + r] : 0.f;
-      bool ok = true;
-      for (int j = 0; j < g.ntiles; ++j, ++gt) {
-        const int b = gt & 1;
-        const int nrow = (2 * j + 1 < g.H) ? 2 : 1;
-        ok = tc::mbar_wait(t_full + 8 * b, (gt >> 1) & 1, abort_flag);
+      if (P == kE4M3) sa = lane < rows ? s1[fi * g.HW + m0 + 32 * q + lane] : 0.f;
+      // waits for the accumulator in TMEM range r (uniform over the warp)
+      auto wait_row = [&](uint32_t r, uint32_t ph) -> bool {
+        const bool ok = tc::mbar_wait(t_full + 8 * r, ph, abort_flag);
         tc::fence_after();
-        if (ok && h < nrow) {
-          constexpr int kHalf = kCvMaxRW / 2;
-          uint32_t v[kHalf];
+        return __all_sync(0xffffffffu, ok);
+      };
+      auto free_row = [&](uint32_t r) {
+        if (lane == 0) tc::mbar_arrive(t_empty + 8 * r);
+      };
+      auto load = [&](uint32_t r, int pc, uint32_t (&v)[16]) { tc::ld16(tq + r * g.RW + 16 * pc, v); };
+      // the 16 values of piece pc of image row i, rounded, in 8 words
+      auto pack = [&](uint32_t (&v)[16], int i, int pc, uint32_t (&w)[8]) {
+        if (P == kE4M3) {
+          const float* sc = s2 + fj * g.HW + (int64_t)i * g.W;
 #pragma unroll
-          for (int c0 = 0; c0 < kHalf; c0 += 8) {
-            if (c0 < hw) {
-              uint32_t t8[8];
-              tc::ld8(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * 256 + h * g.RW + half * hw + c0), t8);
+          for (int k = 0; k < 16; ++k) {
+            const int x = 16 * pc + k;
+            v[k] = __float_as_uint(__uint_as_float(v[k]) * sa * (x < g.W ? __ldg(sc + x) : 0.f));
+          }
+        }
 #pragma unroll
-              for (int k = 0; k < 8; ++k) v[c0 + k] = t8[k];
-            }
+        for (int k = 0; k < 8; ++k) w[k] = pack2<T>(__uint_as_float(v[2 * k]), __uint_as_float(v[2 * k + 1]));
+      };
+      bool ok = true;
+      if (!pooled) {
+        const CvShare sh(g.W);
+        uint4 tail = make_uint4(0, 0, 0, 0);
+        for (int i = i0; i < i1; ++i) {
+          if (!(ok = wait_row(reg, par))) break;
+          const int64_t g0 = px0 * g.HW + (int64_t)i * g.W;
+          CvAppend ap(row, tail, ((int)(g0 & 7) + lane * g.HW) & 7, g.W);
+          uint32_t v[2][16], w[8];
+          load(reg, 0, v[0]);
+          int pc = 0;
+          for (; pc + 2 < np; pc += 2) {                          // the next piece's load runs under this one's stores
+            tc::ld_wait();
+            load(reg, pc + 1, v[1]);
+            pack(v[0], i, pc, w);
+            ap.put_full(w);
+            tc::ld_wait();
+            load(reg, pc + 2, v[0]);
+            pack(v[1], i, pc + 1, w);
+            ap.put_full(w);
           }
           tc::ld_wait();
-          const int xb = half * hw;          // first image column of this warp
-          if (P == kE4M3) {
-            // column scales of the warp's columns (lane c holds columns xb + c, xb + c + 32)
-            float sc[(kHalf + 31) / 32];
+          if (pc + 1 < np) {
+            load(reg, pc + 1, v[1]);
+            pack(v[0], i, pc, w);
+            ap.put_full(w);
+            tc::ld_wait();
 #pragma unroll
-            for (int k = 0; k < (kHalf + 31) / 32; ++k) {
-              const int x = xb + lane + 32 * k;
-              sc[k] = (lane + 32 * k < hw && x < g.W) ? s2[fj * g.HW + (int64_t)(2 * j + h) * g.W + x] : 0.f;
-            }
-#pragma unroll
-            for (int x = 0; x < kHalf; ++x) {
-              const float scale = __shfl_sync(0xffffffffu, sc[x >> 5], x & 31);
-              v[x] = __float_as_uint(__uint_as_float(v[x]) * sa * scale);
-            }
+            for (int k = 0; k < 16; ++k) v[0][k] = v[1][k];
+            ++pc;
           }
-          uint16_t* srow = stg + r * g.SST + h * g.W + xb;
-          const int nv = min(hw, g.W - xb);   // valid columns of this warp
-          auto q16 = [&](int x) -> uint32_t { return (uint32_t)bits16<T>(from_f<T>(__uint_as_float(v[x]))); };
-          if (((h * g.W + xb) & 1) == 0) {
-#pragma unroll
-            for (int x = 0; x < kHalf; x += 2) {
-              if (x + 1 < nv) *reinterpret_cast<uint32_t*>(srow + x) = q16(x) | (q16(x + 1) << 16);
-              else if (x < nv) srow[x] = (uint16_t)q16(x);
-            }
-          } else {
-            if (nv > 0) srow[0] = (uint16_t)q16(0);
-#pragma unroll
-            for (int x = 1; x < kHalf; x += 2) {
-              if (x + 1 < nv) *reinterpret_cast<uint32_t*>(srow + x) = q16(x) | (q16(x + 1) << 16);
-              else if (x < nv) srow[x] = (uint16_t)q16(x);
-            }
-          }
+          tc::fence_before();
+          __syncwarp();
+          free_row(reg);
+          pack(v[0], i, pc, w);
+          ap.put(w);
+          ap.end();
+          tail = run_flush(sh, out.lvl[0], g0, g.HW, g.W, (i - i0) * g.W, i == i1 - 1, rows, chunks, stg);
+          next_row();
         }
-        tc::fence_before();
-        __syncwarp();
-        if (lane == 0) tc::mbar_arrive(t_empty + 8 * b);
-        ok = epi_sync_and(ok);               // uniform over the epilogue warps from here on
-        if (ok) {
-          // ---- level 0: global-aligned 16-byte chunks of this lane's row
-          const int nseg = nrow * g.W;
+      } else {
+        uint8_t* p1 = gb + g.off_p1 + 16 * (32 * q + lane) * g.chunks1;   // per piece: 4 words of level 1, then 2 of level 2
+        uint8_t* p2 = gb + g.off_p2 + 16 * (32 * q + lane) * g.chunks2;   // per piece: 2 words of level 2, then 1 of level 3
+        const CvShare sh1(g.W1), sh2(g.W2), sh3(g.W3);
+        const int HW1 = g.H1 * g.W1, HW2 = g.H2 * g.W2, HW3 = g.H3 * g.W3;
+        uint4 tail1 = make_uint4(0, 0, 0, 0), tail2 = tail1, tail3 = tail1;
+        for (int i = i0; i < i1; i += 2) {
+          const bool two = i + 1 < i1;
+          const int j = i >> 1, j2 = i >> 2, j3 = i >> 3;
+          const uint32_t ra = reg;
+          if (!(ok = wait_row(reg, par))) break;
+          next_row();
+          const uint32_t rb = reg;
+          if (two) {
+            if (!(ok = wait_row(reg, par))) break;
+            next_row();
+          }
+          const bool live = two && g.levels > 1 && g.W1 > 0;
+          int64_t g0 = px0 * HW1 + (int64_t)j * g.W1;
+          if (live) {
+            CvAppend ap(row, tail1, ((int)(g0 & 7) + lane * HW1) & 7, g.W1);
+            for (int pc = 0; pc < np; ++pc) {
+              uint32_t va[16], vb[16], a[8], b[8], w[4];
+              load(ra, pc, va);
+              load(rb, pc, vb);
+              tc::ld_wait();
+              pack(va, i, pc, a);
+              pack(vb, i + 1, pc, b);
+#pragma unroll
+              for (int k = 0; k < 4; ++k)
+                w[k] = pack2<T>(pool4<T>(a[2 * k], b[2 * k]), pool4<T>(a[2 * k + 1], b[2 * k + 1]));
+              uint4* up = reinterpret_cast<uint4*>(p1) + pc;
+              if (j & 1) {                                        // with the row above: two words of level 2
+                const uint4 t = *up;
+                *reinterpret_cast<uint2*>(up) = make_uint2(pack2<T>(pool4<T>(t.x, w[0]), pool4<T>(t.y, w[1])),
+                                                           pack2<T>(pool4<T>(t.z, w[2]), pool4<T>(t.w, w[3])));
+              } else {
+                *up = make_uint4(w[0], w[1], w[2], w[3]);
+              }
+              ap.put(w);
+            }
+            ap.end();
+          }
+          tc::fence_before();
+          __syncwarp();
+          free_row(ra);
+          if (two) free_row(rb);
+          if (!live) continue;
+          tail1 = run_flush(sh1, out.lvl[1], g0, HW1, g.W1, (j - (i0 >> 1)) * g.W1, j == (i1 >> 1) - 1, rows, chunks, stg);
+          if (!(j & 1) || g.levels < 3 || g.W2 == 0) continue;
+          g0 = px0 * HW2 + (int64_t)j2 * g.W2;
           {
-            const int m = m0 + prow;
-            if (m < g.HW) {
-              const int64_t G0 = (e * g.HW + m) * (int64_t)g.HW + (int64_t)(2 * j) * g.W;
-              const int off = (int)(G0 & 7);
-              const int nch = (off + nseg + 7) >> 3;
-              uint16_t* gb0 = out.lvl[0] + (G0 - off);
-              const uint16_t* sr = stg + prow * g.SST;
-              for (int k = pb; k < nch; k += kChunkLanes) {
-                const int c0 = 8 * k - off;
-                if (c0 >= 0 && c0 + 8 <= nseg) {
-                  uint32_t wv[4];
-#pragma unroll
-                  for (int i = 0; i < 4; ++i) wv[i] = (uint32_t)sr[c0 + 2 * i] | ((uint32_t)sr[c0 + 2 * i + 1] << 16);
-                  *reinterpret_cast<uint4*>(gb0 + 8 * k) = make_uint4(wv[0], wv[1], wv[2], wv[3]);
-                } else {
-#pragma unroll
-                  for (int i = 0; i < 8; ++i) {
-                    const int c = c0 + i;
-                    if (c >= 0 && c < nseg) gb0[8 * k + i] = sr[c];
-                  }
-                }
+            CvAppend ap(row, tail2, ((int)(g0 & 7) + lane * HW2) & 7, g.W2);
+            for (int pc = 0; pc < np; ++pc) {
+              const uint2 t = *reinterpret_cast<const uint2*>(reinterpret_cast<const uint4*>(p1) + pc);
+              const uint32_t w[2] = {t.x, t.y};
+              uint2* up = reinterpret_cast<uint2*>(p2) + pc;
+              if (j2 & 1) {                                       // with the row above: a word of level 3
+                const uint2 o = *up;
+                *reinterpret_cast<uint32_t*>(up) = pack2<T>(pool4<T>(o.x, w[0]), pool4<T>(o.y, w[1]));
+              } else {
+                *up = t;
               }
+              ap.put(w);
             }
+            ap.end();
           }
-          // ---- levels 1-3: rows 16 ew .. 16 ew + 15, lanes over x
-          if (g.levels > 1 && j < g.H1) {
-            uint16_t* r1 = ring1 + (j & 1) * 128 * R1;
-            const int rbase = kCvRowsPerWarp * ew;
-            // items (row, x) of the warp's rows, lane-strided, stepped without division
-            int a2 = 0, x = lane;
-            while (x >= g.W1) { x -= g.W1; ++a2; }
-            for (; a2 < kCvRowsPerWarp;) {
-              const int rr = rbase + a2;
-              const uint16_t* sr = stg + rr * g.SST;
-              const uint16_t pv = pool4<T>(sr[2 * x], sr[2 * x + 1], sr[g.W + 2 * x], sr[g.W + 2 * x + 1]);
-              r1[rr * R1 + x] = pv;
-              if (m0 + rr < g.HW) out.lvl[1][(e * g.HW + m0 + rr) * L1n + (int64_t)j * g.W1 + x] = pv;
-              x += 32;
-              while (x >= g.W1) { x -= g.W1; ++a2; }
+          tail2 = run_flush(sh2, out.lvl[2], g0, HW2, g.W2, (j2 - (i0 >> 2)) * g.W2, j2 == (i1 >> 2) - 1, rows, chunks, stg);
+          if (!(j2 & 1) || g.levels < 4 || g.W3 == 0) continue;
+          g0 = px0 * HW3 + (int64_t)j3 * g.W3;
+          {
+            CvAppend ap(row, tail3, ((int)(g0 & 7) + lane * HW3) & 7, g.W3);
+            for (int pc = 0; pc < np; ++pc) {
+              const uint32_t w[1] = {*reinterpret_cast<const uint32_t*>(reinterpret_cast<const uint2*>(p2) + pc)};
+              ap.put(w);
             }
-            __syncwarp();
-            const int j2 = j >> 1;
-            if (g.levels > 2 && (j & 1) && j2 < g.H2) {
-              uint16_t* r2 = ring2 + (j2 & 1) * 128 * R2;
-              a2 = 0;
-              x = lane;
-              while (x >= g.W2) { x -= g.W2; ++a2; }
-              for (; a2 < kCvRowsPerWarp;) {
-                const int rr = rbase + a2;
-                const uint16_t* p0 = ring1 + rr * R1;              // level-1 row j-1 (slot 0)
-                const uint16_t* p1 = ring1 + 128 * R1 + rr * R1;   // level-1 row j (slot 1)
-                const uint16_t pv = pool4<T>(p0[2 * x], p0[2 * x + 1], p1[2 * x], p1[2 * x + 1]);
-                r2[rr * R2 + x] = pv;
-                if (m0 + rr < g.HW) out.lvl[2][(e * g.HW + m0 + rr) * L2n + (int64_t)j2 * g.W2 + x] = pv;
-                x += 32;
-                while (x >= g.W2) { x -= g.W2; ++a2; }
-              }
-              __syncwarp();
-              const int j3 = j2 >> 1;
-              if (g.levels > 3 && (j2 & 1) && j3 < g.H3) {
-                a2 = 0;
-                x = lane;
-                while (x >= g.W3) { x -= g.W3; ++a2; }
-                for (; a2 < kCvRowsPerWarp;) {
-                  const int rr = rbase + a2;
-                  const uint16_t* p0 = ring2 + rr * R2;
-                  const uint16_t* p1 = ring2 + 128 * R2 + rr * R2;
-                  const uint16_t pv = pool4<T>(p0[2 * x], p0[2 * x + 1], p1[2 * x], p1[2 * x + 1]);
-                  if (m0 + rr < g.HW) out.lvl[3][(e * g.HW + m0 + rr) * L3n + (int64_t)j3 * g.W3 + x] = pv;
-                  x += 32;
-                  while (x >= g.W3) { x -= g.W3; ++a2; }
-                }
-              }
-            }
+            ap.end();
           }
+          tail3 = run_flush(sh3, out.lvl[3], g0, HW3, g.W3, (j3 - (i0 >> 3)) * g.W3, j3 == (i1 >> 3) - 1, rows, chunks, stg);
         }
-        epi_sync();                          // the staging tile is rewritten by the next tile
-        if (!ok) break;
       }
       if (!ok) break;
     }
@@ -577,6 +711,8 @@ int cv_launch(const CvGeom& g, void* rows1, void* rows2, const float* s1, const 
   int rc;
   if ((rc = cv_map(&amap, rows1, K1, g.HW, P, 128))) return rc;
   if ((rc = cv_map(&bmap, rows2, K2, g.HW, P, g.RW))) return rc;
+  const int64_t units = g.E * g.mtiles * g.splits;
+  if (units == 0) return HS2_OK;
   static DeviceOnce once;
   int dev = 0;
   HS2_CUDA(cudaGetDevice(&dev));
@@ -590,9 +726,7 @@ int cv_launch(const CvGeom& g, void* rows1, void* rows2, const float* s1, const 
     return HS2_OK;
   });
   if (rc) return rc;
-  const int64_t units = g.E * g.mtiles;
-  if (units == 0) return HS2_OK;
-  const int grid = (int)std::min<int64_t>(units, sms[dev].load());
+  const int grid = (int)std::min<int64_t>(units, 2 * sms[dev].load());
   HS2_PROF("corr_volume", s);
   corr_volume_kernel<P, T><<<grid, kCvThreads, g.smem, s>>>(amap, bmap, ii, jj, K1, K2, s1, s2, g, out, info);
   HS2_LAUNCH_CHECK("corr_volume_kernel");
