@@ -870,3 +870,37 @@ def altcorr_backward(fmap1, fmap2, coords, ii, jj, grad, radius, scale=1.0):
                                         _ptr(info), _ptr(ws), nbytes.value, _stream(fmap1.device)),
                "altcorr_backward")
     return [g1, g2]
+
+
+def corr_lookup_backward_fits(fmap1, radius, levels):
+    """Whether :func:`corr_lookup_backward` takes features [N,C,H,W] like fmap1 at this radius and depth."""
+    n, c, h, w = fmap1.shape
+    return (c == 128 and 0 <= radius <= 6 and 1 <= levels <= 4 and 0 < n <= 65535 and h >> (levels - 1) > 0
+            and w >> (levels - 1) > 0 and h * w <= 1 << 24
+            and fmap1.dtype in (torch.float32, torch.float16, torch.bfloat16))
+
+
+def corr_lookup_backward(fmap1, fmap2, coords, grad, radius, levels):
+    """Gradients of the CorrBlock lookup w.r.t. both feature maps [N,C,H,W], for the output gradient
+    ``grad`` [N, L*(2r+1)^2, H, W] at ``coords`` [N,H,W,2] (all contiguous, grad of the features' dtype)."""
+    for name, t in (("fmap1", fmap1), ("fmap2", fmap2), ("coords", coords), ("grad", grad)):
+        _contig(name, t)
+        _cuda(name, t, fmap1.device)
+    _dtype("fmap2", fmap2, fmap1.dtype)
+    _dtype("grad", grad, fmap1.dtype)
+    _dtype("coords", coords, torch.float32)
+    n, c, h, w = fmap1.shape
+    r, L = int(radius), int(levels)
+    if fmap2.shape != fmap1.shape or tuple(coords.shape) != (n, h, w, 2) \
+            or tuple(grad.shape) != (n, L * (2 * r + 1) ** 2, h, w):
+        raise RuntimeError("corr_lookup_backward: inconsistent shapes fmap1 %s fmap2 %s coords %s grad %s" % (
+            tuple(fmap1.shape), tuple(fmap2.shape), tuple(coords.shape), tuple(grad.shape)))
+    dt, lib, nbytes = _DTYPES[fmap1.dtype], _lib.load(), ctypes.c_size_t(0)
+    _lib.check(lib.hs2_corr_lookup_backward_workspace_size(dt, n, c, h, w, L, r, ctypes.byref(nbytes)),
+               "corr_lookup_backward_workspace_size")
+    ws = torch.empty(nbytes.value, dtype=torch.uint8, device=fmap1.device)
+    g1, g2 = torch.empty_like(fmap1), torch.empty_like(fmap2)
+    _lib.check(lib.hs2_corr_lookup_backward(_ptr(fmap1), _ptr(fmap2), dt, n, c, h, w, _ptr(coords), _ptr(grad), L, r,
+                                            1.0 / 16.0, _ptr(g1), _ptr(g2), _ptr(ws), nbytes.value,
+                                            _stream(fmap1.device)), "corr_lookup_backward")
+    return g1, g2

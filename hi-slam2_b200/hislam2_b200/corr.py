@@ -17,9 +17,10 @@
 * :class:`CorrLookup` is the differentiable lookup of the CorrBlock pyramid with
   respect to the feature maps that stores no pyramid: forward builds the levels
   with ``corr_volume`` and samples them; backward recomputes the pooled feature
-  pyramid of ``fmap2`` and applies the on-the-fly correlation adjoint
-  (``altcorr_backward``), which equals the pyramid lookup's adjoint because the
-  pooled volume is the correlation with the pooled features.
+  pyramid of ``fmap2`` and applies the on-the-fly correlation adjoint at every level
+  (``corr_lookup_backward`` in one pass, or ``altcorr_backward`` per level), which equals
+  the pyramid lookup's adjoint because the pooled volume is the correlation with the
+  pooled features.
 """
 
 import torch
@@ -189,6 +190,12 @@ class CorrLookup(torch.autograd.Function):
         r, L = ctx.radius, ctx.num_levels
         B, N, C, H, W = fmap1.shape
         BN = B * N
+        if backends.corr_lookup_backward_fits(fmap1.reshape(BN, C, H, W), r, L) and grad.dtype == fmap1.dtype \
+                and fmap2.dtype == fmap1.dtype and fmap2.shape == fmap1.shape and coords.dtype == torch.float32:
+            flat = [fmap1.reshape(BN, C, H, W), fmap2.reshape(BN, C, H, W), coords.reshape(BN, H, W, 2),
+                    grad.reshape(BN, -1, H, W)]
+            g1, g2 = backends.corr_lookup_backward(*[t.contiguous() for t in flat], r, L)
+            return g1.view(fmap1.shape), g2.view(fmap2.shape), None, None, None
         f1 = fmap1.reshape(1, BN, C, H, W).float().contiguous()
         with torch.enable_grad():
             f2 = fmap2.reshape(BN, C, H, W).float().detach().requires_grad_(True)

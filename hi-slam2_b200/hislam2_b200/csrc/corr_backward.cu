@@ -357,6 +357,24 @@ corr_bwd_pack_kernel(const T* __restrict__ src, float* __restrict__ dst, float* 
   }
 }
 
+// 2x2 average of a channel-last level (rows of 128 floats), as avg_pool2d sums it; the level's
+// gradient accumulator is zeroed.  One warp per output position.
+__global__ void __launch_bounds__(256)
+corr_bwd_pool_kernel(const float* __restrict__ src, float* __restrict__ dst, float* __restrict__ acc, int H, int W,
+                     int64_t total) {
+  const int H2 = H >> 1, W2 = W >> 1, lane = threadIdx.x & 31;
+  const int64_t at = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (at >= total) return;
+  const int64_t n = at / (H2 * W2);
+  const int rem = (int)(at - n * (H2 * W2)), y = rem / W2, x = rem - y * W2;
+  const float4* s = reinterpret_cast<const float4*>(src) + ((n * H + 2 * y) * W + 2 * x) * 32 + lane;
+  const float4 a = s[0], b = s[32], c = s[(int64_t)W * 32], d = s[(int64_t)W * 32 + 32];
+  reinterpret_cast<float4*>(dst)[at * 32 + lane] =
+      make_float4((a.x + b.x + c.x + d.x) * 0.25f, (a.y + b.y + c.y + d.y) * 0.25f, (a.z + b.z + c.z + d.z) * 0.25f,
+                  (a.w + b.w + c.w + d.w) * 0.25f);
+  reinterpret_cast<float4*>(acc)[at * 32 + lane] = make_float4(0.f, 0.f, 0.f, 0.f);
+}
+
 // FP32 channel-last accumulators -> channel-first gradients of T; frames out of use give 0.
 // With levels > 1 the gradients of the 2x2-averaged levels come back to their pixels (a
 // quarter of the level above's, which holds a quarter of the next).
@@ -477,6 +495,83 @@ int altcorr_bwd_tiled_t(const void* fmap1, const void* fmap2, int b, int n1, int
   return cb_unpack<T>(u, g2, flags + n1, b, n2, s);
 }
 
+// Workspace of the lookup's backward: packed fmap1 and its accumulator, then per level the packed
+// (pooled) fmap2 and its accumulator, then the non-finite flag.
+struct ClLayout {
+  size_t f1, o1, f2[4], o2[4], flag, total;
+};
+ClLayout cl_layout(int64_t n, int h, int w, int levels) {
+  ClLayout L{};
+  size_t o = 0;
+  auto take = [&](size_t bytes) { const size_t at = o; o += up256(bytes); return at; };
+  const size_t row = kCbC * 4;
+  L.f1 = take(n * h * w * row);
+  L.o1 = take(n * h * w * row);
+  for (int l = 0; l < levels; ++l) {
+    L.f2[l] = take(n * (h >> l) * (w >> l) * row);
+    L.o2[l] = take(n * (h >> l) * (w >> l) * row);
+  }
+  L.flag = take(256);
+  L.total = o;
+  return L;
+}
+
+template <typename T>
+int corr_lookup_bwd_t(const void* fmap1, const void* fmap2, int n, int h, int w, const float* coords, const void* grad,
+                      int levels, int radius, float scale, void* g1, void* g2, char* ws, cudaStream_t s) {
+  const ClLayout L = cl_layout(n, h, w, levels);
+  auto at = [&](size_t o) { return reinterpret_cast<float*>(ws + o); };
+  int32_t* bad = reinterpret_cast<int32_t*>(ws + L.flag);
+  HS2_CUDA(cudaMemsetAsync(bad, 0, sizeof(int32_t), s));
+  int rc;
+  if ((rc = cb_pack<T>(fmap1, at(L.f1), nullptr, nullptr, 1, n, h * w, bad, s))) return rc;
+  if ((rc = cb_pack<T>(fmap2, at(L.f2[0]), at(L.o2[0]), nullptr, 1, n, h * w, bad, s))) return rc;
+  for (int l = 1; l < levels; ++l) {
+    const int64_t total = (int64_t)n * (h >> l) * (w >> l);
+    HS2_PROF("corr_bwd_pool", s);
+    corr_bwd_pool_kernel<<<(unsigned)((total + 7) / 8), 256, 0, s>>>(at(L.f2[l - 1]), at(L.f2[l]), at(L.o2[l]),
+                                                                   h >> (l - 1), w >> (l - 1), total);
+    HS2_LAUNCH_CHECK("corr_bwd_pool_kernel");
+  }
+  CbArgs a{};
+  a.f1 = at(L.f1);
+  a.o1 = at(L.o1);
+  a.coords = coords;
+  a.interleaved = 1;
+  a.grad = grad;
+  a.N1 = a.N2 = a.M = n, a.H = h, a.W = w, a.r = radius, a.levels = levels, a.cap = cb_cap(radius);
+  a.scale = scale;
+  a.nonfinite = bad;
+  CbUnpack u{};
+  u.levels = levels;
+  for (int l = 0; l < levels; ++l) {
+    a.f2[l] = at(L.f2[l]);
+    a.o2[l] = at(L.o2[l]);
+    a.H2[l] = u.H[l] = h >> l;
+    a.W2[l] = u.W[l] = w >> l;
+    u.acc[l] = at(L.o2[l]);
+  }
+  if ((rc = cb_tile<T, false>(a, 1, s))) return rc;
+  if ((rc = cb_unpack<T>(u, g2, nullptr, 1, n, s))) return rc;
+  u.levels = 1;
+  u.acc[0] = at(L.o1);
+  return cb_unpack<T>(u, g1, nullptr, 1, n, s);
+}
+
+int cl_check(int dtype, int n, int c, int h, int w, int levels, int radius) {
+  if (dtype != HS2_F32 && dtype != HS2_F16 && dtype != HS2_BF16) {
+    set_error("corr_lookup_backward: unsupported dtype %d (f32, f16, bf16)", dtype);
+    return HS2_ERR_DTYPE;
+  }
+  if (n < 0 || n > 65535 || c != kCbC || h <= 0 || w <= 0 || levels < 1 || levels > 4 || (h >> (levels - 1)) < 1 ||
+      (w >> (levels - 1)) < 1 || radius < 0 || radius > kCbMaxRadius || (int64_t)h * w > (1 << 24)) {
+    set_error("corr_lookup_backward: bad sizes n=%d c=%d h=%d w=%d levels=%d r=%d (128 channels, 1 to 4 levels, "
+              "radius <= %d)", n, c, h, w, levels, radius, kCbMaxRadius);
+    return HS2_ERR_INVALID;
+  }
+  return HS2_OK;
+}
+
 }  // namespace
 
 bool altcorr_bwd_tiled_ok(int b, int n1, int n2, int c, int m, int radius) {
@@ -505,3 +600,44 @@ int altcorr_bwd_tiled(int dtype, const void* fmap1, const void* fmap2, int b, in
 }
 
 }  // namespace hs2
+
+extern "C" int hs2_corr_lookup_backward_workspace_size(int dtype, int n, int c, int h, int w, int levels, int radius,
+                                                       size_t* bytes) {
+  using namespace hs2;
+  if (!bytes) {
+    set_error("corr_lookup_backward_workspace_size: null output");
+    return HS2_ERR_INVALID;
+  }
+  const int rc = cl_check(dtype, n, c, h, w, levels, radius);
+  if (rc) return rc;
+  *bytes = cl_layout(n, h, w, levels).total;
+  return HS2_OK;
+}
+
+extern "C" int hs2_corr_lookup_backward(const void* fmap1, const void* fmap2, int dtype, int n, int c, int h, int w,
+                                        const float* coords, const void* grad, int levels, int radius, float scale,
+                                        void* fmap1_grad, void* fmap2_grad, void* workspace, size_t workspace_bytes,
+                                        hs2_stream_t stream) {
+  using namespace hs2;
+  int rc = cl_check(dtype, n, c, h, w, levels, radius);
+  if (rc) return rc;
+  if (n == 0) return HS2_OK;
+  if (!fmap1 || !fmap2 || !coords || !grad || !fmap1_grad || !fmap2_grad) {
+    set_error("corr_lookup_backward: null pointer argument");
+    return HS2_ERR_INVALID;
+  }
+  const size_t need = cl_layout(n, h, w, levels).total;
+  if (!workspace || workspace_bytes < need) {
+    set_error("corr_lookup_backward: workspace of %zu bytes required", need);
+    return HS2_ERR_WORKSPACE;
+  }
+  if ((rc = bind_device(fmap1_grad))) return rc;
+  cudaStream_t s = (cudaStream_t)stream;
+  char* ws = static_cast<char*>(workspace);
+  if (dtype == HS2_F32)
+    return corr_lookup_bwd_t<float>(fmap1, fmap2, n, h, w, coords, grad, levels, radius, scale, fmap1_grad, fmap2_grad, ws, s);
+  if (dtype == HS2_F16)
+    return corr_lookup_bwd_t<__half>(fmap1, fmap2, n, h, w, coords, grad, levels, radius, scale, fmap1_grad, fmap2_grad, ws, s);
+  return corr_lookup_bwd_t<__nv_bfloat16>(fmap1, fmap2, n, h, w, coords, grad, levels, radius, scale, fmap1_grad, fmap2_grad,
+                                          ws, s);
+}

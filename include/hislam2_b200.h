@@ -265,6 +265,21 @@ int hs2_altcorr_backward(const void* fmap1, const void* fmap2, int dtype, int b,
                          void* fmap1_grad, void* fmap2_grad, int32_t* info, void* workspace,
                          size_t workspace_bytes, hs2_stream_t stream);
 
+/* corr_lookup_backward: gradients of the CorrBlock lookup w.r.t. both feature maps without a stored
+ *   pyramid (the adjoint of hs2_corr_volume + hs2_corr_pyramid_forward; reference: hislam2/modules/
+ *   corr.py:23-71, differentiated by autograd through the volume there).
+ *   fmap1, fmap2 [n,c,h,w] of `dtype` (f32, f16, bf16; c = 128): pair k correlates fmap1[k] with
+ *   fmap2[k]; coords [n,h,w,2] f32; grad [n, levels*(2r+1)^2, h, w] of `dtype`; scale multiplies every
+ *   product (1/16 for the lookup's own scaling); 1 to 4 levels, radius <= 6
+ *   -> fmap1_grad, fmap2_grad [n,c,h,w] of `dtype`, fully written; accumulated in f32.
+ */
+int hs2_corr_lookup_backward_workspace_size(int dtype, int n, int c, int h, int w, int levels, int radius,
+                                            size_t* bytes);
+int hs2_corr_lookup_backward(const void* fmap1, const void* fmap2, int dtype, int n, int c, int h, int w,
+                             const float* coords, const void* grad, int levels, int radius, float scale,
+                             void* fmap1_grad, void* fmap2_grad, void* workspace, size_t workspace_bytes,
+                             hs2_stream_t stream);
+
 /* ---------------------------------------------------------------------------
  * ba  (reference: src/droid.cpp:141-168, src/droid_kernels.cu:1820-1937)
  *   Runs `iterations` damped Gauss-Newton steps over the poses [t0,t1) and the
