@@ -1530,16 +1530,17 @@ __device__ __forceinline__ void dmma_m8n8k4(double& d0, double& d1, double a, do
 // identity outside nsb.  Columns j, j+1 (and b_j, b_j+1) are exchanged through a double-
 // buffered 2 x 36 shared array, one __syncwarp per block step.  Writes L (lower part),
 // the multipliers M_rj = L_rj / L_jj above the diagonal (row j), 1/L_jj to sv and y to bv.
-__device__ __forceinline__ void chol_factor_diag(double (*Pm)[kPLD], double* bv, double* sv, double* xc, int c0,
-                                                 int nsb, int* sfail) {
+// at(r, k) is the sub-block's entry, bv and sv its right-hand side and reciprocal pivots.
+template <typename At>
+__device__ __forceinline__ void chol_factor_diag(At at, double* bv, double* sv, double* xc, int nsb, int* sfail) {
   const int lane = threadIdx.x & 31, rr = lane & 15, hh = lane >> 4;
   double a[8];
 #pragma unroll
   for (int q = 0; q < 8; ++q) {
     const int k = 8 * hh + q;
-    a[q] = (rr < nsb && k < nsb) ? Pm[c0 + rr][c0 + k] : (rr == k ? 1.0 : 0.0);
+    a[q] = (rr < nsb && k < nsb) ? at(rr, k) : (rr == k ? 1.0 : 0.0);
   }
-  double bb = (hh == 0 && rr < nsb) ? bv[c0 + rr] : 0.0;
+  double bb = (hh == 0 && rr < nsb) ? bv[rr] : 0.0;
   double cfac = 1.0;
   // per own column k = 8 hh + q: cd_k and f_k; for the own row: cd, f and b' at its step
   double cq[8], fq[8], my_cd = 1.0, my_f = 1.0, my_b = 0.0;
@@ -1608,14 +1609,14 @@ __device__ __forceinline__ void chol_factor_diag(double (*Pm)[kPLD], double* bv,
       if (k <= rr) {
         const double s = rsqrt(cq[q]);
         const double l = a[q] * s;
-        Pm[c0 + rr][c0 + k] = l;
-        if (k < rr) Pm[c0 + k][c0 + rr] = l * (fq[q] * s);
+        at(rr, k) = l;
+        if (k < rr) at(k, rr) = l * (fq[q] * s);
       }
     }
     if (hh == 0) {
       const double s = rsqrt(my_cd);
-      sv[c0 + rr] = my_f * s;
-      bv[c0 + rr] = my_b * s;
+      sv[rr] = my_f * s;
+      bv[rr] = my_b * s;
     }
   }
   if (lane == 0 && !ok) *sfail = 1;
@@ -1696,7 +1697,8 @@ __device__ bool chol_panel(int n, int kb, int t, int xh, double* __restrict__ A,
       __syncthreads();
     }
     // (b)
-    if (tid < 32) chol_factor_diag(Pm, bv, sv, xc, c0, c1 - c0, sfail);
+    if (tid < 32)
+      chol_factor_diag([&](int r, int k) -> double& { return Pm[c0 + r][c0 + k]; }, bv + c0, sv + c0, xc, c1 - c0, sfail);
     __syncthreads();
     if (*sfail) {
       if (tid == 0) atomicExch(cb.ctl + 2, 1u);
@@ -2045,6 +2047,235 @@ ba_cholesky_kernel(int n, float lm, float ep, BaPtrs w, CholBuf cb, float* __res
   if (blockIdx.x == 0 && tid == 0) atomicAdd(&info[2], 1);
 }
 
+// ---------------------------------------------------- cholesky, one CTA ---
+// The same damped FP64 factorisation and solve for systems of at most kSmallMax unknowns, by one
+// CTA with the whole lower triangle in shared memory as 16x16 blocks (padded with identity
+// rows): no counters, barriers across CTAs or round trips through L2 between the steps.
+// Step k: (1) every row below solves its 16 entries against the factored diagonal block and
+// updates its right-hand side, one thread per row; (2) warp 0 applies column k to the next
+// diagonal block (FP64 MMA) and factors it, while the other warps apply column k to the rest
+// of the trailing blocks and form L_kk^-1 (in place: L_kk itself is not used again).  The
+// back-solve then takes one 16x16 mat-vec and one update of the remaining right-hand side per
+// block.  Entries (r, c) of a block sit at column c ^ 2 (r mod 8): pairs stay aligned, and
+// neither a column nor an MMA fragment meets a bank conflict beyond its size.
+// Bound by the chain factor (3.0k cycles) + row solve (1.8k) + diagonal update per 16 columns.
+// Measured with its launch (one / many CTAs): 20 / 33 us at 36 unknowns, 31 / 78 at 96, 45 / 115
+// at 138, 69 / 134 at 180; from there the one SM's FP64 rate adds up: 90 / 125 at 222.
+constexpr int kSmallMax = 224;
+constexpr int kSmallThreads = 512;
+__host__ __device__ constexpr size_t small_smem(int nb) {
+  return sizeof(double) * ((size_t)nb * (nb + 1) / 2 * 256 + 3 * (size_t)nb * 16 + 72 + 16 * 16);
+}
+
+__device__ __forceinline__ int small_at(int I, int J, int r, int c) {
+  return (I * (I + 1) / 2 + J) * 256 + r * 16 + (c ^ (2 * (r & 7)));
+}
+
+__global__ void __launch_bounds__(kSmallThreads, 1)
+ba_solve_small_kernel(int n, float lm, float ep, BaPtrs w, float* __restrict__ dx_out, int32_t* __restrict__ info) {
+  if (info[0]) return;
+  extern __shared__ __align__(16) double ssm[];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int nb = (n + 15) / 16, N = nb * 16;
+  double* S = ssm;                               // blocks
+  double* bv = S + nb * (nb + 1) / 2 * 256;      // [N] right-hand side, then y, then x
+  double* sv = bv + N;                           // [N] 1 / L_jj
+  double* xv = sv + N;                           // [N] solution
+  double* xc = xv + N;                           // [72] column exchange of the factor
+  double* part = xc + 72;                        // [16][16]
+  __shared__ int sfail;
+  // entries (r, c) and (r, c + 1) of the damped, padded system
+  auto entry2 = [&](int r, int c) {
+    double2 v = make_double2(r == c ? 1.0 : 0.0, r == c + 1 ? 1.0 : 0.0);
+    if (r < n && c < n) {                        // n is even: a pair never leaves the row
+      v = ldcg2(w.A + (int64_t)r * n + c);
+      if (r == c) v.x += (double)ep + (double)lm * v.x;
+      if (r == c + 1) v.y += (double)ep + (double)lm * v.y;
+    }
+    return v;
+  };
+  if (tid == 0) sfail = 0;
+  if (warp == 0) {                               // the first diagonal block and the right-hand side
+    double2 v[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) v[q] = entry2((lane >> 3) + 4 * q, (lane & 7) * 2);
+    for (int i = lane; i < N; i += 32) bv[i] = i < n ? __ldcg(w.b + i) : 0.0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      *reinterpret_cast<double2*>(&S[small_at(0, 0, (lane >> 3) + 4 * q, (lane & 7) * 2)]) = v[q];
+    __syncwarp();
+  } else {                                       // the other blocks, a warp per block, under the first factor
+    for (int blk = warp; blk < nb * (nb + 1) / 2; blk += kSmallThreads / 32 - 1) {
+      int I = (int)((sqrtf(8.f * blk + 1.f) - 1.f) * 0.5f);
+      while (I * (I + 1) / 2 > blk) --I;
+      while ((I + 1) * (I + 2) / 2 <= blk) ++I;
+      const int J = blk - I * (I + 1) / 2;
+      double2 v[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) v[q] = entry2(16 * I + (lane >> 3) + 4 * q, 16 * J + (lane & 7) * 2);
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        *reinterpret_cast<double2*>(&S[small_at(I, J, (lane >> 3) + 4 * q, (lane & 7) * 2)]) = v[q];
+    }
+  }
+  auto factor = [&](int k) {
+    chol_factor_diag([&](int r, int c) -> double& { return S[small_at(k, k, r, c)]; }, bv + 16 * k, sv + 16 * k, xc, 16,
+                     &sfail);
+  };
+  // S(I, J) -= X_I X_J^T with X = column block k, by one warp
+  auto update = [&](int I, int J, int k) {
+    double d[2][2][2] = {};
+#pragma unroll
+    for (int k0 = 0; k0 < 16; k0 += 4) {
+      const int r = lane >> 2, c = k0 + (lane & 3);
+      const double a0 = S[small_at(I, k, r, c)], a1 = S[small_at(I, k, r + 8, c)];
+      const double b0 = S[small_at(J, k, r, c)], b1 = S[small_at(J, k, r + 8, c)];
+      dmma_m8n8k4(d[0][0][0], d[0][0][1], a0, b0);
+      dmma_m8n8k4(d[0][1][0], d[0][1][1], a0, b1);
+      dmma_m8n8k4(d[1][0][0], d[1][0][1], a1, b0);
+      dmma_m8n8k4(d[1][1][0], d[1][1][1], a1, b1);
+    }
+#pragma unroll
+    for (int a = 0; a < 2; ++a)
+#pragma unroll
+      for (int b = 0; b < 2; ++b) {
+        double2* p = reinterpret_cast<double2*>(&S[small_at(I, J, 8 * a + (lane >> 2), 8 * b + 2 * (lane & 3))]);
+        double2 v = *p;
+        v.x -= d[a][b][0];
+        v.y -= d[a][b][1];
+        *p = v;
+      }
+  };
+  if (warp == 0) factor(0);
+  __syncthreads();
+  for (int k = 0; k < nb; ++k) {
+    if (sfail) break;
+    const int m = nb - k - 1;
+    // (1) rows below: u_j = v_j - sum_{i<j} u_i M_ij with M above the diagonal of block k, x = u / L_jj
+    for (int t = tid; t < 16 * m; t += kSmallThreads) {
+      const int I = k + 1 + (t >> 4), r = t & 15;
+      double v[16];
+#pragma unroll
+      for (int l = 0; l < 16; l += 2) {
+        const double2 x = *reinterpret_cast<const double2*>(&S[small_at(I, k, r, l)]);
+        v[l] = x.x;
+        v[l + 1] = x.y;
+      }
+#pragma unroll
+      for (int j = 0; j < 15; ++j)
+#pragma unroll
+        for (int l = (j + 1) & ~1; l < 16; l += 2) {
+          const double2 mm = *reinterpret_cast<const double2*>(&S[small_at(k, k, j, l)]);
+          if (l > j) v[l] = fma(-v[j], mm.x, v[l]);
+          v[l + 1] = fma(-v[j], mm.y, v[l + 1]);
+        }
+      double acc = 0.0;
+#pragma unroll
+      for (int l = 0; l < 16; l += 2) {
+        double2 x;
+        x.x = v[l] * sv[16 * k + l];
+        x.y = v[l + 1] * sv[16 * k + l + 1];
+        acc = fma(x.x, bv[16 * k + l], acc);
+        acc = fma(x.y, bv[16 * k + l + 1], acc);
+        *reinterpret_cast<double2*>(&S[small_at(I, k, r, l)]) = x;
+      }
+      bv[16 * I + r] -= acc;
+    }
+    __syncthreads();
+    // (2)
+    if (warp == 0) {
+      if (m > 0) {
+        update(k + 1, k + 1, k);
+        __syncwarp();
+        factor(k + 1);
+      }
+    } else {
+      // task 0: L_kk^-1, lane = column; the others: the trailing blocks but (k + 1, k + 1), column by column
+      for (int t = warp - 1; t < m * (m + 1) / 2; t += kSmallThreads / 32 - 1) {
+        if (t == 0) {
+          double x[16];
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            double acc = 0.0;
+#pragma unroll
+            for (int l = 0; l < 16; ++l)
+              if (l < i) acc = fma(S[small_at(k, k, i, l)], x[l], acc);
+            x[i] = lane == i ? sv[16 * k + i] : (lane < i ? -acc * sv[16 * k + i] : 0.0);
+          }
+          __syncwarp();
+          if (lane < 16) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i)
+              if (lane <= i) S[small_at(k, k, i, lane)] = x[i];
+          }
+          continue;
+        }
+        int J = 0, rem = t;                            // column J holds m - J blocks
+        while (rem >= m - J) {
+          rem -= m - J;
+          ++J;
+        }
+        update(k + 1 + J + rem, k + 1 + J, k);
+      }
+    }
+    __syncthreads();
+  }
+  if (sfail) {
+    for (int i = tid; i < n; i += kSmallThreads) {
+      w.x[i] = 0.0;
+      dx_out[i] = 0.0f;
+    }
+    if (tid == 0) atomicAdd(&info[2], 1);
+    return;
+  }
+  // the last block's inverse has no trailing update to run under
+  if (warp == 0) {
+    const int k = nb - 1;
+    double x[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      double acc = 0.0;
+#pragma unroll
+      for (int l = 0; l < 16; ++l)
+        if (l < i) acc = fma(S[small_at(k, k, i, l)], x[l], acc);
+      x[i] = lane == i ? sv[16 * k + i] : (lane < i ? -acc * sv[16 * k + i] : 0.0);
+    }
+    __syncwarp();
+    if (lane < 16) {
+#pragma unroll
+      for (int i = 0; i < 16; ++i)
+        if (lane <= i) S[small_at(k, k, i, lane)] = x[i];
+    }
+  }
+  __syncthreads();
+  // L^T x = y from the last block: x_k = L_kk^-T y_k, then y_J -= L_kJ^T x_k for the blocks above
+  for (int k = nb - 1; k >= 0; --k) {
+    if (tid < 256) {                                   // x_c = sum_{r >= c} Linv[r][c] y_r, 16 lanes per column
+      const int c = tid >> 4, r = tid & 15;
+      double v = r >= c ? S[small_at(k, k, r, c)] * bv[16 * k + r] : 0.0;
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      if (r == 0) xv[16 * k + c] = v;
+    }
+    __syncthreads();
+    for (int t = tid; t < 16 * k; t += kSmallThreads) {
+      const int J = t >> 4, c = t & 15;
+      double a0 = 0.0, a1 = 0.0;
+#pragma unroll
+      for (int r = 0; r < 16; r += 2) {
+        a0 = fma(S[small_at(k, J, r, c)], xv[16 * k + r], a0);
+        a1 = fma(S[small_at(k, J, r + 1, c)], xv[16 * k + r + 1], a1);
+      }
+      bv[t] -= a0 + a1;
+    }
+    __syncthreads();
+  }
+  for (int i = tid; i < n; i += kSmallThreads) {
+    w.x[i] = xv[i];
+    dx_out[i] = (float)xv[i];
+  }
+}
+
 // -------------------------------------------------------------- backsub ---
 template <int NT, int PPT = kLinPPT>
 __device__ __forceinline__ void ba_backsub_body(int s, int chunk, float* __restrict__ disps, int HW, int P, BaPtrs w,
@@ -2187,6 +2418,22 @@ static int run_cholesky(int n, float lm, float ep, BaPtrs w, CholBuf cb, float* 
                         cudaStream_t s) {
   if (n == 0) return HS2_OK;
   HS2_PROF("ba_cholesky", s);
+  // up to kSmallMax unknowns (the whole triangle fits one CTA's shared memory, and one CTA is still
+  // the faster: 90 us against 125 us at 222) no other CTA takes part
+  if (n <= kSmallMax) {
+    static DeviceOnce small_once;
+    int dev = 0;
+    HS2_CUDA(cudaGetDevice(&dev));
+    const int rc = small_once.run(dev, [&]() -> int {
+      HS2_CUDA(cudaFuncSetAttribute(ba_solve_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)small_smem(kSmallMax / 16)));
+      return HS2_OK;
+    });
+    if (rc) return rc;
+    ba_solve_small_kernel<<<1, kSmallThreads, small_smem((n + 15) / 16), s>>>(n, lm, ep, w, dx, info);
+    HS2_LAUNCH_CHECK("ba_solve_small_kernel");
+    return HS2_OK;
+  }
   const int nbk = (n + kNB - 1) / kNB;
   // panel: [128][kPLD] + b, 1/L_jj, exchange; tile: [192][kPLD]; backward: 2 x 64 x 64 + 256
   const size_t smem = sizeof(double) * std::max<size_t>(128 * kPLD + 128 + 64 + 72 + 2, 192 * kPLD);
