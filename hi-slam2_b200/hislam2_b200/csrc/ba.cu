@@ -1445,8 +1445,8 @@ static int encode_erows_map(CUtensorMap* map, float* erows, int HW, int64_t plan
 // for t == 0; b the right-hand side) and eliminates the 64 columns in four 16-column
 // sub-panels, left-looking: (a) the sub-panel columns receive the updates of the
 // sub-panels left of them, (b) one warp factors the 16x16 diagonal sub-block and
-// its part of b in registers, exchanging columns by shuffles, (c) every row below
-// solves its 16 entries against that sub-block.  Task 0 writes L11, the reciprocal
+// its part of b in registers and forms the inverse, (c) the rows below are multiplied
+// by it.  Task 0 writes L11, the reciprocal
 // pivots and y = L11^-1 b1; the others write L21 and b2 - L21 y1.
 //
 // A non-positive pivot is seen identically by every CTA that factors the panel; the
@@ -1600,9 +1600,10 @@ __device__ __forceinline__ void dmma_m8n8k4(double& d0, double& d1, double a, do
                : "+d"(d0), "+d"(d1) : "d"(a), "d"(b));
 }
 
-// (b) One warp factors the nsb x nsb diagonal sub-block at (c0, c0) in registers,
-// fraction-free with 2 x 2 pivot blocks: with u, v the trailing columns j, j+1, the block
-// P = [p q; q s] and det = p s - q^2, step (j, j+1) replaces the trailing entries by
+// (b) One warp factors the nsb x nsb diagonal sub-block, A = L L^T, in registers and forms
+// L^-T along with it, fraction-free with 2 x 2 pivot blocks: with u, v the trailing columns
+// j, j+1, the block P = [p q; q s] and det = p s - q^2, step (j, j+1) replaces the trailing
+// entries by
 //   (A_rk det - [u_r v_r] adj(P) [u_k v_k]^T) 2^-E,   E the binary exponent of det,
 // so no reciprocal sits on the chain from one pivot block to the next and the exact
 // power-of-two scale keeps the entries in range.  The trailing block is then c times the
@@ -1611,51 +1612,41 @@ __device__ __forceinline__ void dmma_m8n8k4(double& d0, double& d1, double a, do
 // cd = (c p, c p det) and f = (c, c p) for the two columns:
 //   L_rk = num_rk / sqrt(cd_k),   1/L_kk = f_k / sqrt(cd_k),   y_k = b'_k / sqrt(cd_k),
 // num = u_r resp. w_r and b' = b_j resp. p b_j+1 - q b_j.  The products are recorded per
-// column and L is formed after the loop, off the elimination chain.  Lane = row (0..15)
-// + 16 * column half; a lane holds the 8 entries of its row in its half, padded with the
-// identity outside nsb.  Columns j, j+1 (and b_j, b_j+1) are exchanged through a double-
-// buffered 2 x 36 shared array, one __syncwarp per block step.  Writes L (lower part),
-// the multipliers M_rj = L_rj / L_jj above the diagonal (row j), 1/L_jj to sv and y to bv.
-// at(r, k) is the sub-block's entry, bv and sv its right-hand side and reciprocal pivots.
+// column and the square roots taken after the loop, off the elimination chain, one per lane.
+// Lane = row: lanes 0..15 the sub-block's rows, lanes 16..31 the rows of an identity below
+// them, whose elimination leaves I L^-T (the other rows' triangular solves become products
+// with it: (c) took 1.8k cycles as a 15-step substitution; 1740 unknowns 725 -> 677 us).  Columns j, j+1 (and b_j, b_j+1) are
+// exchanged through a double-buffered 2 x 36 shared array, one __syncwarp per block step.
+// Rows and columns outside nsb are those of the identity.  Writes L (lower part), L^-T above
+// the diagonal, 1/L_jj to sv and y to bv.  at(r, k) is the sub-block's entry, bv and sv its
+// right-hand side and reciprocal pivots.
 template <typename At>
 __device__ __forceinline__ void chol_factor_diag(At at, double* bv, double* sv, double* xc, int nsb, int* sfail) {
-  const int lane = threadIdx.x & 31, rr = lane & 15, hh = lane >> 4;
-  double a[8];
+  const int lane = threadIdx.x & 31, rr = lane & 15;
+  const bool own = lane < 16;
+  double a[16];
 #pragma unroll
-  for (int q = 0; q < 8; ++q) {
-    const int k = 8 * hh + q;
-    a[q] = (rr < nsb && k < nsb) ? at(rr, k) : (rr == k ? 1.0 : 0.0);
+  for (int k = 0; k < 16; ++k) a[k] = (own && rr < nsb && k < nsb) ? at(rr, k) : (rr == k ? 1.0 : 0.0);
+  if (own) {   // the sub-block is symmetric: its upper part may hold anything
+#pragma unroll
+    for (int k = 0; k < 16; ++k)
+      if (k > rr) a[k] = 0.0;
   }
-  double bb = (hh == 0 && rr < nsb) ? bv[rr] : 0.0;
-  double cfac = 1.0;
-  // per own column k = 8 hh + q: cd_k and f_k; for the own row: cd, f and b' at its step
-  double cq[8], fq[8], my_cd = 1.0, my_f = 1.0, my_b = 0.0;
-#pragma unroll
-  for (int q = 0; q < 8; ++q) cq[q] = fq[q] = 1.0;
+  double bb = (own && rr < nsb) ? bv[rr] : 0.0;
+  double cfac = 1.0, my_cd = 1.0, my_f = 1.0, my_b = 0.0;
   bool ok = true;
 #pragma unroll
   for (int j = 0; j < 16; j += 2) {
-    const int hj = j >> 3, qj = j & 7;
     double* col = xc + ((j >> 1) & 1) * 36;   // [0,16) u, [16,32) v, [32] b_j, [33] b_j+1
-    if (hh == hj) {
-      col[rr] = a[qj];
-      col[16 + rr] = a[qj + 1];
+    if (own) {
+      col[rr] = a[j];
+      col[16 + rr] = a[j + 1];
     }
     if (lane == j || lane == j + 1) col[32 + lane - j] = bb;
     __syncwarp();
     const double p = col[j], q = col[j + 1], s = col[16 + j + 1];
-    const double ur = col[rr], vr = col[16 + rr];
+    const double ur = a[j], vr = a[j + 1];
     const double2 bjj = *reinterpret_cast<const double2*>(&col[32]);
-    double uk[8], vk[8];
-#pragma unroll
-    for (int t = 0; t < 8; t += 2) {
-      const double2 x = *reinterpret_cast<const double2*>(&col[8 * hh + t]);
-      const double2 y = *reinterpret_cast<const double2*>(&col[16 + 8 * hh + t]);
-      uk[t] = x.x;
-      uk[t + 1] = x.y;
-      vk[t] = y.x;
-      vk[t + 1] = y.y;
-    }
     const double det = fma(p, s, -(q * q));
     ok = ok && (p > 0.0) && (det > 0.0);
     const long long bits = __double_as_longlong(det);
@@ -1663,19 +1654,17 @@ __device__ __forceinline__ void chol_factor_diag(At at, double* bv, double* sv, 
     const double w1 = fma(s, ur, -(q * vr)), w2 = fma(p, vr, -(q * ur));
     const double dets = det * sc, w1s = w1 * sc, w2s = w2 * sc;
 #pragma unroll
-    for (int t = 0; t < 8; ++t)
-      if (8 * hh + t > j + 1) a[t] = fma(a[t], dets, -fma(w1s, uk[t], w2s * vk[t]));
-    const double bj1 = fma(p, bjj.y, -(q * bjj.x));
-    if (hh == 0 && rr > j + 1) bb = fma(bb, dets, -fma(w1s, bjj.x, w2s * bjj.y));
-    // columns j, j+1 are final: only registers are written here
-    const double cp = cfac * p, cpd = cp * det;
-    if (hh == hj) {
-      a[qj + 1] = w2;
-      cq[qj] = cp;
-      fq[qj] = cfac;
-      cq[qj + 1] = cpd;
-      fq[qj + 1] = cp;
+    for (int t = j + 2; t < 16; t += 2) {
+      const double2 u = *reinterpret_cast<const double2*>(&col[t]);
+      const double2 v = *reinterpret_cast<const double2*>(&col[16 + t]);
+      a[t] = fma(a[t], dets, -fma(w1s, u.x, w2s * v.x));
+      a[t + 1] = fma(a[t + 1], dets, -fma(w1s, u.y, w2s * v.y));
     }
+    const double bj1 = fma(p, bjj.y, -(q * bjj.x));
+    if (own && rr > j + 1) bb = fma(bb, dets, -fma(w1s, bjj.x, w2s * bjj.y));
+    // columns j, j+1 are final
+    const double cp = cfac * p, cpd = cp * det;
+    a[j + 1] = w2;
     if (rr == j) {
       my_cd = cp;
       my_f = cfac;
@@ -1688,24 +1677,45 @@ __device__ __forceinline__ void chol_factor_diag(At at, double* bv, double* sv, 
     }
     cfac *= dets;
   }
-  if (rr < nsb) {
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      const int k = 8 * hh + q;
-      if (k <= rr) {
-        const double s = rsqrt(cq[q]);
-        const double l = a[q] * s;
-        at(rr, k) = l;
-        if (k < rr) at(k, rr) = l * (fq[q] * s);
-      }
-    }
-    if (hh == 0) {
-      const double s = rsqrt(my_cd);
+  const double s = rsqrt(my_cd);
+  double* xs = xc;                             // buffer 0: the last step used buffer 1
+  if (own) {
+    xs[rr] = s;
+    if (rr < nsb) {
       sv[rr] = my_f * s;
       bv[rr] = my_b * s;
     }
   }
+  __syncwarp();
+#pragma unroll
+  for (int k = 0; k < 16; k += 2) {
+    const double2 sk = *reinterpret_cast<const double2*>(&xs[k]);
+    if (rr < nsb && k < nsb && (own ? k <= rr : k > rr)) at(rr, k) = a[k] * sk.x;
+    if (rr < nsb && k + 1 < nsb && (own ? k + 1 <= rr : k + 1 > rr)) at(rr, k + 1) = a[k + 1] * sk.y;
+  }
   if (lane == 0 && !ok) *sfail = 1;
+}
+
+// (c) One warp solves eight rows below a factored sub-block, X = A L^-T, on the FP64 tensor
+// cores: row(r, k) is the entry of row r (0..7), tr(l, c) that of L^-T.  In place; lane l is
+// left with X[l / 4][8 h + 2 (l % 4) + {0, 1}] in x[2 h + {0, 1}].
+template <typename Row, typename Tr>
+__device__ __forceinline__ void chol_solve_rows(Row row, Tr tr, double (&x)[4]) {
+  const int lane = threadIdx.x & 31, r = lane >> 2, q = lane & 3;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) x[i] = 0.0;
+#pragma unroll
+  for (int k0 = 0; k0 < 16; k0 += 4) {
+    const double av = row(r, k0 + q);
+    if (k0 < 8) dmma_m8n8k4(x[0], x[1], av, tr(k0 + q, r));   // L^-T is upper: no k >= 8 in columns 0..7
+    dmma_m8n8k4(x[2], x[3], av, tr(k0 + q, 8 + r));
+  }
+  __syncwarp();
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    row(r, 8 * h + 2 * q) = x[2 * h];
+    row(r, 8 * h + 2 * q + 1) = x[2 * h + 1];
+  }
 }
 
 // Panel kb, task t (0: D only; t >= 1: D and the (t-1)-th tile below it).  Returns
@@ -1790,28 +1800,18 @@ __device__ bool chol_panel(int n, int kb, int t, int xh, double* __restrict__ A,
       if (tid == 0) atomicExch(cb.ctl + 2, 1u);
       return false;
     }
-    // (c) rows below the sub-block solve x L_ss^T = v: with u_j = x_j L_jj,
-    // u_j = v_j - sum_{i<j} u_i M_ji (M above the diagonal of the sub-block), x = u / L_jj
-    if (tid < 128) {
-      const int r = tid;
-      if (r >= kNB ? (r - kNB < nr) : (r >= c1 && r < nb)) {
-        double v[16];
-#pragma unroll
-        for (int l = 0; l < 16; ++l) v[l] = c0 + l < c1 ? Pm[r][c0 + l] : 0.0;
-#pragma unroll
-        for (int j = 0; j < 15; ++j) {
-          if (c0 + j < c1) {
-#pragma unroll
-            for (int l = (j + 1) & ~1; l < 16; l += 2) {
-              const double2 m = *reinterpret_cast<const double2*>(&Pm[c0 + j][c0 + l]);
-              if (l > j) v[l] = fma(-v[j], m.x, v[l]);
-              v[l + 1] = fma(-v[j], m.y, v[l + 1]);
-            }
-          }
-        }
-#pragma unroll
-        for (int l = 0; l < 16; ++l)
-          if (c0 + l < c1) Pm[r][c0 + l] = v[l] * sv[c0 + l];
+    // (c) rows below the sub-block: X = A L_ss^-T, eight rows per warp and step
+    {
+      const int warp = tid >> 5;
+      const int td = (nb - c1 + 7) >> 3, tx = (nr + 7) >> 3;   // c1 = c0 + 16 wherever D has rows below
+      for (int tile = warp; tile < td + tx; tile += kCholThreads / 32) {
+        const int rt = tile < td ? c1 + 8 * tile : kNB + 8 * (tile - td);
+        double x[4];
+        chol_solve_rows([&](int r, int k) -> double& { return Pm[rt + r][c0 + k]; },
+                        [&](int l, int c) -> double {
+                          if (l > c) return 0.0;
+                          return l == c ? (c0 + l < c1 ? sv[c0 + l] : 1.0) : Pm[c0 + l][c0 + c];
+                        }, x);
       }
     }
     __syncthreads();
@@ -1858,12 +1858,13 @@ __device__ __forceinline__ void cp_async_wait_all() {
 
 // A[ri + i][rj + j] -= sum_k L[ri + i][o + k] L[rj + j][o + k] over the 16*RG rows
 // at ri and the 64 columns at rj; `diag` keeps only entries on or below the
-// diagonal of A.  Thread (ty, tx) owns rows ty + 16a and columns tx + 16c.  Both L row
+// diagonal of A.  FP64 tensor-core MMA (m8n8k4): the 4x4-per-thread SIMT form read shared
+// memory for half its time (the solve of 1740 unknowns: 677 us with it, 610 us so).  Both L row
 // blocks and the target tile itself arrive by 16-byte cp.async copies issued together
 // (one L2 round trip; rows and columns outside the matrix are zero-filled).
 template <int RG>
 __device__ void chol_update_tile(int n, double* __restrict__ A, int o, int ri, int rj, bool diag, double* csm) {
-  const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
+  const int tid = threadIdx.x;
   const int ni = min(16 * RG, n - ri), nj = min(kNB, n - rj);
   if (ni <= 0) return;
   constexpr int kRows = 16 * RG;
@@ -1903,33 +1904,32 @@ __device__ void chol_update_tile(int n, double* __restrict__ A, int o, int ri, i
     cp_async_wait_all();
   }
   __syncthreads();
-  double acc[RG][4];
+  // warp: an 8-row strip and kT of its 8-column tiles (all eight of a 64-row tile, two of a 16-row
+  // slice); a diagonal tile stops at its strip
+  constexpr int kT = RG == 4 ? 8 : 2;
+  const int lane = tid & 31, warp = tid >> 5, r = lane >> 2, q = lane & 3;
+  const int strip = RG == 4 ? warp : warp & 1, t0 = RG == 4 ? 0 : (warp >> 1) * kT;
+  const int row = ri + 8 * strip;                    // first row of the strip
+  const int nt = diag ? min(kT, (row + 7 - rj - 8 * t0) / 8 + 1) : kT;
+  double acc[kT][2];
 #pragma unroll
-  for (int a = 0; a < RG; ++a)
+  for (int t = 0; t < kT; ++t) acc[t][0] = acc[t][1] = 0.0;
+#pragma unroll 4
+  for (int k = 0; k < kNB; k += 4) {
+    const double av = Ai[8 * strip + r][k + q];
 #pragma unroll
-    for (int c = 0; c < 4; ++c) acc[a][c] = 0.0;
-#pragma unroll 2
-  for (int k = 0; k < kNB; k += 2) {
-    double2 va[RG], vb[4];
-#pragma unroll
-    for (int a = 0; a < RG; ++a) va[a] = *reinterpret_cast<const double2*>(&Ai[ty + 16 * a][k]);
-#pragma unroll
-    for (int c = 0; c < 4; ++c) vb[c] = *reinterpret_cast<const double2*>(&Aj[tx + 16 * c][k]);
-#pragma unroll
-    for (int a = 0; a < RG; ++a)
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        acc[a][c] = fma(va[a].x, vb[c].x, acc[a][c]);
-        acc[a][c] = fma(va[a].y, vb[c].y, acc[a][c]);
-      }
+    for (int t = 0; t < kT; ++t)
+      if (t < nt) dmma_m8n8k4(acc[t][0], acc[t][1], av, Aj[8 * (t0 + t) + r][k + q]);
   }
 #pragma unroll
-  for (int a = 0; a < RG; ++a)
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const int i = ty + 16 * a, j = tx + 16 * c;
-      if (i < ni && j < nj && (!diag || rj + j <= ri + i)) A[(int64_t)(ri + i) * n + rj + j] = Cs[i][j] - acc[a][c];
-    }
+  for (int t = 0; t < kT; ++t) {
+    const int i = 8 * strip + r, j = 8 * (t0 + t) + 2 * q;   // nj is even: a pair never leaves the matrix
+    if (t >= nt || i >= ni || j >= nj || (diag && rj + j > ri + i)) continue;
+    const double2 c = *reinterpret_cast<const double2*>(&Cs[i][j]);
+    double* dst = A + (int64_t)(ri + i) * n + rj + j;
+    if (diag && rj + j + 1 > ri + i) *dst = c.x - acc[t][0];
+    else *reinterpret_cast<double2*>(dst) = make_double2(c.x - acc[t][0], c.y - acc[t][1]);
+  }
 }
 
 // Backward substitution L^T x = y, block c on CTA c mod G (blocks taken from the
@@ -2137,20 +2137,19 @@ ba_cholesky_kernel(int n, float lm, float ep, BaPtrs w, CholBuf cb, float* __res
 // The same damped FP64 factorisation and solve for systems of at most kSmallMax unknowns, by one
 // CTA with the whole lower triangle in shared memory as 16x16 blocks (padded with identity
 // rows): no counters, barriers across CTAs or round trips through L2 between the steps.
-// Step k: (1) every row below solves its 16 entries against the factored diagonal block and
-// updates its right-hand side, one thread per row; (2) warp 0 applies column k to the next
-// diagonal block (FP64 MMA) and factors it, while the other warps apply column k to the rest
-// of the trailing blocks and form L_kk^-1 (in place: L_kk itself is not used again).  The
-// back-solve then takes one 16x16 mat-vec and one update of the remaining right-hand side per
-// block.  Entries (r, c) of a block sit at column c ^ 2 (r mod 8): pairs stay aligned, and
+// Step k: (1) the rows below are multiplied by L_kk^-T (FP64 MMA, eight rows per warp) and
+// update their right-hand side; (2) warp 0 applies column k to the next diagonal block and
+// factors it, while the other warps apply column k to the rest of the trailing blocks.  The
+// back-solve then takes one 16x16 mat-vec with L_kk^-T and one update of the remaining
+// right-hand side per block.  Entries (r, c) of a block sit at column c ^ 2 (r mod 8): pairs stay aligned, and
 // neither a column nor an MMA fragment meets a bank conflict beyond its size.
-// Bound by the chain factor (3.0k cycles) + row solve (1.8k) + diagonal update per 16 columns.
-// Measured with its launch (one / many CTAs): 20 / 33 us at 36 unknowns, 31 / 78 at 96, 45 / 115
-// at 138, 69 / 134 at 180; from there the one SM's FP64 rate adds up: 90 / 125 at 222.
+// Bound by the chain factor + row products + diagonal update per 16 columns.
+// Measured with its launch (one / many CTAs): 17 / 33 us at 36 unknowns, 27 / 78 at 96, 41 / 115
+// at 138, 62 / 125 at 180; from there the one SM's FP64 rate adds up: 82 / 110 at 222.
 constexpr int kSmallMax = 224;
 constexpr int kSmallThreads = 512;
 __host__ __device__ constexpr size_t small_smem(int nb) {
-  return sizeof(double) * ((size_t)nb * (nb + 1) / 2 * 256 + 3 * (size_t)nb * 16 + 72 + 16 * 16);
+  return sizeof(double) * ((size_t)nb * (nb + 1) / 2 * 256 + 3 * (size_t)nb * 16 + 72);
 }
 
 __device__ __forceinline__ int small_at(int I, int J, int r, int c) {
@@ -2168,7 +2167,6 @@ ba_solve_small_kernel(int n, float lm, float ep, BaPtrs w, float* __restrict__ d
   double* sv = bv + N;                           // [N] 1 / L_jj
   double* xv = sv + N;                           // [N] solution
   double* xc = xv + N;                           // [72] column exchange of the factor
-  double* part = xc + 72;                        // [16][16]
   __shared__ int sfail;
   // entries (r, c) and (r, c + 1) of the damped, padded system
   auto entry2 = [&](int r, int c) {
@@ -2237,35 +2235,19 @@ ba_solve_small_kernel(int n, float lm, float ep, BaPtrs w, float* __restrict__ d
   for (int k = 0; k < nb; ++k) {
     if (sfail) break;
     const int m = nb - k - 1;
-    // (1) rows below: u_j = v_j - sum_{i<j} u_i M_ij with M above the diagonal of block k, x = u / L_jj
-    for (int t = tid; t < 16 * m; t += kSmallThreads) {
-      const int I = k + 1 + (t >> 4), r = t & 15;
-      double v[16];
-#pragma unroll
-      for (int l = 0; l < 16; l += 2) {
-        const double2 x = *reinterpret_cast<const double2*>(&S[small_at(I, k, r, l)]);
-        v[l] = x.x;
-        v[l + 1] = x.y;
-      }
-#pragma unroll
-      for (int j = 0; j < 15; ++j)
-#pragma unroll
-        for (int l = (j + 1) & ~1; l < 16; l += 2) {
-          const double2 mm = *reinterpret_cast<const double2*>(&S[small_at(k, k, j, l)]);
-          if (l > j) v[l] = fma(-v[j], mm.x, v[l]);
-          v[l + 1] = fma(-v[j], mm.y, v[l + 1]);
-        }
-      double acc = 0.0;
-#pragma unroll
-      for (int l = 0; l < 16; l += 2) {
-        double2 x;
-        x.x = v[l] * sv[16 * k + l];
-        x.y = v[l + 1] * sv[16 * k + l + 1];
-        acc = fma(x.x, bv[16 * k + l], acc);
-        acc = fma(x.y, bv[16 * k + l + 1], acc);
-        *reinterpret_cast<double2*>(&S[small_at(I, k, r, l)]) = x;
-      }
-      bv[16 * I + r] -= acc;
+    // (1) rows below: X = A L_kk^-T, b -= X y_k
+    for (int t = warp; t < 2 * m; t += kSmallThreads / 32) {
+      const int I = k + 1 + (t >> 1), h0 = 8 * (t & 1);
+      double x[4];
+      chol_solve_rows([&](int r, int c) -> double& { return S[small_at(I, k, h0 + r, c)]; },
+                      [&](int l, int c) -> double {
+                        return l > c ? 0.0 : l == c ? sv[16 * k + l] : S[small_at(k, k, l, c)];
+                      }, x);
+      const double* yk = bv + 16 * k + 2 * (lane & 3);
+      double acc = fma(x[0], yk[0], x[1] * yk[1]) + fma(x[2], yk[8], x[3] * yk[9]);
+      acc += __shfl_xor_sync(0xffffffffu, acc, 1);
+      acc += __shfl_xor_sync(0xffffffffu, acc, 2);
+      if ((lane & 3) == 0) bv[16 * I + h0 + (lane >> 2)] -= acc;
     }
     __syncthreads();
     // (2)
@@ -2275,27 +2257,10 @@ ba_solve_small_kernel(int n, float lm, float ep, BaPtrs w, float* __restrict__ d
         __syncwarp();
         factor(k + 1);
       }
-    } else {
-      // task 0: L_kk^-1, lane = column; the others: the trailing blocks but (k + 1, k + 1), column by column
-      for (int t = warp - 1; t < m * (m + 1) / 2; t += kSmallThreads / 32 - 1) {
-        if (t == 0) {
-          double x[16];
-#pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            double acc = 0.0;
-#pragma unroll
-            for (int l = 0; l < 16; ++l)
-              if (l < i) acc = fma(S[small_at(k, k, i, l)], x[l], acc);
-            x[i] = lane == i ? sv[16 * k + i] : (lane < i ? -acc * sv[16 * k + i] : 0.0);
-          }
-          __syncwarp();
-          if (lane < 16) {
-#pragma unroll
-            for (int i = 0; i < 16; ++i)
-              if (lane <= i) S[small_at(k, k, i, lane)] = x[i];
-          }
-          continue;
-        }
+    } else if (warp & 3) {
+      // the trailing blocks but (k + 1, k + 1), column by column, on the twelve warps that do not share
+      // warp 0's scheduler and FP64 pipe
+      for (int t = (warp >> 2) * 3 + (warp & 3); t < m * (m + 1) / 2; t += kSmallThreads / 32 * 3 / 4) {
         int J = 0, rem = t;                            // column J holds m - J blocks
         while (rem >= m - J) {
           rem -= m - J;
@@ -2314,31 +2279,11 @@ ba_solve_small_kernel(int n, float lm, float ep, BaPtrs w, float* __restrict__ d
     if (tid == 0) atomicAdd(&info[2], 1);
     return;
   }
-  // the last block's inverse has no trailing update to run under
-  if (warp == 0) {
-    const int k = nb - 1;
-    double x[16];
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      double acc = 0.0;
-#pragma unroll
-      for (int l = 0; l < 16; ++l)
-        if (l < i) acc = fma(S[small_at(k, k, i, l)], x[l], acc);
-      x[i] = lane == i ? sv[16 * k + i] : (lane < i ? -acc * sv[16 * k + i] : 0.0);
-    }
-    __syncwarp();
-    if (lane < 16) {
-#pragma unroll
-      for (int i = 0; i < 16; ++i)
-        if (lane <= i) S[small_at(k, k, i, lane)] = x[i];
-    }
-  }
-  __syncthreads();
   // L^T x = y from the last block: x_k = L_kk^-T y_k, then y_J -= L_kJ^T x_k for the blocks above
   for (int k = nb - 1; k >= 0; --k) {
-    if (tid < 256) {                                   // x_c = sum_{r >= c} Linv[r][c] y_r, 16 lanes per column
+    if (tid < 256) {                                   // 16 lanes per row of L_kk^-T
       const int c = tid >> 4, r = tid & 15;
-      double v = r >= c ? S[small_at(k, k, r, c)] * bv[16 * k + r] : 0.0;
+      double v = r < c ? 0.0 : (r == c ? sv[16 * k + r] : S[small_at(k, k, c, r)]) * bv[16 * k + r];
 #pragma unroll
       for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
       if (r == 0) xv[16 * k + c] = v;
@@ -2505,7 +2450,7 @@ static int run_cholesky(int n, float lm, float ep, BaPtrs w, CholBuf cb, float* 
   if (n == 0) return HS2_OK;
   HS2_PROF("ba_cholesky", s);
   // up to kSmallMax unknowns (the whole triangle fits one CTA's shared memory, and one CTA is still
-  // the faster: 90 us against 125 us at 222) no other CTA takes part
+  // the faster: 82 us against about 110 us at 222) no other CTA takes part
   if (n <= kSmallMax) {
     static DeviceOnce small_once;
     int dev = 0;
