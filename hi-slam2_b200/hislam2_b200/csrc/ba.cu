@@ -294,14 +294,48 @@ __device__ __forceinline__ float warp_transpose_sum(float (&v)[32]) {
   return v[0];
 }
 
-// One (depth frame s, pixel chunk) of the linearisation on a CTA of NT threads.
+// Edge stages of the linearisations: the targets and weights of a CTA's NT * PPT pixels and the
+// edge's table arrive by cp.async while the edge before is linearised (a thread reads back only
+// the pixels it copied itself; the table is shared).  Register prefetch of the 16 values spilled.
+template <int NT, int PPT, int TAB>
+struct EdgeStage {
+  static constexpr int kPix = NT * PPT;
+  static constexpr int kFloats = 2 * (4 * kPix + TAB);   // two stages
+  float* base;
+  __device__ float* px(int st, int a) const { return base + st * (4 * kPix + TAB) + a * kPix + threadIdx.x; }
+  __device__ float* tab(int st) const { return base + st * (4 * kPix + TAB) + 4 * kPix; }
+  // pixel k of thread t is first + k * NT
+  __device__ void load(int st, const float* __restrict__ trg, const float* __restrict__ wgt,
+                       const float* __restrict__ table, int first, int HW) const {
+    const float* src[4] = {trg, trg + HW, wgt, wgt + HW};
+#pragma unroll
+    for (int k = 0; k < PPT; ++k) {
+      const int p = first + k * NT;
+      if (p < HW) {
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(px(st, a) + k * NT)),
+                       "l"(src[a] + p) : "memory");
+      }
+    }
+    if (threadIdx.x < TAB)
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(tab(st) + threadIdx.x)),
+                   "l"(table + threadIdx.x) : "memory");
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  __device__ static void wait() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
+};
+
+// One (depth frame s, pixel chunk) of the linearisation on a CTA of NT threads; `stage`:
+// EdgeStage<NT, kLinPPT, kEtab>::kFloats floats of shared memory.  One barrier per edge: it
+// publishes the edge's table and the previous edge's partial sums.
 template <int NT>
 __device__ __forceinline__ void ba_linearize_body(int s, int chunk, const float* __restrict__ disps, int HW, int wd,
                                                   const float* __restrict__ intr, const float* __restrict__ targets,
                                                   const float* __restrict__ weights, const float* __restrict__ eta,
                                                   int64_t eta_rows, const int64_t* __restrict__ jj, int t0, int t1,
                                                   int motion_only, int skip_fusable, BaPtrs w,
-                                                  const int32_t* __restrict__ info) {
+                                                  const int32_t* __restrict__ info, float* __restrict__ stage) {
   constexpr int kChunk = NT * kLinPPT;
   if (info[0]) return;
   const int M = info[1];
@@ -310,12 +344,18 @@ __device__ __forceinline__ void ba_linearize_body(int s, int chunk, const float*
   const int f = w.kx[s];
   const bool inwin = f >= t0 && f < t1;
   const float fx = intr[0], fy = intr[1], cx = intr[2], cy = intr[3];
+  const EdgeStage<NT, kLinPPT, kEtab> es{stage};
 
-  __shared__ float tab[kEtab];
-  __shared__ float red[NT / 32][32];
+  __shared__ float red[2][NT / 32][32];
 
   int pix[kLinPPT];
   float dsp[kLinPPT], xn[kLinPPT], yn[kLinPPT], Cs[kLinPPT], Ws[kLinPPT], Ei[kLinPPT][6];
+  const int g0 = w.gptr[s], g1 = w.gptr[s + 1];
+  int e = g0 < g1 ? w.gedge[g0] : 0, prev = -1;
+  __syncthreads();                              // the stages' readers of a unit before
+  if (g0 < g1)
+    es.load(0, targets + (int64_t)e * 2 * HW, weights + (int64_t)e * 2 * HW, w.etab + (int64_t)e * kEtab,
+            chunk * kChunk + threadIdx.x, HW);
 #pragma unroll
   for (int k = 0; k < kLinPPT; ++k) {
     pix[k] = chunk * kChunk + k * NT + threadIdx.x;
@@ -330,25 +370,27 @@ __device__ __forceinline__ void ba_linearize_body(int s, int chunk, const float*
     for (int r = 0; r < 6; ++r) Ei[k][r] = 0.f;
   }
 
-  const int g0 = w.gptr[s], g1 = w.gptr[s + 1];
-  for (int g = g0; g < g1; ++g) {
-    const int e = w.gedge[g];
-    __syncthreads();
-    if (threadIdx.x < kEtab) tab[threadIdx.x] = w.etab[(int64_t)e * kEtab + threadIdx.x];
-    __syncthreads();
-    const bool self = (jj[e] == f);
-    const float* trg = targets + (int64_t)e * 2 * HW;
-    const float* wgt = weights + (int64_t)e * 2 * HW;
-    float* Erow = w.erows + ((int64_t)w.epos[e] * 6) * HWs;
-    float tu[kLinPPT], tv[kLinPPT], wgu[kLinPPT], wgv[kLinPPT];
+  // the block's sum of an edge's 27 Hessian / gradient partial sums
+  auto add_edge = [&](int edge, int buf) {
+    if (threadIdx.x < 27) {
+      double acc = 0.0;
 #pragma unroll
-    for (int k = 0; k < kLinPPT; ++k) {
-      const bool ok = pix[k] < HW;
-      tu[k] = ok ? trg[pix[k]] : 0.f;
-      tv[k] = ok ? trg[HW + pix[k]] : 0.f;
-      wgu[k] = ok ? wgt[pix[k]] : 0.f;
-      wgv[k] = ok ? wgt[HW + pix[k]] : 0.f;
+      for (int q2 = 0; q2 < NT / 32; ++q2) acc += (double)red[buf][q2][threadIdx.x];
+      atomicAdd(&w.hedge[(int64_t)edge * 27 + threadIdx.x], acc);
     }
+  };
+  for (int g = g0; g < g1; ++g) {
+    const int st = (g - g0) & 1;
+    const bool self = (jj[e] == f);
+    float* Erow = w.erows + ((int64_t)w.epos[e] * 6) * HWs;
+    es.wait();
+    __syncthreads();
+    const int next = g + 1 < g1 ? w.gedge[g + 1] : -1;
+    if (next >= 0)
+      es.load(st ^ 1, targets + (int64_t)next * 2 * HW, weights + (int64_t)next * 2 * HW, w.etab + (int64_t)next * kEtab,
+              chunk * kChunk + threadIdx.x, HW);
+    if (prev >= 0) add_edge(prev, st ^ 1);
+    const float* tab = es.tab(st);
 
     float H[32];
 #pragma unroll
@@ -358,8 +400,8 @@ __device__ __forceinline__ void ba_linearize_body(int s, int chunk, const float*
       const int p = pix[k];
       if (p >= HW) continue;
       float Ej[6];
-      lin_pixel(tab, fx, fy, cx, cy, xn[k], yn[k], dsp[k], tu[k], tv[k], wgu[k], wgv[k], self,
-                H, Cs[k], Ws[k], Ej);
+      lin_pixel(tab, fx, fy, cx, cy, xn[k], yn[k], dsp[k], es.px(st, 0)[k * NT], es.px(st, 1)[k * NT],
+                es.px(st, 2)[k * NT], es.px(st, 3)[k * NT], self, H, Cs[k], Ws[k], Ej);
       if (!motion_only) {
 #pragma unroll
         for (int r = 0; r < 6; ++r) Erow[(int64_t)r * HWs + p] = Ej[r];
@@ -374,16 +416,13 @@ __device__ __forceinline__ void ba_linearize_body(int s, int chunk, const float*
         }
       }
     }
-    // block reduction of the 27 Hessian/gradient partial sums of this edge
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    red[warp][lane] = warp_transpose_sum(H);
+    red[st][threadIdx.x >> 5][threadIdx.x & 31] = warp_transpose_sum(H);
+    prev = e;
+    e = next;
+  }
+  if (prev >= 0) {
     __syncthreads();
-    if (threadIdx.x < 27) {
-      double acc = 0.0;
-#pragma unroll
-      for (int q2 = 0; q2 < NT / 32; ++q2) acc += (double)red[q2][threadIdx.x];
-      atomicAdd(&w.hedge[(int64_t)e * 27 + threadIdx.x], acc);
-    }
+    add_edge(prev, (g1 - 1 - g0) & 1);
   }
 
   if (motion_only) return;
@@ -408,8 +447,9 @@ ba_linearize_kernel(const float* __restrict__ disps, int HW, int wd, const float
                     const float* __restrict__ eta, int64_t eta_rows, const int64_t* __restrict__ jj,
                     int t0, int t1, int motion_only, int skip_fusable, BaPtrs w,
                     const int32_t* __restrict__ info) {
+  __shared__ float stage[EdgeStage<kLinThreads, kLinPPT, kEtab>::kFloats];
   ba_linearize_body<kLinThreads>(blockIdx.x, blockIdx.y, disps, HW, wd, intr, targets, weights, eta, eta_rows, jj, t0,
-                                 t1, motion_only, skip_fusable, w, info);
+                                 t1, motion_only, skip_fusable, w, info, stage);
 }
 
 // ------------------------------------------------------------- assemble ---
@@ -3224,11 +3264,16 @@ pg_linearize_kernel(const float* __restrict__ disps, int HW, int wd, const float
   const int f = w.kx[s];
   const bool inwin = f >= t0 && f < t1;
   const size_t HWs = (size_t)row_stride(HW);
-  __shared__ float tab[kPgTab];
-  __shared__ float red[kPgThreads / 32][kPgH];
+  __shared__ float stage[EdgeStage<kPgThreads, kPgPPT, kPgTab>::kFloats];
+  __shared__ float red[2][kPgThreads / 32][kPgH];
+  const EdgeStage<kPgThreads, kPgPPT, kPgTab> es{stage};
   const float fx = intr[0], fy = intr[1], cx = intr[2], cy = intr[3];
   const int base = blockIdx.y * kPgChunk + threadIdx.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int g0 = w.gptr[s], g1 = w.gptr[s + 1];
+  int e = g0 < g1 ? w.gedge[g0] : 0, prev = -1;
+  if (g0 < g1)
+    es.load(0, targets + (int64_t)e * 2 * HW, weights + (int64_t)e * 2 * HW, ptab + (int64_t)e * kPgTab, base, HW);
   float xn[kPgPPT], yn[kPgPPT], hd[kPgPPT], C[kPgPPT], W[kPgPPT], Ei[kPgPPT][kPgD];
 #pragma unroll
   for (int k = 0; k < kPgPPT; ++k) {
@@ -3242,15 +3287,26 @@ pg_linearize_kernel(const float* __restrict__ disps, int HW, int wd, const float
 #pragma unroll
     for (int d = 0; d < kPgD; ++d) Ei[k][d] = 0.f;
   }
-  for (int g = w.gptr[s]; g < w.gptr[s + 1]; ++g) {
-    const int e = w.gedge[g];
-    __syncthreads();   // tab / red of the previous edge are consumed
-    if (threadIdx.x < kPgTab) tab[threadIdx.x] = ptab[(int64_t)e * kPgTab + threadIdx.x];
-    __syncthreads();
+  auto add_edge = [&](int edge, int buf) {
+    if (threadIdx.x < kPgH) {
+      double acc = 0.0;
+#pragma unroll
+      for (int q = 0; q < kPgThreads / 32; ++q) acc += (double)red[buf][q][threadIdx.x];
+      atomicAdd(&hedge[(int64_t)edge * kPgH + threadIdx.x], acc);
+    }
+  };
+  for (int g = g0; g < g1; ++g) {
+    const int st = (g - g0) & 1;
     const bool self = jj[e] == (int64_t)f;
     const size_t row = (size_t)w.epos[e];
-    const float* tg = targets + (int64_t)e * 2 * HW;
-    const float* wg = weights + (int64_t)e * 2 * HW;
+    es.wait();
+    __syncthreads();
+    const int next = g + 1 < g1 ? w.gedge[g + 1] : -1;
+    if (next >= 0)
+      es.load(st ^ 1, targets + (int64_t)next * 2 * HW, weights + (int64_t)next * 2 * HW, ptab + (int64_t)next * kPgTab,
+              base, HW);
+    if (prev >= 0) add_edge(prev, st ^ 1);
+    const float* tab = es.tab(st);
     float h[kPgH];
 #pragma unroll
     for (int i = 0; i < kPgH; ++i) h[i] = 0.f;
@@ -3267,10 +3323,10 @@ pg_linearize_kernel(const float* __restrict__ disps, int HW, int wd, const float
       const float z = bad ? 0.f : Z;
       const float dd = bad ? 0.f : 1.f / Z;
       const float d2 = dd * dd;
-      float wu = bad ? 0.f : 0.001f * wg[p];
-      float wv = bad ? 0.f : 0.001f * wg[HW + p];
-      const float ru = tg[p] - (fx * (x / Z) + cx);
-      const float rv = tg[HW + p] - (fy * (y / Z) + cy);
+      float wu = bad ? 0.f : 0.001f * es.px(st, 2)[k * kPgThreads];
+      float wv = bad ? 0.f : 0.001f * es.px(st, 3)[k * kPgThreads];
+      const float ru = es.px(st, 0)[k * kPgThreads] - (fx * (x / Z) + cx);
+      const float rv = es.px(st, 1)[k * kPgThreads] - (fy * (y / Z) + cy);
       const float Jp0 = fx * dd, Jp2 = fx * (-x * d2), Jp4 = fy * dd, Jp5 = fy * (-y * d2);
       const float Jzu = Jp0 * tab[0] + Jp2 * tab[2];
       const float Jzv = Jp4 * tab[1] + Jp5 * tab[2];
@@ -3312,17 +3368,16 @@ pg_linearize_kernel(const float* __restrict__ disps, int HW, int wd, const float
 #pragma unroll
       for (int i = 32; i < kPgH; ++i) {
         const float v = warp_sum(h[i]);
-        if (lane == 0) red[warp][i] = v;
+        if (lane == 0) red[st][warp][i] = v;
       }
-      red[warp][lane] = warp_transpose_sum(*reinterpret_cast<float(*)[32]>(h));   // consumes h[0..31]
+      red[st][warp][lane] = warp_transpose_sum(*reinterpret_cast<float(*)[32]>(h));   // consumes h[0..31]
     }
+    prev = e;
+    e = next;
+  }
+  if (prev >= 0) {
     __syncthreads();
-    if (threadIdx.x < kPgH) {
-      double acc = 0.0;
-#pragma unroll
-      for (int q = 0; q < kPgThreads / 32; ++q) acc += (double)red[q][threadIdx.x];
-      atomicAdd(&hedge[(int64_t)e * kPgH + threadIdx.x], acc);
-    }
+    add_edge(prev, (g1 - 1 - g0) & 1);
   }
   const int64_t er = eta_rows == 1 ? 0 : s;
   const size_t wrow = inwin ? (size_t)w.wpos[f - t0] : 0;

@@ -280,6 +280,7 @@ __device__ void batch_cholesky_blocked(int n, float lm, float ep, BaPtrs w, floa
 constexpr int kGramRows = 256;        // rows with w's: 42 blocks
 constexpr int kGramTiles = (kGramRows / 8) * (kGramRows / 8 + 1) / 2;
 constexpr int kGramStages = 4;
+static_assert(sizeof(float) * EdgeStage<kBatchThreads, kLinPPT, kEtab>::kFloats <= kBatchDynSmem, "edge stages");
 
 __device__ __forceinline__ void cp_async4_zfill(uint32_t dst, const void* src, uint32_t bytes) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
@@ -455,7 +456,8 @@ __device__ void batch_unit(const BatchWin& W, int ph, int idx, float lm, float e
       break;
     case 1:
       ba_linearize_body<kBatchThreads>(idx / W.nlin, idx % W.nlin, W.disps, W.HW, W.wd, W.intr, W.targets,
-                                       W.weights, W.eta, W.eta_rows, W.jj, W.t0, W.t1, 0, 0, w, W.info);
+                                       W.weights, W.eta, W.eta_rows, W.jj, W.t0, W.t1, 0, 0, w, W.info,
+                                       reinterpret_cast<float*>(pv));
       break;
     case 2:
       if (idx < W.nasm) {
