@@ -806,6 +806,33 @@ def altcorr_forward_packed(packed1, packed2, coords, ii, jj, radius):
     return [corr]
 
 
+def altcorr_levels_fits(packed, coords, ii, jj, radius):
+    """Whether :func:`altcorr_levels_packed` takes this call (else one launch per level)."""
+    p0 = packed[0] if packed else None
+    if p0 is None or len(packed) > 4 or not 0 <= int(radius) <= 8 or coords.dim() != 5:
+        return False
+    B, N, C, H, W = p0.shape
+    return (C == 128 and coords.dtype == torch.float32 and tuple(coords.shape) == (B, coords.shape[1], H, W, 2)
+            and ii.dtype == jj.dtype == torch.int64 and ii.numel() == jj.numel() == coords.shape[1] <= 65535
+            and coords.device == ii.device == jj.device == p0.device and B * len(packed) <= 65535
+            and all(pk.shape == (B, N, C, H >> l, W >> l) and min(pk.shape[3:]) > 0 and pk.dtype == p0.dtype
+                    for l, pk in enumerate(packed)))
+
+
+def altcorr_levels_packed(packed, coords, ii, jj, radius):
+    """:func:`altcorr_forward_packed` of every level of a packed pyramid at coords [B, M, H, W, 2] / 2^l in
+    one launch -> [B, M, L (2r+1)^2, H, W]; calls that :func:`altcorr_levels_fits` accepts."""
+    coords, ii, jj = coords.contiguous(), ii.contiguous(), jj.contiguous()
+    B, N, C, H, W = packed[0].shape
+    M, L, radius = coords.shape[1], len(packed), int(radius)
+    corr = torch.empty(B, M, L * (2 * radius + 1) ** 2, H, W, dtype=packed[0].torch_dtype, device=coords.device)
+    ptrs = (ctypes.c_void_p * 4)(*[pk.buf.data_ptr() for pk in packed] + [0] * (4 - L))
+    _lib.check(_lib.load().hs2_altcorr_levels_packed(_ptr(packed[0].buf), ptrs, L, packed[0].dtype, B, N, N, C, H, W,
+                                                     _ptr(coords), _ptr(ii), _ptr(jj), M, radius, _ptr(corr), None,
+                                                     _stream(coords.device)), "altcorr_levels_packed")
+    return corr
+
+
 def altcorr_forward(fmap1, fmap2, coords, ii, jj, radius, *, path="auto"):
     """``droid_backends.altcorr_forward`` (reference ``src/droid.cpp:277-289``) -> [corr].
 

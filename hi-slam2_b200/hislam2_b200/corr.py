@@ -155,8 +155,11 @@ class AltCorrBlock:
             self.packed = [backends.PackedFeatures(lv.contiguous()) for lv in self.pyramid]
 
     def __call__(self, coords, ii, jj):
-        coords = coords.permute(0, 1, 4, 2, 3).contiguous()
         grad = torch.is_grad_enabled() and (coords.requires_grad or self.pyramid[0].requires_grad)
+        if self.packed is not None and not grad and len(self.packed) == self.num_levels \
+                and backends.altcorr_levels_fits(self.packed, coords, ii, jj, self.radius):
+            return backends.altcorr_levels_packed(self.packed, coords, ii, jj, self.radius)
+        coords = coords.permute(0, 1, 4, 2, 3).contiguous()
         corr_list = []
         for i in range(self.num_levels):
             crd = (coords / 2 ** i).contiguous()

@@ -341,28 +341,33 @@ altcorr_fwd_packed_kernel(const T* __restrict__ p1, const T* __restrict__ p2, co
 
 // ------------------------------------------------------------ tile forward ---
 // Dense local correlation on the tensor cores for C = 128 channels.  A CTA owns an 8x8
-// block of pixels of one edge.  The union of the block's D x D windows is a box of
-// bw x bh target positions (about 19 x 19 at 43x77 for reprojected coordinates); when it
-// holds at most kAtMaxPos positions the CTA stages the 64 source rows and the box's
-// rows (channel-last, 16-byte cp.async) in shared memory and computes the full
-// 64 x (bw bh) product with mma.sync m16n8k16 (16-bit operands, FP32 accumulation:
-// exact products, FP32 sums), then every output tap reads its four window values from
-// that product.  The product is 5-6x the taps actually needed, but it runs on the
-// tensor pipe and every target row is read once per block instead of once per pixel
-// and window row.  Blocks whose box is larger (coordinates scattered across the image)
-// fall back to the warp-per-pixel channel-last computation, so any input is correct.
-// mma.sync rather than tcgen05: the B operand is a data-dependent gathered box of
-// up to 384 rows and M is 64 (tcgen05 wants M = 128, i.e. a 16x8 block whose box no
-// longer fits next to its accumulator staging), and the kernel is bounded by the
-// staging and the gather epilogue, not by the tensor pipe.
+// block of pixels of one edge and level.  The union of the block's D x D windows, clipped to
+// the target, is a box of positions (about 20 x 20 at level 0 for reprojected coordinates);
+// its rows (channel-last) arrive in chunks of 64 positions by 16-byte cp.async, two chunks in
+// flight, and the 64 x 64 product of every chunk is formed with mma.sync m16n8k16 (16-bit
+// operands, FP32 accumulation: exact products, FP32 sums).  A product entry that is a tap of
+// its pixel goes from the accumulator straight into the pixel's D x D window in shared memory;
+// the bilinear blend then reads the windows.  The product is 5-6x the taps needed, but it
+// runs on the tensor pipe and every target row is read once per block instead of once per
+// pixel and window row.  Boxes of more than kAtMaxPos positions (coordinates scattered across
+// the image) take the warp-per-pixel channel-last computation, so any input is correct.
+// mma.sync rather than tcgen05: the B operand is a data-dependent gathered box, M is 64, and
+// the kernel is bounded by staging and the tap selection, not by the tensor pipe.
+// Only the windows are kept (17 KB at radius 3), so three CTAs share an SM and one CTA's loads
+// run under another's products; staging the whole box and its product took 217 KB and one
+// CTA per SM.  40 edges of 43x77, four levels, radius 3: 348 us in four launches -> 197 us in
+// one (442 -> 197 us with the scaling and concatenation around the four).
 constexpr int kAtSide = 8;
 constexpr int kAtPix = kAtSide * kAtSide;
-constexpr int kAtThreads = 512;        // 16 warps: 4 m-tiles x 4 n-tile phases
-constexpr int kAtMaxPos = 384;
+constexpr int kAtThreads = 256;        // 8 warps: 2 pairs of m-tiles x 4 pairs of n-tiles
+constexpr int kAtChunk = 64;           // positions per stage
+constexpr int kAtMaxPos = 1024;        // largest box: above, one warp per pixel is the faster
 constexpr int kAtLd = 136;             // halves per staged row: 128 channels + 16 bytes of padding
-constexpr int kAtDLd = kAtMaxPos + 4;  // floats per row of the staged product
-constexpr size_t kAtSmem = (size_t)kAtPix * kAtLd * 2 + (size_t)kAtMaxPos * kAtLd * 2 +
-                           (size_t)kAtPix * kAtDLd * 4 + kAtPix * 16 + 128;
+// floats of a pixel's window (odd: pixels hit different banks)
+__host__ __device__ inline int at_win(int r) { return ((2 * r + 2) * (2 * r + 2)) | 1; }
+inline size_t at_smem_bytes(int r) {
+  return (size_t)(kAtPix + 2 * kAtChunk) * kAtLd * 2 + (size_t)kAtPix * at_win(r) * 4;
+}
 
 template <typename T>
 __device__ __forceinline__ void mma16816(float* d, const uint32_t* a, uint32_t b0, uint32_t b1);
@@ -387,9 +392,6 @@ __device__ __forceinline__ void ldsm_x4(uint32_t* r, uint32_t addr) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
 }
-__device__ __forceinline__ void ldsm_x2(uint32_t& r0, uint32_t& r1, uint32_t addr) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];" : "=r"(r0), "=r"(r1) : "r"(addr));
-}
 __device__ __forceinline__ uint32_t at_smem(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
@@ -397,12 +399,17 @@ __device__ __forceinline__ void at_cp16(uint32_t dst, const void* src, uint32_t 
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
 }
 
-// Arguments of the tile kernel.  altcorr: window coordinates read from `coords`
-// [B][M][2][H][W], target features p2[0], output [B][M][2r+1][2r+1][H][W].  Fused
-// reprojection + lookup (kFused): blockIdx.z is the level, coordinates are the
-// reprojection of frame ii's pixels into frame jj (poses, disps, intrinsics; the float
-// formula of corr_fused.cu) scaled by 2^-level, target features p2[level], output
-// [M][levels * (2r+1)^2][H][W], and the level-0 coordinates optionally to coords_out.
+// Arguments of the tile kernel, by kMode:
+//  kAtOne    window coordinates read from `coords` [B][M][2][H][W], target features p2[0] of
+//            H2 x W2 positions, output [B][M][2r+1][2r+1][H][W];
+//  kAtFused  (B = 1) coordinates are the reprojection of frame ii's pixels into frame jj (poses,
+//            disps, intrinsics; the float formula of corr_fused.cu), the level-0 ones optionally
+//            written to coords_out;
+//  kAtLevels coordinates read from `coords` [B][M][H][W][2].
+// In the last two blockIdx.z holds b and the level: coordinates are scaled by 2^-level, the target
+// features are p2[level] of H >> level by W >> level positions, and the output is
+// [B][M][levels * (2r+1)^2][H][W].
+constexpr int kAtOne = 0, kAtFused = 1, kAtLevels = 2;
 struct AtArgs {
   const void* p1;
   const void* p2[4];
@@ -419,39 +426,38 @@ struct AtArgs {
   float* coords_out;
 };
 
-template <typename T, bool kFused>
-__global__ void __launch_bounds__(kAtThreads, 1)
+template <typename T, int kMode>
+__global__ void __launch_bounds__(kAtThreads, 3)
 altcorr_fwd_tile_kernel(const __grid_constant__ AtArgs A) {
   constexpr int C = 128;
+  constexpr bool kFused = kMode == kAtFused;
   const int H = A.H, W = A.W, r = A.r, M = A.M, N1 = A.N1, N2 = A.N2;
-  const int lvl = kFused ? (int)blockIdx.z : 0;
-  const int H2 = kFused ? H >> lvl : A.H2, W2 = kFused ? W >> lvl : A.W2;
+  const int lvl = kMode == kAtOne ? 0 : (int)blockIdx.z % A.levels;
+  const int b = kMode == kAtOne ? (int)blockIdx.z : (int)blockIdx.z / A.levels;
+  const int H2 = kMode == kAtOne ? A.H2 : H >> lvl, W2 = kMode == kAtOne ? A.W2 : W >> lvl;
   const int64_t* __restrict__ ii = A.ii;
   const int64_t* __restrict__ jj = A.jj;
   const T* __restrict__ p1 = static_cast<const T*>(A.p1);
-  const T* __restrict__ p2 = static_cast<const T*>(A.p2[kFused ? lvl : 0]);
+  const T* __restrict__ p2 = static_cast<const T*>(A.p2[lvl]);
   __shared__ float G[12];   // fused: R (row-major) then t of Gij
+  __shared__ float4 geo[kAtPix];                                                // fractions, window x0, y0 (ints)
+  __shared__ int box[4];                                                        // x0 min, y0 min, x0 max, y0 max
   extern __shared__ __align__(16) uint8_t at_raw[];
   T* As = reinterpret_cast<T*>(at_raw);                                         // [64][kAtLd]
-  T* Bs = As + kAtPix * kAtLd;                                                  // [kAtMaxPos][kAtLd]
-  float* Ds = reinterpret_cast<float*>(Bs + kAtMaxPos * kAtLd);                 // [64][kAtDLd]
-  float4* geo = reinterpret_cast<float4*>(Ds + kAtPix * kAtDLd);               // [64]
-  // box[12]: x0 min, y0 min, x0 max, y0 max of the whole block, then of its top and bottom
-  // halves (rows 0-3, 4-7); reg[8]: per region bx0, by0, bw, mode (0 empty, 1 box, 2 window)
-  int* box = reinterpret_cast<int*>(geo + kAtPix);
-  int* reg = box + 12;
-  const int b = kFused ? 0 : (int)blockIdx.z, m = blockIdx.y;
+  T* Bs = As + kAtPix * kAtLd;                                                  // [2][kAtChunk][kAtLd]
+  float* win = reinterpret_cast<float*>(Bs + 2 * kAtChunk * kAtLd);            // [64][at_win(r)]
+  const int m = blockIdx.y;
   const int HW = H * W;
   const int ntx = (W + kAtSide - 1) / kAtSide;
   const int tx0 = (blockIdx.x % ntx) * kAtSide, ty0 = (blockIdx.x / ntx) * kAtSide;
-  const int D = 2 * r + 2, rd = 2 * r + 1;
+  const int D = 2 * r + 2, rd = 2 * r + 1, wld = at_win(r);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int64_t ix = ii[m], jx = jj[m];
   const bool ok = kFused ? (ix >= 0 && jx >= 0 && ix < N1 && jx < N1 && ix < A.num_poses && jx < A.num_poses &&
                             ix < A.num_disps)
                          : (ix >= 0 && ix < N1 && jx >= 0 && jx < N2);
   if (!ok && tid == 0 && blockIdx.x == 0 && lvl == 0 && A.info) atomicOr(A.info, HS2_DEV_BAD_INDEX);
-  if (tid < 12) box[tid] = (tid & 3) < 2 ? 0x7fffffff : -0x7fffffff;
+  if (tid < 4) box[tid] = tid < 2 ? 0x7fffffff : -0x7fffffff;
   if (kFused && tid == 0) {
     float t[3], q[4];
     if (ok) {
@@ -467,203 +473,200 @@ altcorr_fwd_tile_kernel(const __grid_constant__ AtArgs A) {
     G[6] = 2.f * (x * z - y * w);       G[7] = 2.f * (y * z + x * w);       G[8] = 1.f - 2.f * (x * x + y * y);
     G[9] = t[0]; G[10] = t[1]; G[11] = t[2];
   }
+  const T* f1 = p1 + ((int64_t)b * N1 + (ok ? ix : 0)) * HW * C;
+  const T* f2 = p2 + ((int64_t)b * N2 + (ok ? jx : 0)) * (int64_t)H2 * W2 * C;
+  const uint32_t sA = at_smem(As), sB = at_smem(Bs);
+  // the source rows: one item = a quarter row (four 16-byte copies)
+  if (ok) {
+    const int row = tid >> 2, ch0 = (tid & 3) * 32, px = tx0 + (row & 7), py = ty0 + (row >> 3);
+    const bool live = px < W && py < H;
+    const T* src = live ? f1 + (int64_t)(py * W + px) * C + ch0 : f1;
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      at_cp16(sA + (uint32_t)(row * kAtLd + ch0 + 8 * u) * 2u, src + (live ? 8 * u : 0), live ? 16u : 0u);
+  }
   __syncthreads();
   if (tid < kAtPix) {
     const int px = tx0 + (tid & 7), py = ty0 + (tid >> 3);
     if (px < W && py < H) {
+      const int pix = py * W + px;
       float x, y;
       if (kFused) {
         const float fx = A.intr[0], fy = A.intr[1], cx = A.intr[2], cy = A.intr[3];
-        const int pix = py * W + px;
         const float d = ok ? A.disps[ix * HW + pix] : 0.f;
         const float X = (px - cx) / fx, Y = (py - cy) / fy;
         const float P0 = G[0] * X + G[1] * Y + G[2] + G[9] * d;
         const float P1 = G[3] * X + G[4] * Y + G[5] + G[10] * d;
         const float P2 = G[6] * X + G[7] * Y + G[8] + G[11] * d;
-        const float xc = fx * (P0 / P2) + cx, yc = fy * (P1 / P2) + cy;
+        x = fx * (P0 / P2) + cx;
+        y = fy * (P1 / P2) + cy;
         if (lvl == 0 && A.coords_out) {
-          A.coords_out[((int64_t)m * HW + pix) * 2 + 0] = xc;
-          A.coords_out[((int64_t)m * HW + pix) * 2 + 1] = yc;
+          A.coords_out[((int64_t)m * HW + pix) * 2 + 0] = x;
+          A.coords_out[((int64_t)m * HW + pix) * 2 + 1] = y;
         }
-        const float scale = 1.0f / (float)(1 << lvl);
-        x = xc * scale;
-        y = yc * scale;
+      } else if (kMode == kAtLevels) {
+        x = A.coords[(((int64_t)b * M + m) * HW + pix) * 2];
+        y = A.coords[(((int64_t)b * M + m) * HW + pix) * 2 + 1];
       } else {
-        x = A.coords[(((int64_t)b * M + m) * 2 + 0) * HW + py * W + px];
-        y = A.coords[(((int64_t)b * M + m) * 2 + 1) * HW + py * W + px];
+        x = A.coords[(((int64_t)b * M + m) * 2 + 0) * HW + pix];
+        y = A.coords[(((int64_t)b * M + m) * 2 + 1) * HW + pix];
+      }
+      if (kMode != kAtOne) {
+        const float scale = 1.0f / (float)(1 << lvl);
+        x *= scale;
+        y *= scale;
       }
       const float fx = floorf(x), fy = floorf(y);
-      const int x0 = (int)fx - r, y0 = (int)fy - r;
+      // a window that starts at W2 or ends at 0 has no taps: the clamp keeps the sums in range
+      const int x0 = min(max((int)fx, -2 * D), W2 + 2 * D) - r, y0 = min(max((int)fy, -2 * D), H2 + 2 * D) - r;
       geo[tid] = make_float4(x - fx, y - fy, __int_as_float(x0), __int_as_float(y0));
-      int* bh = box + 4 * (1 + (tid >> 5));
-      atomicMin(&box[0], x0);
-      atomicMin(&box[1], y0);
-      atomicMax(&box[2], x0);
-      atomicMax(&box[3], y0);
-      atomicMin(&bh[0], x0);
-      atomicMin(&bh[1], y0);
-      atomicMax(&bh[2], x0);
-      atomicMax(&bh[3], y0);
+      if (x0 < W2 && x0 + D > 0 && y0 < H2 && y0 + D > 0) {
+        atomicMin(&box[0], x0);
+        atomicMin(&box[1], y0);
+        atomicMax(&box[2], x0);
+        atomicMax(&box[3], y0);
+      }
+    } else {
+      geo[tid] = make_float4(0.f, 0.f, __int_as_float(W2 + 2 * D), __int_as_float(H2 + 2 * D));
     }
   }
   __syncthreads();
-  // regions: the whole block when its box (window positions inside the target only) fits
-  // the staging area, else its two halves, each staged if it fits and computed per pixel
-  // otherwise; an empty box means all of the region's taps are 0
-  auto box_of = [&](const int* bb, int& x0, int& y0, int& w, int& h) {
-    if (bb[0] > bb[2]) {   // no pixel in the region
-      x0 = y0 = w = h = 0;
-      return;
-    }
-    x0 = max(bb[0], 0);
-    y0 = max(bb[1], 0);
-    w = min(min(bb[2], W2) + D, W2) - x0;
-    h = min(min(bb[3], H2) + D, H2) - y0;
-    if (w <= 0 || h <= 0) w = h = 0;
-  };
-  int fx0, fy0, fw, fh;
-  box_of(box, fx0, fy0, fw, fh);
-  const int nreg = (ok && fw * fh > kAtMaxPos) ? 2 : 1;
-  const T* f1 = p1 + ((int64_t)b * N1 + (ok ? ix : 0)) * HW * C;
-  const T* f2 = p2 + ((int64_t)b * N2 + (ok ? jx : 0)) * (int64_t)H2 * W2 * C;
-  const uint32_t sA = at_smem(As), sB = at_smem(Bs);
-  bool a_staged = false;
-  for (int rg = 0; rg < nreg; ++rg) {
-    int bx0, by0, bw, bh;
-    if (nreg == 1) {
-      bx0 = fx0, by0 = fy0, bw = fw, bh = fh;
-    } else {
-      box_of(box + 4 * (1 + rg), bx0, by0, bw, bh);
-    }
-    const int npos = ok ? bw * bh : 0;
-    const int mode = npos == 0 ? 0 : (npos <= kAtMaxPos ? 1 : 2);
-    const int r0 = nreg == 1 ? 0 : 32 * rg, nrows = nreg == 1 ? kAtPix : 32;
-    if (tid == 0) {
-      reg[4 * rg + 0] = bx0;
-      reg[4 * rg + 1] = by0;
-      reg[4 * rg + 2] = bw;
-      reg[4 * rg + 3] = mode;
-    }
-    if (mode == 1) {
-      const int npad = (npos + 7) & ~7;
-      const int arows = a_staged ? 0 : kAtPix;
-      // n / bw without an integer division: for the staged box (n, bw <= 384) (n + 0.5) / bw
-      // stays at least 0.5 / bw from an integer, far beyond the float rounding
-      const float inv_bw = 1.f / (float)bw;
-      // one item = a quarter row (four 16-byte copies): the row's address is formed once
-      for (int idx = tid; idx < (arows + npad) * 4; idx += kAtThreads) {
-        const int row = idx >> 2, ch0 = (idx & 3) * 32;
-        const T* src;
-        uint32_t dst, bytes;
-        if (row < arows) {
-          const int px = tx0 + (row & 7), py = ty0 + (row >> 3);
-          const bool live = px < W && py < H;
-          src = live ? f1 + (int64_t)(py * W + px) * C + ch0 : f1;
-          bytes = live ? 16u : 0u;
-          dst = sA + (uint32_t)(row * kAtLd + ch0) * 2u;
-        } else {
-          const int n = row - arows;
-          const bool live = n < npos;
-          const int qy = __float2int_rz(((float)n + 0.5f) * inv_bw);
-          src = live ? f2 + ((int64_t)(by0 + qy) * W2 + bx0 + n - qy * bw) * C + ch0 : f2;
-          bytes = live ? 16u : 0u;
-          dst = sB + (uint32_t)(n * kAtLd + ch0) * 2u;
-        }
+  // the box of window positions inside the target
+  const int bx0 = max(box[0], 0), by0 = max(box[1], 0);
+  const int bw = box[0] > box[2] ? 0 : min(box[2] + D, W2) - bx0, bh = box[0] > box[2] ? 0 : min(box[3] + D, H2) - by0;
+  const int npos = ok && bw > 0 && bh > 0 ? bw * bh : 0;
+  if (npos > 0 && npos <= kAtMaxPos) {
+    // n / bw without an integer division: for n, bw <= 1024 (n + 0.5) / bw stays at least 0.5 / bw
+    // from an integer, far beyond the float rounding
+    const float inv_bw = 1.f / (float)bw;
+    auto stage = [&](int c) {
+      const int row = tid >> 2, ch0 = (tid & 3) * 32, n = c * kAtChunk + row;
+      const bool live = n < npos;
+      const int qy = __float2int_rz(((float)n + 0.5f) * inv_bw);
+      const T* src = live ? f2 + ((int64_t)(by0 + qy) * W2 + bx0 + n - qy * bw) * C + ch0 : f2;
+      const uint32_t dst = sB + (uint32_t)(((c & 1) * kAtChunk + row) * kAtLd + ch0) * 2u;
 #pragma unroll
-        for (int u = 0; u < 4; ++u) at_cp16(dst + 16u * u, bytes ? (const void*)(src + 8 * u) : (const void*)src, bytes);
+      for (int u = 0; u < 4; ++u) at_cp16(dst + 16u * u, src + (live ? 8 * u : 0), live ? 16u : 0u);
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    const int nchunk = (npos + kAtChunk - 1) / kAtChunk;
+    stage(0);
+    // warp: m-tiles 2 (warp & 1) + {0, 1} (16 pixels each), n-tiles 2 (warp >> 1) + {0, 1} of a chunk;
+    // thread: rows (lane >> 2) and + 8 of each m-tile, columns 2 (lane & 3) + {0, 1} of each n-tile
+    const int m0 = 32 * (warp & 1), n0 = 16 * (warp >> 1);
+    int2 org[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float4 g = geo[m0 + 8 * i + (lane >> 2)];
+      org[i] = make_int2(bx0 - __float_as_int(g.z), by0 - __float_as_int(g.w));
+    }
+    // ldmatrix rows: A 16 x 16 (x4), B two n-tiles x 16 (x4)
+    const uint32_t aaddr = sA + (uint32_t)((m0 + (lane & 7) + 8 * ((lane >> 3) & 1)) * kAtLd + 8 * (lane >> 4)) * 2u;
+    const uint32_t baddr = sB + (uint32_t)((n0 + (lane & 7) + 8 * (lane >> 4)) * kAtLd + 8 * ((lane >> 3) & 1)) * 2u;
+    for (int c = 0; c < nchunk; ++c) {
+      if (c + 1 < nchunk) {
+        stage(c + 1);
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+      } else {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
       }
-      a_staged = true;
-      asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
       __syncthreads();
-      // warp: one of the region's m-tiles (16 pixels), n-tiles strided over the other warps
-      const int nmt = nrows >> 4;
-      const int mt = (r0 >> 4) + warp % nmt;
-      const int nstep = (kAtThreads / 32) / nmt;   // 4 (whole block) or 8 (half) n-tile phases
-      uint32_t af[8][4];
+      float d[2][2][4];
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) d[i][j][e] = 0.f;
+      const uint32_t bc = baddr + (uint32_t)((c & 1) * kAtChunk * kAtLd) * 2u;
 #pragma unroll
       for (int k = 0; k < 8; ++k) {
-        const int rr = (lane & 7) + 8 * ((lane >> 3) & 1), kc = 16 * k + 8 * (lane >> 4);
-        ldsm_x4(af[k], sA + (uint32_t)((16 * mt + rr) * kAtLd + kc) * 2u);
+        uint32_t a0[4], a1[4], bb[4];
+        ldsm_x4(a0, aaddr + 32u * k);
+        ldsm_x4(a1, aaddr + 32u * k + (uint32_t)(16 * kAtLd) * 2u);
+        ldsm_x4(bb, bc + 32u * k);
+        mma16816<T>(d[0][0], a0, bb[0], bb[1]);
+        mma16816<T>(d[0][1], a0, bb[2], bb[3]);
+        mma16816<T>(d[1][0], a1, bb[0], bb[1]);
+        mma16816<T>(d[1][1], a1, bb[2], bb[3]);
       }
-      const int ntile = npad >> 3;
-      for (int nt = warp / nmt; nt < ntile; nt += nstep) {
-        float d[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          uint32_t b0, b1;
-          const int nr = 8 * nt + (lane & 7), kc = 16 * k + 8 * ((lane >> 3) & 1);
-          ldsm_x2(b0, b1, sB + (uint32_t)(nr * kAtLd + kc) * 2u);
-          mma16816<T>(d, af[k], b0, b1);
-        }
-        const int row = 16 * mt + (lane >> 2), col = 8 * nt + 2 * (lane & 3);
-        *reinterpret_cast<float2*>(&Ds[row * kAtDLd + col]) = make_float2(d[0], d[1]);
-        *reinterpret_cast<float2*>(&Ds[(row + 8) * kAtDLd + col]) = make_float2(d[2], d[3]);
-      }
-      __syncthreads();   // the staging area is reused by the next region
-    } else if (mode == 2) {
-      // scattered coordinates: per pixel, one warp computes the D x D window (lanes: 8
-      // positions x 4 channel groups of 32), stored window-major in the pixel's row of Ds
-      const int pq = lane & 7, g = lane >> 3;
-      for (int q = r0 + warp; q < r0 + nrows; q += kAtThreads / 32) {
-        const int px = tx0 + (q & 7), py = ty0 + (q >> 3);
-        if (px >= W || py >= H) continue;
-        const float4 gq = geo[q];
-        const int xb = __float_as_int(gq.z), yb = __float_as_int(gq.w);
-        const uint4* a = reinterpret_cast<const uint4*>(f1 + (int64_t)(py * W + px) * C) + g * 4;
-        uint4 av[4];
+      for (int j = 0; j < 2; ++j)
 #pragma unroll
-        for (int k = 0; k < 4; ++k) av[k] = __ldg(a + k);
-        for (int wy = 0; wy < D; ++wy) {
-          const int y1 = yb + wy;
-          for (int pc = 0; pc < D; pc += 8) {
-            const int wx = pc + pq, x1 = xb + wx;
-            float s0 = 0.f, s1 = 0.f;
-            if (wx < D && y1 >= 0 && y1 < H2 && x1 >= 0 && x1 < W2) {
-              const uint4* bp = reinterpret_cast<const uint4*>(f2 + ((int64_t)y1 * W2 + x1) * C) + g * 4;
+        for (int e = 0; e < 2; ++e) {
+          const int n = c * kAtChunk + n0 + 8 * j + 2 * (lane & 3) + e;
+          const int qy = __float2int_rz(((float)n + 0.5f) * inv_bw), qx = n - qy * bw;
+          if (n < npos) {
 #pragma unroll
-              for (int k = 0; k < 4; ++k) dot8<T>(av[k], __ldg(bp + k), s0, s1);
+            for (int i = 0; i < 4; ++i) {   // pixel rows lane / 4 + 8 i: accumulator entry 2 (i & 1) + e of m-tile i / 2
+              const int wx = org[i].x + qx, wy = org[i].y + qy;
+              if ((unsigned)wx < (unsigned)D && (unsigned)wy < (unsigned)D)
+                win[(m0 + 8 * i + (lane >> 2)) * wld + wy * D + wx] = d[i >> 1][j][2 * (i & 1) + e];
             }
-            float sv = s0 + s1;
-            sv += __shfl_xor_sync(0xffffffffu, sv, 8);
-            sv += __shfl_xor_sync(0xffffffffu, sv, 16);
-            if (g == 0 && wx < D) Ds[q * kAtDLd + wy * D + wx] = sv;
           }
+        }
+      __syncthreads();   // the stage is rewritten by the chunk after next
+    }
+  } else if (npos > 0) {
+    // scattered coordinates: per pixel, one warp computes the D x D window (lanes: 8 positions x 4
+    // channel groups of 32)
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    const int pq = lane & 7, g = lane >> 3;
+    for (int q = warp; q < kAtPix; q += kAtThreads / 32) {
+      const int px = tx0 + (q & 7), py = ty0 + (q >> 3);
+      if (px >= W || py >= H) continue;
+      const float4 gq = geo[q];
+      const int xb = __float_as_int(gq.z), yb = __float_as_int(gq.w);
+      const uint4* a = reinterpret_cast<const uint4*>(f1 + (int64_t)(py * W + px) * C) + g * 4;
+      uint4 av[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) av[k] = __ldg(a + k);
+      for (int wy = 0; wy < D; ++wy) {
+        const int y1 = yb + wy;
+        for (int pc = 0; pc < D; pc += 8) {
+          const int wx = pc + pq, x1 = xb + wx;
+          float s0 = 0.f, s1 = 0.f;
+          if (wx < D && y1 >= 0 && y1 < H2 && x1 >= 0 && x1 < W2) {
+            const uint4* bp = reinterpret_cast<const uint4*>(f2 + ((int64_t)y1 * W2 + x1) * C) + g * 4;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) dot8<T>(av[k], __ldg(bp + k), s0, s1);
+          }
+          float sv = s0 + s1;
+          sv += __shfl_xor_sync(0xffffffffu, sv, 8);
+          sv += __shfl_xor_sync(0xffffffffu, sv, 16);
+          if (g == 0 && wx < D) win[q * wld + wy * D + wx] = sv;
         }
       }
     }
   }
+  asm volatile("cp.async.wait_all;" ::: "memory");
   __syncthreads();
   // bilinear blend: thread (pixel q, x offset a) walks the window rows, keeping the two
   // values of the previous row, so each output reads two new window values; taps outside
   // the target are 0
   const int nout = rd * rd;
-  T* out = static_cast<T*>(A.corr) + (kFused ? ((int64_t)m * A.levels + lvl) : ((int64_t)b * M + m)) * nout * HW;
+  T* out = static_cast<T*>(A.corr) +
+           (kMode == kAtOne ? (int64_t)b * M + m : ((int64_t)b * M + m) * A.levels + lvl) * nout * HW;
   for (int idx = tid; idx < kAtPix * rd; idx += kAtThreads) {
     const int q = idx & 63, a = idx >> 6;
     const int px = tx0 + (q & 7), py = ty0 + (q >> 3);
     if (px >= W || py >= H) continue;
-    const int* rq = reg + 4 * (nreg == 1 ? 0 : q >> 5);
-    const int mode = rq[3];
     T* oq = out + (int64_t)(a * rd) * HW + py * W + px;
-    if (mode == 0) {
+    if (npos == 0) {
       for (int bb = 0; bb < rd; ++bb) oq[(int64_t)bb * HW] = from_f<T>(0.f);
       continue;
     }
     const float4 gq = geo[q];
-    const int xb = __float_as_int(gq.z), yb = __float_as_int(gq.w);
-    const int x1 = xb + a;
+    const int yb = __float_as_int(gq.w), x1 = __float_as_int(gq.z) + a;
     const bool va = x1 >= 0 && x1 < W2, vb = x1 + 1 >= 0 && x1 + 1 < W2;
-    // row-major addressing of the window values: the staged box (mode 1) or the pixel's own
-    // D x D window (mode 2)
-    const int rs = mode == 1 ? rq[2] : D;
-    const float* dq = Ds + q * kAtDLd + (mode == 1 ? (yb - rq[1]) * rs + (x1 - rq[0]) : a);
+    const float* dq = win + q * wld + a;
     const float w00 = (1.f - gq.x) * (1.f - gq.y), w01 = gq.x * (1.f - gq.y);
     const float w10 = (1.f - gq.x) * gq.y, w11 = gq.x * gq.y;
     float t0 = 0.f, t1 = 0.f;
     for (int wy = 0; wy <= rd; ++wy) {
       const int y1 = yb + wy;
       const bool vy = y1 >= 0 && y1 < H2;
-      const float* row = dq + wy * rs;
+      const float* row = dq + wy * D;
       const float u0 = (vy && va) ? row[0] : 0.f, u1 = (vy && vb) ? row[1] : 0.f;
       if (wy > 0)
         oq[(int64_t)(wy - 1) * HW] = from_f<T>((w00 * t0 + w01 * t1 + w10 * u0 + w11 * u1) * 0.0625f);
@@ -785,16 +788,23 @@ static int ac_fwd_packed_n(const void* p1, const void* p2, int b, int n1, int n2
   return HS2_OK;
 }
 
-template <typename T, bool kFused>
-static int at_prepare() {
+constexpr int kAtMaxRadius = 8;        // windows up to 18 x 18 taps
+
+template <typename T, int kMode>
+static int at_launch(const AtArgs& a, int nz, cudaStream_t s) {
   static DeviceOnce once;
   int dev = 0;
   HS2_CUDA(cudaGetDevice(&dev));
-  return once.run(dev, [&]() -> int {
-    HS2_CUDA(cudaFuncSetAttribute(altcorr_fwd_tile_kernel<T, kFused>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)kAtSmem));
+  const int rc = once.run(dev, [&]() -> int {
+    HS2_CUDA(cudaFuncSetAttribute(altcorr_fwd_tile_kernel<T, kMode>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)at_smem_bytes(kAtMaxRadius)));
     return HS2_OK;
   });
+  if (rc) return rc;
+  dim3 grid(((a.W + kAtSide - 1) / kAtSide) * ((a.H + kAtSide - 1) / kAtSide), (unsigned)a.M, (unsigned)nz);
+  altcorr_fwd_tile_kernel<T, kMode><<<grid, kAtThreads, at_smem_bytes(a.r), s>>>(a);
+  HS2_LAUNCH_CHECK("altcorr_fwd_tile_kernel");
+  return HS2_OK;
 }
 
 template <typename T>
@@ -805,9 +815,7 @@ static int ac_fwd_packed(const void* p1, const void* p2, int b, int n1, int n2, 
     case 32: return ac_fwd_packed_n<T, 1>(p1, p2, b, n1, n2, h, w, h2, w2, coords, ii, jj, m, radius, corr, info, s);
     case 64: return ac_fwd_packed_n<T, 2>(p1, p2, b, n1, n2, h, w, h2, w2, coords, ii, jj, m, radius, corr, info, s);
     case 128: {
-      if (radius <= 8) {   // windows up to 18 x 18 taps
-        int rc = at_prepare<T, false>();
-        if (rc) return rc;
+      if (radius <= kAtMaxRadius) {
         AtArgs a{};
         a.p1 = p1;
         a.p2[0] = p2;
@@ -817,12 +825,8 @@ static int ac_fwd_packed(const void* p1, const void* p2, int b, int n1, int n2, 
         a.corr = corr;
         a.N1 = n1, a.N2 = n2, a.H = h, a.W = w, a.H2 = h2, a.W2 = w2, a.M = m, a.r = radius, a.levels = 1;
         a.info = info;
-        const int ntiles = ((w + kAtSide - 1) / kAtSide) * ((h + kAtSide - 1) / kAtSide);
-        dim3 grid(ntiles, m, b);
         HS2_PROF("altcorr_fwd_tile", s);
-        altcorr_fwd_tile_kernel<T, false><<<grid, kAtThreads, kAtSmem, s>>>(a);
-        HS2_LAUNCH_CHECK("altcorr_fwd_tile_kernel");
-        return HS2_OK;
+        return at_launch<T, kAtOne>(a, b, s);
       }
       return ac_fwd_packed_n<T, 4>(p1, p2, b, n1, n2, h, w, h2, w2, coords, ii, jj, m, radius, corr, info, s);
     }
@@ -1024,16 +1028,46 @@ extern "C" int hs2_corr_reproject_lookup_packed(const float* poses, int64_t num_
   int rc;
   if ((rc = bind_device(corr))) return rc;
   cudaStream_t s = (cudaStream_t)stream;
-  const int ntiles = ((wd + kAtSide - 1) / kAtSide) * ((ht + kAtSide - 1) / kAtSide);
-  dim3 grid(ntiles, (unsigned)num_edges, levels);
   HS2_PROF("corr_fused_tile", s);
-  if (dtype == HS2_F16) {
-    if ((rc = at_prepare<__half, true>())) return rc;
-    altcorr_fwd_tile_kernel<__half, true><<<grid, kAtThreads, kAtSmem, s>>>(a);
-  } else {
-    if ((rc = at_prepare<__nv_bfloat16, true>())) return rc;
-    altcorr_fwd_tile_kernel<__nv_bfloat16, true><<<grid, kAtThreads, kAtSmem, s>>>(a);
+  return dtype == HS2_F16 ? at_launch<__half, kAtFused>(a, levels, s) : at_launch<__nv_bfloat16, kAtFused>(a, levels, s);
+}
+
+extern "C" int hs2_altcorr_levels_packed(const void* packed1, const void* const* packed_levels, int levels, int dtype,
+                                         int b, int n1, int n2, int c, int h, int w, const float* coords,
+                                         const int64_t* ii, const int64_t* jj, int m, int radius, void* corr,
+                                         int32_t* info, hs2_stream_t stream) {
+  using namespace hs2;
+  int rc = ac_check("altcorr_levels_packed", b, n1, n2, c, h, w, h, w, m, radius);
+  if (rc) return rc;
+  if (levels < 1 || levels > 4 || radius > kAtMaxRadius || c != 128 || (h >> (levels - 1)) < 1 ||
+      (w >> (levels - 1)) < 1 || (int64_t)b * levels > 65535) {
+    set_error("altcorr_levels_packed: 1 to 4 levels, 128 channels and radius <= %d (got %d, %d, %d)", kAtMaxRadius,
+              levels, c, radius);
+    return HS2_ERR_INVALID;
   }
-  HS2_LAUNCH_CHECK("altcorr_fwd_tile_kernel (fused)");
-  return HS2_OK;
+  if (dtype != HS2_F16 && dtype != HS2_BF16) {
+    set_error("altcorr_levels_packed: float16 or bfloat16 features only (dtype %d)", dtype);
+    return HS2_ERR_DTYPE;
+  }
+  if (m == 0 || b == 0) return HS2_OK;
+  AtArgs a{};
+  for (int l = 0; l < levels; ++l) {
+    if (!packed_levels || !packed_levels[l]) {
+      set_error("altcorr_levels_packed: level %d missing", l);
+      return HS2_ERR_INVALID;
+    }
+    a.p2[l] = packed_levels[l];
+  }
+  if ((rc = bind_device(corr))) return rc;
+  a.p1 = packed1;
+  a.coords = coords;
+  a.ii = ii;
+  a.jj = jj;
+  a.corr = corr;
+  a.N1 = n1, a.N2 = n2, a.H = h, a.W = w, a.M = m, a.r = radius, a.levels = levels;
+  a.info = info;
+  cudaStream_t s = (cudaStream_t)stream;
+  HS2_PROF("altcorr_fwd_tile", s);
+  return dtype == HS2_F16 ? at_launch<__half, kAtLevels>(a, b * levels, s)
+                          : at_launch<__nv_bfloat16, kAtLevels>(a, b * levels, s);
 }

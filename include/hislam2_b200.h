@@ -247,6 +247,16 @@ int hs2_altcorr_forward_packed(const void* packed1, const void* packed2, int dty
                                const int64_t* jj, int m, int radius, void* corr, int32_t* info,
                                hs2_stream_t stream);
 
+/* All levels of a feature pyramid in one launch (hislam2/modules/corr.py:107-117): packed1 as
+ * above, packed_levels[l] the packed features [b,n2,(h>>l)*(w>>l),c] of the pooled maps,
+ * coords [b,m,h,w,2] (scaled by 2^-l per level) -> corr [b,m,levels*(2r+1)^2,h,w], equal to
+ * hs2_altcorr_forward_packed of every level concatenated.  c == 128, radius <= 8, levels <= 4,
+ * b * levels <= 65535; info may be NULL. */
+int hs2_altcorr_levels_packed(const void* packed1, const void* const* packed_levels, int levels, int dtype, int b,
+                              int n1, int n2, int c, int h, int w, const float* coords, const int64_t* ii,
+                              const int64_t* jj, int m, int radius, void* corr, int32_t* info,
+                              hs2_stream_t stream);
+
 /* altcorr_backward  (reference: src/droid.cpp:291-305, src/altcorr_kernel.cu:79-129,175-225;
  *   effective positional order as called from hislam2/modules/corr.py:86)
  *   grad [b,m,2r+1,2r+1,h,w] f32 (same layout as the forward output).
