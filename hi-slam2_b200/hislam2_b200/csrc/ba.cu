@@ -1470,31 +1470,38 @@ static int encode_erows_map(CUtensorMap* map, float* erows, int HW, int64_t plan
 // cooperative (persistent) launch, one CTA per SM:
 //
 //   damping   diag += ep + lm*diag                                          | barrier
-//   panel 0                                                                 | barrier
+//   panel 0
 //   for kb = 0 .. nbk-2 (look-ahead by one panel)
-//     A   column block kb+1 -= L[:, kb] L[kb+1, kb]^T in 16-row slices      | per-row counters
-//     B   panel kb+1 on `rest` CTAs (each waits for its two block rows'
-//         slices), in parallel with the remaining tiles of update kb
-//         (column blocks kb+2 ..) on the other CTAs                         | barrier
+//     panel kb+1 (column block kb+1 with update kb applied on the way) on one CTA per task, in
+//     parallel with the tiles of update kb right of it (column blocks kb+2 ..) on the
+//     other CTAs; both wait for the L blocks and tiles they read by counters  | barrier
 //   backward  x_c = L_cc^-T (y_c - sum_{j>c} L_jc^T x_j), one CTA per block c,
 //             ordered by per-block ready flags instead of grid barriers; L_cc^-1
 //             formed in shared memory while the blocks above are solved
 //
 // Panel kb, task t: the CTA holds [D; X | b] in shared memory (D the 64x64 diagonal
-// block, redundantly in every CTA of the panel; X the t-th 64-row tile below D, none
-// for t == 0; b the right-hand side) and eliminates the 64 columns in four 16-column
-// sub-panels, left-looking: (a) the sub-panel columns receive the updates of the
-// sub-panels left of them, (b) one warp factors the 16x16 diagonal sub-block and
-// its part of b in registers and forms the inverse, (c) the rows below are multiplied
-// by it.  Task 0 writes L11, the reciprocal
-// pivots and y = L11^-1 b1; the others write L21 and b2 - L21 y1.
+// block, redundantly in every CTA of the panel; X half of the t-th 64-row tile below D, none
+// for t == 0; b the right-hand side) and the L rows of panel kb-1 for the same rows, and
+// eliminates the 64 columns in four 16-column sub-panels: (1) warp 0 applies the sub-panel
+// left of it to the 16x16 diagonal sub-block, factors it and its part of b and forms the
+// inverse, while the six warps off its FP64 pipe bring the rows below and the next sub-panel of D
+// up to date (in the last, two of them fetch the next panel's tiles); (2) the rows below are multiplied
+// by the inverse.  Task 0 writes L11, the reciprocal pivots and y = L11^-1 b1; the
+// others write L21 and b2 - L21 y1.
+// Bound by this chain (24k cycles per panel: four factors of 3k, their row products, 3k for one
+// hop through L2) once fewer than about 18 block rows are left, by the tiles before that.  With
+// update kb of column block kb+1 as tasks of their own (a further hop), unpipelined tiles and
+// their static assignment / now: 141 / 110 us at 384 unknowns, 370 / 280 at 1152, 605 / 433 at
+// 1740, 2471 / 1137 at 3000, 57700 / 3770 at 4800 (where panel tasks held all CTAs but a few).
 //
 // A non-positive pivot is seen identically by every CTA that factors the panel; the
 // solution is then 0, as in the reference's solver fallback.  Every spin (grid
 // barrier, ready flag) is bounded: on timeout the kernel sets HS2_DEV_TIMEOUT and
 // returns.  Data written inside the launch is read through L2 (ld.global.cg).
 constexpr int kCholThreads = 256;
-constexpr int kPLD = 66;   // padded row length (doubles) of panel/tile rows in shared memory
+// padded row length (doubles) of panel/tile rows in shared memory: rows 8 banks apart, so the 4 x 4
+// doubles of a half-warp's MMA fragment meet no bank conflict (66 gave two-way ones)
+constexpr int kPLD = 68;
 constexpr unsigned kBarrierSpins = 1u << 22;
 constexpr int kCtlFlags = 4;   // ctl[4 + c]: x of block c is final
 // A panel's X tile (the 64 rows of one block row below D) is split over kXSplit tasks of
@@ -1503,14 +1510,18 @@ constexpr int kCtlFlags = 4;   // ctl[4 + c]: x of block c is final
 constexpr int kXSplit = 2;
 constexpr int kXRows = 64 / kXSplit;
 
+// Tiles per remaining CTA from which the CTAs of a panel take tiles too (a tile takes about a third of
+// a panel): 2 / 3 / 5 gave 433 / 435 / 439 us at 1740 unknowns, 1137 / 1142 / 1160 at 3000.
+constexpr int kHelpTiles = 2;
+
 struct CholBuf {
-  double* L11;      // [nbk][64][64] factored diagonal blocks (zero above the diagonal)
+  double* L11;      // [nbk][64][64] factored diagonal blocks (zero on and above the diagonal)
   double* dinv;     // [nbk][64] reciprocals of their diagonals
   double* y;        // [n] forward-substituted right-hand side
   unsigned* ctl;    // [0] barrier count, [1] barrier generation, [2] failed, [4 + c] ready flags,
-                    // [4 + nbk + R] phase-A slices done on block row R,
+                    // [4 + nbk + kb] tiles of update kb handed out,
                     // [4 + 2 nbk + R] panels whose L of block row R is written,
-                    // [4 + 3 nbk + R nbk + C] trailing (phase-B) updates applied to tile (R, C)
+                    // [4 + 3 nbk + R nbk + C] updates applied to tile (R, C) by tile tasks
 };
 
 __device__ __forceinline__ double2 ldcg2(const double* p) {
@@ -1566,31 +1577,6 @@ __device__ __forceinline__ void red_release_add_gpu(unsigned* p, unsigned v) {
   asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
-// Panel kb+1, task t reads block rows kb+1 (D) and kb+1+t (X) of column block kb+1: waits
-// until the four phase-A slices of each have been applied for every panel up to kb.
-__device__ bool chol_wait_slices(const unsigned* slices, int kb, int t, int32_t* info) {
-  __shared__ int s_bad;
-  if (threadIdx.x == 0) {
-    const unsigned target = 4u * (unsigned)(kb + 1);
-    int bad = 0;
-    for (int k = 0; k < (t > 0 ? 2 : 1) && !bad; ++k) {
-      const unsigned* c = slices + kb + 1 + (k ? t : 0);
-      unsigned spins = 0;
-      while (ld_acquire_gpu(c) < target) {
-        if (++spins > kBarrierSpins) {
-          atomicOr(info, HS2_DEV_TIMEOUT);
-          bad = 1;
-          break;
-        }
-        if (spins > 64) __nanosleep(32);
-      }
-    }
-    s_bad = bad;
-  }
-  __syncthreads();
-  return s_bad == 0;
-}
-
 // Waits (thread 0) until *c >= target; false on timeout, or at once when another wait of
 // the launch has already timed out.
 __device__ __forceinline__ bool wait_count(const unsigned* c, unsigned target, int32_t* info) {
@@ -1606,18 +1592,19 @@ __device__ __forceinline__ bool wait_count(const unsigned* c, unsigned target, i
   return true;
 }
 
-// A trailing-update task on tile (R, C) with panel kb: waits until panel kb has written
-// the L blocks of rows R and C and the tile holds the phase-B updates of panels < kb
-// (tcnt >= tdone).  CTA-wide result.
-__device__ bool chol_wait_tile(const unsigned* lcnt, const unsigned* tcnt, int nbk, int kb, int R, int C,
-                               unsigned tdone, int32_t* info) {
-  __shared__ int s_ok;
-  __syncthreads();
-  if (threadIdx.x == 0)
-    s_ok = wait_count(lcnt + R, kXSplit * (kb + 1), info) && wait_count(lcnt + C, kXSplit * (kb + 1), info) &&
-           wait_count(tcnt + (int64_t)R * nbk + C, tdone, info);
-  __syncthreads();
-  return s_ok != 0;
+// A trailing-update task on tile (R, C) with panel kb starts when panel kb has written
+// the L blocks of rows R and C and the tile holds the updates of panels < kb: thread i < 3 takes
+// the i-th counter, `wait` until it is there.  CTA-wide result.
+__device__ __forceinline__ bool chol_tile_ready(const unsigned* lcnt, const unsigned* tcnt, int nbk, int kb, int R, int C,
+                                                bool wait, int32_t* info) {
+  const int i = threadIdx.x;
+  bool ok = true;
+  if (i < 3) {
+    const unsigned* c = i == 0 ? lcnt + R : i == 1 ? lcnt + C : tcnt + (int64_t)R * nbk + C;
+    const unsigned target = i < 2 ? kXSplit * (kb + 1) : kb;
+    ok = wait ? wait_count(c, target, info) : ld_acquire_gpu(c) >= target;
+  }
+  return __syncthreads_and(ok) != 0;
 }
 
 // Waits (thread 0) until the ready flag is set; false on timeout.
@@ -1640,7 +1627,7 @@ __device__ __forceinline__ void dmma_m8n8k4(double& d0, double& d1, double a, do
                : "+d"(d0), "+d"(d1) : "d"(a), "d"(b));
 }
 
-// (b) One warp factors the nsb x nsb diagonal sub-block, A = L L^T, in registers and forms
+// One warp factors the nsb x nsb diagonal sub-block, A = L L^T, in registers and forms
 // L^-T along with it, fraction-free with 2 x 2 pivot blocks: with u, v the trailing columns
 // j, j+1, the block P = [p q; q s] and det = p s - q^2, step (j, j+1) replaces the trailing
 // entries by
@@ -1655,12 +1642,16 @@ __device__ __forceinline__ void dmma_m8n8k4(double& d0, double& d1, double a, do
 // column and the square roots taken after the loop, off the elimination chain, one per lane.
 // Lane = row: lanes 0..15 the sub-block's rows, lanes 16..31 the rows of an identity below
 // them, whose elimination leaves I L^-T (the other rows' triangular solves become products
-// with it: (c) took 1.8k cycles as a 15-step substitution; 1740 unknowns 725 -> 677 us).  Columns j, j+1 (and b_j, b_j+1) are
-// exchanged through a double-buffered 2 x 36 shared array, one __syncwarp per block step.
-// Rows and columns outside nsb are those of the identity.  Writes L (lower part), L^-T above
-// the diagonal, 1/L_jj to sv and y to bv.  at(r, k) is the sub-block's entry, bv and sv its
+// with it; a 15-step substitution took 1.8k cycles).  Columns j,
+// j+1 (and b_j, b_j+1) are exchanged through a triple-buffered 2 x 36 shared array, one
+// __syncwarp per block step; the next block's columns are updated and handed over first, so the
+// exchange and the chain to the next determinant run under the update of the other columns.
+// kAhead forms the next determinant before
+// it too: 281 -> 274 us at 1152 unknowns in the panels; in the one-CTA solve, at 128 registers a
+// thread, the spills cost more (78 -> 82 us at 222).  Rows and columns outside nsb are those of the identity.  Writes L below the diagonal, L^-T on
+// and above it, 1/L_jj to sv and y to bv.  at(r, k) is the sub-block's entry, bv and sv its
 // right-hand side and reciprocal pivots.
-template <typename At>
+template <bool kAhead, typename At>
 __device__ __forceinline__ void chol_factor_diag(At at, double* bv, double* sv, double* xc, int nsb, int* sfail) {
   const int lane = threadIdx.x & 31, rr = lane & 15;
   const bool own = lane < 16;
@@ -1675,40 +1666,55 @@ __device__ __forceinline__ void chol_factor_diag(At at, double* bv, double* sv, 
   double bb = (own && rr < nsb) ? bv[rr] : 0.0;
   double cfac = 1.0, my_cd = 1.0, my_f = 1.0, my_b = 0.0;
   bool ok = true;
-#pragma unroll
-  for (int j = 0; j < 16; j += 2) {
-    double* col = xc + ((j >> 1) & 1) * 36;   // [0,16) u, [16,32) v, [32] b_j, [33] b_j+1
+  // columns j, j+1 into buffer (j / 2) % 3: [0,16) u, [16,32) v, [32] b_j, [33] b_j+1
+  auto hand_over = [&](int j, double u, double v) {
+    double* col = xc + ((j >> 1) % 3) * 36;
     if (own) {
-      col[rr] = a[j];
-      col[16 + rr] = a[j + 1];
+      col[rr] = u;
+      col[16 + rr] = v;
     }
     if (lane == j || lane == j + 1) col[32 + lane - j] = bb;
     __syncwarp();
-    const double p = col[j], q = col[j + 1], s = col[16 + j + 1];
+  };
+  double p, q, s, det, sc;
+  double2 bjj;
+  auto take = [&](int j) {                      // the pivot block of step j, its determinant and 2^-E
+    const double* col = xc + ((j >> 1) % 3) * 36;
+    p = col[j], q = col[j + 1], s = col[16 + j + 1];
+    bjj = *reinterpret_cast<const double2*>(&col[32]);
+    det = fma(p, s, -(q * q));
+    sc = __longlong_as_double((2046LL - ((__double_as_longlong(det) >> 52) & 0x7FF)) << 52);
+  };
+  hand_over(0, a[0], a[1]);
+  if (kAhead) take(0);
+#pragma unroll
+  for (int j = 0; j < 16; j += 2) {
+    const double* col = xc + ((j >> 1) % 3) * 36;
+    if (!kAhead) take(j);
     const double ur = a[j], vr = a[j + 1];
-    const double2 bjj = *reinterpret_cast<const double2*>(&col[32]);
-    const double det = fma(p, s, -(q * q));
     ok = ok && (p > 0.0) && (det > 0.0);
-    const long long bits = __double_as_longlong(det);
-    const double sc = __longlong_as_double((2046LL - ((bits >> 52) & 0x7FF)) << 52);   // 2^-E
     const double w1 = fma(s, ur, -(q * vr)), w2 = fma(p, vr, -(q * ur));
     const double dets = det * sc, w1s = w1 * sc, w2s = w2 * sc;
+    const double bj1 = fma(p, bjj.y, -(q * bjj.x)), bj0 = bjj.x;
+    const double cp = cfac * p, cpd = cp * det;
+    if (own && rr > j + 1) bb = fma(bb, dets, -fma(w1s, bjj.x, w2s * bjj.y));
 #pragma unroll
     for (int t = j + 2; t < 16; t += 2) {
       const double2 u = *reinterpret_cast<const double2*>(&col[t]);
       const double2 v = *reinterpret_cast<const double2*>(&col[16 + t]);
       a[t] = fma(a[t], dets, -fma(w1s, u.x, w2s * v.x));
       a[t + 1] = fma(a[t + 1], dets, -fma(w1s, u.y, w2s * v.y));
+      if (t == j + 2) {
+        hand_over(t, a[t], a[t + 1]);
+        if (kAhead) take(t);
+      }
     }
-    const double bj1 = fma(p, bjj.y, -(q * bjj.x));
-    if (own && rr > j + 1) bb = fma(bb, dets, -fma(w1s, bjj.x, w2s * bjj.y));
     // columns j, j+1 are final
-    const double cp = cfac * p, cpd = cp * det;
     a[j + 1] = w2;
     if (rr == j) {
       my_cd = cp;
       my_f = cfac;
-      my_b = bjj.x;
+      my_b = bj0;
     }
     if (rr == j + 1) {
       my_cd = cpd;
@@ -1717,26 +1723,26 @@ __device__ __forceinline__ void chol_factor_diag(At at, double* bv, double* sv, 
     }
     cfac *= dets;
   }
-  const double s = rsqrt(my_cd);
-  double* xs = xc;                             // buffer 0: the last step used buffer 1
+  const double rs = rsqrt(my_cd);
+  double* xs = xc;                             // buffer 0: last read before the hand-over of the last block
   if (own) {
-    xs[rr] = s;
+    xs[rr] = rs;
     if (rr < nsb) {
-      sv[rr] = my_f * s;
-      bv[rr] = my_b * s;
+      sv[rr] = my_f * rs;
+      bv[rr] = my_b * rs;
     }
   }
   __syncwarp();
 #pragma unroll
   for (int k = 0; k < 16; k += 2) {
     const double2 sk = *reinterpret_cast<const double2*>(&xs[k]);
-    if (rr < nsb && k < nsb && (own ? k <= rr : k > rr)) at(rr, k) = a[k] * sk.x;
-    if (rr < nsb && k + 1 < nsb && (own ? k + 1 <= rr : k + 1 > rr)) at(rr, k + 1) = a[k + 1] * sk.y;
+    if (rr < nsb && k < nsb && (own ? k < rr : k >= rr)) at(rr, k) = a[k] * sk.x;
+    if (rr < nsb && k + 1 < nsb && (own ? k + 1 < rr : k + 1 >= rr)) at(rr, k + 1) = a[k + 1] * sk.y;
   }
   if (lane == 0 && !ok) *sfail = 1;
 }
 
-// (c) One warp solves eight rows below a factored sub-block, X = A L^-T, on the FP64 tensor
+// One warp solves eight rows below a factored sub-block, X = A L^-T, on the FP64 tensor
 // cores: row(r, k) is the entry of row r (0..7), tr(l, c) that of L^-T.  In place; lane l is
 // left with X[l / 4][8 h + 2 (l % 4) + {0, 1}] in x[2 h + {0, 1}].
 template <typename Row, typename Tr>
@@ -1758,137 +1764,6 @@ __device__ __forceinline__ void chol_solve_rows(Row row, Tr tr, double (&x)[4]) 
   }
 }
 
-// Panel kb, task t (0: D only; t >= 1: D and the (t-1)-th tile below it).  Returns
-// false when a pivot is not positive (ctl[2] is then set).
-__device__ bool chol_panel(int n, int kb, int t, int xh, double* __restrict__ A, double* __restrict__ bvec,
-                           CholBuf cb, double* csm) {
-  const int tid = threadIdx.x;
-  const int o = kb * kNB, nb = min(kNB, n - o);
-  const int r0 = o + nb + (t - 1) * kNB + xh * kXRows;
-  const int nr = t == 0 ? 0 : max(0, min(kXRows, n - r0));
-  double (*Pm)[kPLD] = reinterpret_cast<double (*)[kPLD]>(csm);   // [128][kPLD]: D rows, then X rows
-  double* bv = csm + 128 * kPLD;                                   // [128]
-  double* sv = bv + 128;                                           // [64] 1/L_jj
-  double* xc = sv + 64;                                            // [72] column exchange of (b)
-  int* sfail = reinterpret_cast<int*>(xc + 72);
-  __syncthreads();
-#pragma unroll
-  for (int half = 0; half < 2; ++half) {
-    double2 v[8];
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      const int idx = tid + (half * 8 + q) * kCholThreads;   // double2 index in the 128 x 32 grid
-      const int r = idx >> 5, k = (idx & 31) * 2;
-      const bool live = r < kNB ? r < nb : r - kNB < nr;
-      const double* src = A + (int64_t)(r < kNB ? o + r : r0 + r - kNB) * n + o + k;
-      v[q] = make_double2(0.0, 0.0);
-      if (live && k + 1 < nb) v[q] = ldcg2(src);   // n is even: a pair never leaves the row
-      else if (live && k < nb) v[q].x = __ldcg(src);
-    }
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      const int idx = tid + (half * 8 + q) * kCholThreads;
-      *reinterpret_cast<double2*>(&Pm[idx >> 5][(idx & 31) * 2]) = v[q];
-    }
-  }
-  if (tid < 128) {
-    const int r = tid;
-    bv[r] = r < kNB ? (r < nb ? __ldcg(&bvec[o + r]) : 0.0) : (r - kNB < nr ? __ldcg(&bvec[r0 + r - kNB]) : 0.0);
-  }
-  if (tid == 0) *sfail = 0;
-  __syncthreads();
-  for (int c0 = 0; c0 < nb; c0 += 16) {
-    const int c1 = min(c0 + 16, nb);
-    if (c0 > 0) {
-      const int lane = tid & 31, warp = tid >> 5;
-      // (a) left-looking update of the sub-panel columns [c0, c0+16) of the rows >= c0 and the
-      // X rows by FP64 tensor-core MMA (m8n8k4): a warp owns an 8-row tile and both 8-column
-      // halves, k runs over the c0 columns already eliminated.
-      const int td = (((nb + 7) >> 3) - (c0 >> 3)), tx = (nr + 7) >> 3;
-      for (int tile = warp; tile < td + tx; tile += kCholThreads / 32) {
-        const int rt = tile < td ? c0 + 8 * tile : kNB + 8 * (tile - td);
-        double d00 = 0.0, d01 = 0.0, d10 = 0.0, d11 = 0.0;
-        for (int k0 = 0; k0 < c0; k0 += 4) {
-          const double av = Pm[rt + (lane >> 2)][k0 + (lane & 3)];
-          const double b0 = Pm[c0 + (lane >> 2)][k0 + (lane & 3)];
-          const double b1 = Pm[c0 + 8 + (lane >> 2)][k0 + (lane & 3)];
-          dmma_m8n8k4(d00, d01, av, b0);
-          dmma_m8n8k4(d10, d11, av, b1);
-        }
-        double* row = Pm[rt + (lane >> 2)] + c0 + (lane & 3) * 2;
-        row[0] -= d00;
-        row[1] -= d01;
-        row[8] -= d10;
-        row[9] -= d11;
-      }
-      if (tid < c1 - c0) {
-        const int r = c0 + tid;
-        double b0 = 0.0, b1 = 0.0;
-        for (int k = 0; k < c0; k += 2) {
-          b0 = fma(Pm[r][k], bv[k], b0);
-          b1 = fma(Pm[r][k + 1], bv[k + 1], b1);
-        }
-        bv[r] -= b0 + b1;
-      }
-      __syncthreads();
-    }
-    // (b)
-    if (tid < 32)
-      chol_factor_diag([&](int r, int k) -> double& { return Pm[c0 + r][c0 + k]; }, bv + c0, sv + c0, xc, c1 - c0, sfail);
-    __syncthreads();
-    if (*sfail) {
-      if (tid == 0) atomicExch(cb.ctl + 2, 1u);
-      return false;
-    }
-    // (c) rows below the sub-block: X = A L_ss^-T, eight rows per warp and step
-    {
-      const int warp = tid >> 5;
-      const int td = (nb - c1 + 7) >> 3, tx = (nr + 7) >> 3;   // c1 = c0 + 16 wherever D has rows below
-      for (int tile = warp; tile < td + tx; tile += kCholThreads / 32) {
-        const int rt = tile < td ? c1 + 8 * tile : kNB + 8 * (tile - td);
-        double x[4];
-        chol_solve_rows([&](int r, int k) -> double& { return Pm[rt + r][c0 + k]; },
-                        [&](int l, int c) -> double {
-                          if (l > c) return 0.0;
-                          return l == c ? (c0 + l < c1 ? sv[c0 + l] : 1.0) : Pm[c0 + l][c0 + c];
-                        }, x);
-      }
-    }
-    __syncthreads();
-  }
-  // X rows: b2 -= L21 y1 (four threads per row)
-  {
-    const int i = tid >> 2, part = tid & 3;
-    double s = 0.0;
-    if (i < nr)
-      for (int k = part; k < nb; k += 4) s = fma(Pm[kNB + i][k], bv[k], s);
-    s += __shfl_xor_sync(0xffffffffu, s, 1);
-    s += __shfl_xor_sync(0xffffffffu, s, 2);
-    __syncthreads();
-    if (i < nr && part == 0) bv[kNB + i] -= s;
-  }
-  __syncthreads();
-  if (t == 0) {
-    for (int idx = tid; idx < kNB * kNB; idx += kCholThreads) {
-      const int i = idx >> 6, l = idx & 63;
-      cb.L11[((int64_t)kb * kNB + i) * kNB + l] = (l <= i && i < nb) ? Pm[i][l] : 0.0;
-    }
-    if (tid < kNB) {
-      cb.dinv[(int64_t)kb * kNB + tid] = tid < nb ? sv[tid] : 0.0;
-      if (tid < nb) cb.y[o + tid] = bv[tid];
-    }
-  } else {
-    for (int idx = tid; idx < nr * (kNB / 2); idx += kCholThreads) {
-      const int i = idx >> 5, k = (idx & 31) * 2;
-      double* dst = A + (int64_t)(r0 + i) * n + o + k;
-      if (k + 1 < nb) *reinterpret_cast<double2*>(dst) = *reinterpret_cast<const double2*>(&Pm[kNB + i][k]);
-      else if (k < nb) *dst = Pm[kNB + i][k];
-    }
-    if (tid < nr) bvec[r0 + tid] = bv[kNB + tid];
-  }
-  return true;
-}
-
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, uint32_t src_bytes) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(src_bytes) : "memory");
 }
@@ -1896,74 +1771,220 @@ __device__ __forceinline__ void cp_async_wait_all() {
   asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
 }
 
-// A[ri + i][rj + j] -= sum_k L[ri + i][o + k] L[rj + j][o + k] over the 16*RG rows
-// at ri and the 64 columns at rj; `diag` keeps only entries on or below the
-// diagonal of A.  FP64 tensor-core MMA (m8n8k4): the 4x4-per-thread SIMT form read shared
-// memory for half its time (the solve of 1740 unknowns: 677 us with it, 610 us so).  Both L row
-// blocks and the target tile itself arrive by 16-byte cp.async copies issued together
-// (one L2 round trip; rows and columns outside the matrix are zero-filled).
-template <int RG>
-__device__ void chol_update_tile(int n, double* __restrict__ A, int o, int ri, int rj, bool diag, double* csm) {
+// Panel kb, task t (0: D only; t >= 1: D and half xh of the t-th tile below it).  Returns false
+// when a wait timed out; a pivot that is not positive sets ctl[2].  Shared memory: the tiles of even
+// panels, the L rows of panel kb-1, the tiles of odd panels; `prefetch`: this CTA's next task is
+// task (t, xh) of the next panel.
+constexpr int kPanelRows = kNB + kXRows;
+constexpr size_t kPanelDoubles = (size_t)3 * kPanelRows * kPLD + 128 + 64 + 108 + 2;
+__device__ bool chol_panel(int n, int nbk, int kb, int t, int xh, double* __restrict__ A, double* __restrict__ bvec,
+                           CholBuf cb, const unsigned* lcnt, const unsigned* tcnt, bool prefetch, int32_t* info,
+                           double* csm) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, lr = lane >> 2, lq = lane & 3;
+  const int o = kb * kNB, nb = min(kNB, n - o);
+  const int r0 = o + nb + (t - 1) * kNB + xh * kXRows;
+  const int nr = t == 0 ? 0 : max(0, min(kXRows, n - r0));
+  double (*Pm)[kPLD] = reinterpret_cast<double (*)[kPLD]>(csm + (kb & 1) * 2 * kPanelRows * kPLD);   // D rows, X rows
+  double (*Lm)[kPLD] = reinterpret_cast<double (*)[kPLD]>(csm + kPanelRows * kPLD);   // their L rows of panel kb-1
+  double* bv = csm + 3 * kPanelRows * kPLD;                        // [128] right-hand side of the rows
+  double* sv = bv + 128;                                           // [64] 1/L_jj
+  double* xc = sv + 64;                                            // [108] exchange of the factor
+  int* sfail = reinterpret_cast<int*>(xc + 108);
+  __shared__ int s_fetched;                                        // the panel's tiles are prefetched
+  const int rows = t == 0 ? kNB : kPanelRows;
+  // rows first, first + step, .. < end of panel k's task from column c (`cols` of them live) to dst, by one warp
+  auto fetch = [&](int first, int step, int end, double* dst, int k, int c, int cols) {
+    const bool col = 2 * lane < cols;                              // n is even: a pair never leaves the row
+    const int od = k * kNB, ox = (k + t) * kNB + xh * kXRows - kNB;
+    const double* src = A + c + 2 * lane;
+    const uint32_t sb = smem_u32(dst) + 16u * lane;
+#pragma unroll 4
+    for (int r = first; r < end; r += step) {
+      const int g = r + (r < kNB ? od : ox);
+      const bool live = col && g < n;
+      cp_async16(sb + (uint32_t)(r * kPLD) * 8u, live ? src + (int64_t)g * n : A, live ? 16u : 0u);
+    }
+  };
+  // one thread waits for the counter of D's rows, another for that of X's; false on timeout
+  auto ready = [&](const unsigned* cd, const unsigned* cx, unsigned target) {
+    const bool ok = tid == 0 ? wait_count(cd, target, info) : tid == 32 && t > 0 ? wait_count(cx, target, info) : true;
+    return __syncthreads_and(ok) != 0;
+  };
+  __syncthreads();
+  const bool got = kb > 0 && s_fetched;
+  if (kb > 0 && !got && !ready(tcnt + (int64_t)kb * nbk + kb, tcnt + (int64_t)(kb + t) * nbk + kb, kb - 1))
+    return false;
+  if (!got) fetch(warp, kCholThreads / 32, rows, &Pm[0][0], kb, o, nb);
+  __syncthreads();
+  if (tid == 0) *sfail = s_fetched = 0;
+  bool go = true;
+  if (kb > 0 && (go = ready(lcnt + kb, lcnt + kb + t, kXSplit * kb)))
+    fetch(warp, kCholThreads / 32, rows, &Lm[0][0], kb, o - kNB, kNB);
+  if (tid < 128)
+    bv[tid] = tid < kNB ? (tid < nb ? __ldcg(&bvec[o + tid]) : 0.0)
+                        : (tid - kNB < nr ? __ldcg(&bvec[r0 + tid - kNB]) : 0.0);
+  cp_async_wait_all();
+  __syncthreads();
+  if (!go) return false;
+  // Pm[rt..rt+8)[c..c+8 kT) -= sum over panel kb-1 (prev) and over the columns [k0, k1) of this panel
+  auto update = [&](auto tiles, int rt, int c, bool prev, int k0, int k1) {
+    constexpr int kT = decltype(tiles)::value;
+    double d[2][kT][2] = {};
+    auto product = [&](const double* ar, const double* br, int ka, int ke) {
+#pragma unroll 2
+      for (int k = ka; k < ke; k += 8)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const double av = ar[k + 4 * h];
+#pragma unroll
+          for (int j = 0; j < kT; ++j) dmma_m8n8k4(d[h][j][0], d[h][j][1], av, br[8 * j * kPLD + k + 4 * h]);
+        }
+    };
+    if (prev) product(&Lm[rt + lr][lq], &Lm[c + lr][lq], 0, kNB);
+    product(&Pm[rt + lr][lq], &Pm[c + lr][lq], k0, k1);
+#pragma unroll
+    for (int j = 0; j < kT; ++j) {
+      double2* e = reinterpret_cast<double2*>(&Pm[rt + lr][c + 8 * j + 2 * lq]);
+      double2 v = *e;
+      v.x -= d[0][j][0] + d[1][j][0];
+      v.y -= d[0][j][1] + d[1][j][1];
+      *e = v;
+    }
+  };
+  const std::integral_constant<int, 1> one{};
+  const std::integral_constant<int, 2> two{};
+  if (kb > 0) {                                     // panel kb-1 on the first diagonal sub-block
+    if (warp < 3) update(one, warp > 0 ? 8 : 0, warp > 1 ? 8 : 0, true, 0, 0);
+    __syncthreads();
+  }
+  const int tx = (nr + 7) >> 3;
+  for (int c0 = 0; c0 < nb; c0 += 16) {
+    const int c1 = min(c0 + 16, nb);
+    const int td = (nb - c1 + 7) >> 3;              // 8-row strips of D below; c1 = c0 + 16 wherever there are any
+    auto below = [&](int i) { return i < td ? c1 + 8 * i : kNB + 8 * (i - td); };
+    if (warp == 0) {
+      if (c0 > 0) {
+        // the sub-panel to the left on the lower three 8x8 tiles of the sub-block
+        double d[3][2] = {};
+        const double* l = &Pm[c0 + lr][c0 - 16 + lq];
+#pragma unroll
+        for (int k = 0; k < 16; k += 4) {
+          const double a0 = l[k], a1 = l[8 * kPLD + k];
+          dmma_m8n8k4(d[0][0], d[0][1], a0, a0);
+          dmma_m8n8k4(d[1][0], d[1][1], a1, a0);
+          dmma_m8n8k4(d[2][0], d[2][1], a1, a1);
+        }
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+          double2* e = reinterpret_cast<double2*>(&Pm[c0 + (i > 0) * 8 + lr][c0 + (i > 1) * 8 + 2 * lq]);
+          const double2 v = *e;
+          *e = make_double2(v.x - d[i][0], v.y - d[i][1]);
+        }
+        __syncwarp();
+      }
+      chol_factor_diag<true>([&](int r, int k) -> double& { return Pm[c0 + r][c0 + k]; }, bv + c0, sv + c0, xc, c1 - c0,
+                       sfail);
+    } else if (warp & 3) {
+      // D rows below: the sub-panel to the left (sub-panel 0: panel kb-1); X rows: all that is to
+      // the left; D rows of the next sub-panel: all but this one
+      for (int i = (warp >> 2) * 3 + (warp & 3) - 1; i < 2 * td + tx && c0 + kb > 0; i += 6) {
+        if (i < td) update(two, c1 + 8 * i, c0, c0 == 0, c0 == 0 ? 0 : c0 - 16, c0);
+        else if (i < td + tx) update(two, kNB + 8 * (i - td), c0, kb > 0, 0, c0);
+        else update(two, c1 + 8 * (i - td - tx), c0 + 16, kb > 0, 0, c0);
+      }
+    } else if (prefetch && kb + 1 + t < nbk && c0 == 32) {
+      // do the next panel's tiles hold their updates?
+      const unsigned* c = tcnt + (int64_t)(kb + 1 + (lane & 1) * t) * nbk + kb + 1;
+      const bool full = __all_sync(0xffffffffu, ld_acquire_gpu(c) >= (unsigned)kb);
+      if (lane == 0) s_fetched = full;
+    }
+    // then the two warps without strips in the last phase fetch them
+    if (c0 == 48 && warp >= 6 && s_fetched)
+      fetch(warp - 6, 2, rows, csm + ((kb + 1) & 1) * 2 * kPanelRows * kPLD, kb + 1, o + kNB, min(kNB, n - o - kNB));
+    __syncthreads();
+    if (*sfail) {
+      if (tid == 0) atomicExch(cb.ctl + 2, 1u);
+      return true;
+    }
+    // rows below the sub-block: X = A L_ss^-T, b -= X y_s, eight rows per warp and step
+    for (int i = warp; i < td + tx; i += kCholThreads / 32) {
+      const int rt = below(i);
+      double x[4];
+      chol_solve_rows([&](int r, int k) -> double& { return Pm[rt + r][c0 + k]; },
+                      [&](int l, int c) -> double {
+                        return l > c ? 0.0 : Pm[c0 + l][c0 + c];
+                      }, x);
+      if (i >= td && rt - kNB + lr < nr) {
+        double* dst = A + (int64_t)(r0 + rt - kNB + lr) * n + o + c0 + 2 * lq;
+        *reinterpret_cast<double2*>(dst) = make_double2(x[0], x[1]);
+        *reinterpret_cast<double2*>(dst + 8) = make_double2(x[2], x[3]);
+      }
+      const double* ys = bv + c0 + 2 * lq;
+      double acc = fma(x[0], ys[0], x[1] * ys[1]) + fma(x[2], ys[8], x[3] * ys[9]);
+      acc += __shfl_xor_sync(0xffffffffu, acc, 1);
+      acc += __shfl_xor_sync(0xffffffffu, acc, 2);
+      if (lq == 0) bv[rt + lr] -= acc;
+    }
+    __syncthreads();
+  }
+  if (t == 0) {
+    for (int idx = tid; idx < kNB * kNB; idx += kCholThreads) {
+      const int i = idx >> 6, l = idx & 63;
+      cb.L11[((int64_t)kb * kNB + i) * kNB + l] = (l < i && i < nb) ? Pm[i][l] : 0.0;
+    }
+    if (tid < kNB) {
+      cb.dinv[(int64_t)kb * kNB + tid] = tid < nb ? sv[tid] : 0.0;
+      if (tid < nb) cb.y[o + tid] = bv[tid];
+    }
+  } else if (tid < nr) {
+    bvec[r0 + tid] = bv[kNB + tid];
+  }
+  return true;
+}
+
+// Trailing-update task: A[ri + i][rj + j] -= sum_k L[ri + i][o + k] L[rj + j][o + k] over the 64
+// rows at ri and the 64 columns at rj.  FP64 tensor-core MMA (m8n8k4): the 4x4-per-thread SIMT
+// form read shared memory for half its time.  Both L row blocks and the tile itself arrive by 16-byte cp.async copies issued
+// together (one L2 round trip; rows and columns outside the matrix are zero-filled), those of the
+// next task under the products of this one.
+constexpr size_t kTileDoubles = (size_t)192 * kPLD;
+__device__ __forceinline__ void chol_load_tile(int n, const double* __restrict__ A, int o, int ri, int rj,
+                                               double* csm) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t sb = smem_u32(csm) + 16u * lane;
+#pragma unroll 4
+  for (int r = warp; r < 192; r += kCholThreads / 32) {   // L rows of the block rows, of the block columns, the tile
+    const int g = (r < 64 || r >= 128 ? ri : rj) + (r & 63), c = (r < 128 ? o : rj) + 2 * lane;
+    const bool live = g < n && c < n;                     // n is even: a pair never leaves the row
+    cp_async16(sb + (uint32_t)(r * kPLD) * 8u, live ? A + (int64_t)g * n + c : A, live ? 16u : 0u);
+  }
+  asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
+// The products of a loaded tile; `diag` keeps only entries on or below the diagonal of A.
+__device__ __forceinline__ void chol_update_tile(int n, double* __restrict__ A, int ri, int rj, bool diag,
+                                                 double* csm) {
   const int tid = threadIdx.x;
-  const int ni = min(16 * RG, n - ri), nj = min(kNB, n - rj);
-  if (ni <= 0) return;
-  constexpr int kRows = 16 * RG;
+  const int ni = min(kNB, n - ri), nj = min(kNB, n - rj);
   double (*Ai)[kPLD] = reinterpret_cast<double (*)[kPLD]>(csm);
   double (*Aj)[kPLD] = reinterpret_cast<double (*)[kPLD]>(csm + 64 * kPLD);
   double (*Cs)[kPLD] = reinterpret_cast<double (*)[kPLD]>(csm + 128 * kPLD);
-  __syncthreads();
-  {
-    const uint32_t sb = smem_u32(csm);
-    for (int idx = tid; idx < (2 * kRows + 64) * 32; idx += kCholThreads) {
-      const int r = idx >> 5, k = (idx & 31) * 2;
-      int srow, a;
-      int64_t grow;
-      int gcol;
-      bool live;
-      if (r < kRows) {                       // L rows of the tile's block rows
-        srow = r;
-        live = r < ni;
-        grow = ri + r;
-        gcol = o + k;
-      } else if (r < kRows + 64) {           // L rows of the tile's block columns
-        a = r - kRows;
-        srow = 64 + a;
-        live = a < nj;
-        grow = rj + a;
-        gcol = o + k;
-      } else {                               // the tile
-        a = r - kRows - 64;
-        srow = 128 + a;
-        live = a < ni && k < nj;
-        grow = ri + a;
-        gcol = rj + k;
-      }
-      cp_async16(sb + (uint32_t)(srow * kPLD + k) * 8u, live ? (const void*)(A + grow * n + gcol) : (const void*)A,
-                 live ? 16u : 0u);
-    }
-    cp_async_wait_all();
-  }
-  __syncthreads();
-  // warp: an 8-row strip and kT of its 8-column tiles (all eight of a 64-row tile, two of a 16-row
-  // slice); a diagonal tile stops at its strip
-  constexpr int kT = RG == 4 ? 8 : 2;
+  // warp: an 8-row strip and its eight 8-column tiles; a diagonal tile stops at its strip
   const int lane = tid & 31, warp = tid >> 5, r = lane >> 2, q = lane & 3;
-  const int strip = RG == 4 ? warp : warp & 1, t0 = RG == 4 ? 0 : (warp >> 1) * kT;
-  const int row = ri + 8 * strip;                    // first row of the strip
-  const int nt = diag ? min(kT, (row + 7 - rj - 8 * t0) / 8 + 1) : kT;
-  double acc[kT][2];
+  const int nt = diag ? min(8, (ri + 8 * warp + 7 - rj) / 8 + 1) : 8;
+  double acc[8][2];
 #pragma unroll
-  for (int t = 0; t < kT; ++t) acc[t][0] = acc[t][1] = 0.0;
+  for (int t = 0; t < 8; ++t) acc[t][0] = acc[t][1] = 0.0;
 #pragma unroll 4
   for (int k = 0; k < kNB; k += 4) {
-    const double av = Ai[8 * strip + r][k + q];
+    const double av = Ai[8 * warp + r][k + q];
 #pragma unroll
-    for (int t = 0; t < kT; ++t)
-      if (t < nt) dmma_m8n8k4(acc[t][0], acc[t][1], av, Aj[8 * (t0 + t) + r][k + q]);
+    for (int t = 0; t < 8; ++t)
+      if (t < nt) dmma_m8n8k4(acc[t][0], acc[t][1], av, Aj[8 * t + r][k + q]);
   }
 #pragma unroll
-  for (int t = 0; t < kT; ++t) {
-    const int i = 8 * strip + r, j = 8 * (t0 + t) + 2 * q;   // nj is even: a pair never leaves the matrix
+  for (int t = 0; t < 8; ++t) {
+    const int i = 8 * warp + r, j = 8 * t + 2 * q;   // nj is even: a pair never leaves the matrix
     if (t >= nt || i >= ni || j >= nj || (diag && rj + j > ri + i)) continue;
     const double2 c = *reinterpret_cast<const double2*>(&Cs[i][j]);
     double* dst = A + (int64_t)(ri + i) * n + rj + j;
@@ -2093,70 +2114,82 @@ ba_cholesky_kernel(int n, float lm, float ep, BaPtrs w, CholBuf cb, float* __res
   if (!grid_barrier(cb.ctl, G, info)) return;
 
   // Dataflow instead of a grid barrier per panel: every task waits (acquire) only for the
-  // tasks that write its inputs and counts itself (release) when done.  A task of stage
-  // A(kb) / B(kb) depends only on tasks of earlier stages and every CTA runs its tasks in
+  // tasks that write its inputs and counts itself (release) when done.  A task of stage kb
+  // depends only on tasks of earlier stages and every CTA runs its tasks in
   // stage order, so with all CTAs resident (cooperative launch) no wait can cycle.  A
   // failed factorisation does not stop the schedule (results are discarded at the end).
-  unsigned* slices = cb.ctl + kCtlFlags + nbk;
+  unsigned* queue = cb.ctl + kCtlFlags + nbk;
   unsigned* lcnt = cb.ctl + kCtlFlags + 2 * nbk;
   unsigned* tcnt = cb.ctl + kCtlFlags + 3 * nbk;
+  __shared__ unsigned s_tile[2];
+  constexpr unsigned kNoTile = 0xffffffffu;
   // panel task tau of a panel with `rest` block rows from its diagonal down: tau = 0 is D
-  // alone, tau >= 1 is half (tau - 1) % kXSplit of block row 1 + (tau - 1) / kXSplit
-  for (int tau = blockIdx.x; tau < 1 + kXSplit * (nbk - 1); tau += G) {
+  // alone, tau >= 1 is half (tau - 1) % kXSplit of block row 1 + (tau - 1) / kXSplit.  A task
+  // counts the L block it writes on its block row.
+  auto panel_task = [&](int kb, int tau, bool more) -> bool {
     const int t = tau == 0 ? 0 : 1 + (tau - 1) / kXSplit, xh = tau == 0 ? 0 : (tau - 1) % kXSplit;
-    chol_panel(n, 0, t, xh, A, bvec, cb, csm);
+    if (!chol_panel(n, nbk, kb, t, xh, A, bvec, cb, lcnt, tcnt, more, info, csm)) return false;
     __syncthreads();
-    if (threadIdx.x == 0 && t > 0) red_release_add_gpu(lcnt + t, 1u);
-  }
+    if (tid == 0 && t > 0) red_release_add_gpu(lcnt + kb + t, 1u);
+    return true;
+  };
+  for (int tau = blockIdx.x; tau < 1 + kXSplit * (nbk - 1); tau += G)
+    if (!panel_task(0, tau, (int)G > kXSplit * (nbk - 1))) return;
 
   for (int kb = 0; kb + 1 < nbk; ++kb) {
-    const int o = kb * kNB;
-    const int rest = nbk - kb - 1;
-    // A: column block kb+1, 16-row slices of the tiles below panel kb; each slice counts
-    // itself on its block row, which the panel tasks of phase B wait for
-    for (int t = blockIdx.x; t < rest * 4; t += G) {
-      const int I = t >> 2, q = t & 3;
-      if (!chol_wait_tile(lcnt, tcnt, nbk, kb, kb + 1 + I, kb + 1, (unsigned)kb, info)) return;
-      chol_update_tile<1>(n, A, o, o + kNB + I * kNB + 16 * q, o + kNB, I == 0, csm);
-      __syncthreads();
-      if (threadIdx.x == 0) red_release_add_gpu(slices + kb + 1 + I, 1u);
-    }
-    // B: panel kb+1 (tasks 0..rest-1) || tiles (I, J), 1 <= J <= I < rest, of update kb.
-    // The panel tasks sit on CTAs of their own (they are the longer tasks); the tiles go
-    // round-robin over the remaining CTAs.  A panel task counts the L block it writes on
-    // its block row; a tile counts the update it applied.
+    // panel kb+1 || tiles (I, J), 1 <= J <= I < rest, of update kb.  The panel tasks sit on the
+    // first CTAs (they carry the chain); the others take tiles from a counter, column by column:
+    // panel kb+2 waits for the first.  A tile counts the update it applied.
+    const int o = kb * kNB, rest = nbk - kb - 1;
     const int ntiles = rest * (rest - 1) / 2;
     const int ntask = 1 + kXSplit * (rest - 1);
-    const bool split = (int)G > ntask;
-    const int tfirst = split ? ((int)blockIdx.x < ntask ? ntiles : (int)blockIdx.x - ntask) : (int)blockIdx.x;
-    const int tstep = split ? (int)G - ntask : (int)G;
-    auto panel_task = [&](int tau) -> bool {
-      const int t = tau == 0 ? 0 : 1 + (tau - 1) / kXSplit, xh = tau == 0 ? 0 : (tau - 1) % kXSplit;
-      if (!chol_wait_slices(slices, kb, t, info)) return false;
-      chol_panel(n, kb + 1, t, xh, A, bvec, cb, csm);
-      __syncthreads();
-      if (threadIdx.x == 0 && t > 0) red_release_add_gpu(lcnt + kb + 1 + t, 1u);
-      return true;
-    };
-    if (split && (int)blockIdx.x < ntask) {
-      if (!panel_task(blockIdx.x)) return;
+    // the panel's CTAs go on to the next panel unless more than kHelpTiles tiles are left to each of the others
+    const int others = (int)G - ntask;
+    const bool help = ntiles > kHelpTiles * others;
+    const bool ahead = ntiles > (help ? (int)G : others);   // a task in advance where there is one for every CTA
+    for (int tau = blockIdx.x; tau < ntask; tau += G)
+      if (!panel_task(kb + 1, tau, !help)) return;
+    if (!help && (int)blockIdx.x < ntask) continue;
+    __syncthreads();
+    if (tid == 0) {
+      s_tile[0] = atomicAdd(queue + kb, 1u);
+      s_tile[1] = ahead ? atomicAdd(queue + kb, 1u) : kNoTile;
     }
-    for (int t = tfirst; t < (split ? ntiles : ntask + ntiles); t += tstep) {
-      if (!split && t < ntask) {
-        if (!panel_task(t)) return;
-        continue;
+    __syncthreads();
+    unsigned cur = s_tile[0], nxt = s_tile[1];
+    bool loaded = false;
+    auto place = [&](unsigned tt, int& I, int& J) {       // tt counts the tiles column by column
+      J = 1;
+      for (; (int)tt >= rest - J; ++J) tt -= rest - J;
+      I = J + (int)tt;
+    };
+    for (int buf = 0; cur < (unsigned)ntiles; buf ^= 1) {
+      int I, J;
+      place(cur, I, J);
+      double* tile = csm + buf * kTileDoubles;
+      if (!loaded) {
+        if (!chol_tile_ready(lcnt, tcnt, nbk, kb, kb + 1 + I, kb + 1 + J, true, info)) return;
+        chol_load_tile(n, A, o, o + kNB + I * kNB, o + kNB + J * kNB, tile);
       }
-      int I = 0, tt = split ? t : t - ntask;
-      while (tt > I) {
-        tt -= I + 1;
-        ++I;
+      loaded = false;
+      if (nxt < (unsigned)ntiles) {
+        int In, Jn;
+        place(nxt, In, Jn);
+        loaded = chol_tile_ready(lcnt, tcnt, nbk, kb, kb + 1 + In, kb + 1 + Jn, false, info);
+        if (loaded) chol_load_tile(n, A, o, o + kNB + In * kNB, o + kNB + Jn * kNB, csm + (buf ^ 1) * kTileDoubles);
       }
-      const int J = tt + 1;
-      ++I;
-      if (!chol_wait_tile(lcnt, tcnt, nbk, kb, kb + 1 + I, kb + 1 + J, (unsigned)kb, info)) return;
-      chol_update_tile<4>(n, A, o, o + kNB + I * kNB, o + kNB + J * kNB, I == J, csm);
+      unsigned next = kNoTile;
+      if (tid == 0 && (nxt < (unsigned)ntiles || !ahead)) next = atomicAdd(queue + kb, 1u);
+      if (loaded) asm volatile("cp.async.wait_group 1;" ::: "memory");
+      else asm volatile("cp.async.wait_group 0;" ::: "memory");
       __syncthreads();
-      if (threadIdx.x == 0) red_release_add_gpu(tcnt + (int64_t)(kb + 1 + I) * nbk + kb + 1 + J, 1u);
+      chol_update_tile(n, A, o + kNB + I * kNB, o + kNB + J * kNB, I == J, tile);
+      if (tid == 0) s_tile[0] = next;
+      __syncthreads();
+      if (tid == 0) red_release_add_gpu(tcnt + (int64_t)(kb + 1 + I) * nbk + kb + 1 + J, 1u);
+      cur = ahead ? nxt : s_tile[0];
+      nxt = ahead ? s_tile[0] : kNoTile;
+      __syncthreads();
     }
   }
   if (!grid_barrier(cb.ctl, G, info)) return;
@@ -2184,12 +2217,12 @@ ba_cholesky_kernel(int n, float lm, float ep, BaPtrs w, CholBuf cb, float* __res
 // right-hand side per block.  Entries (r, c) of a block sit at column c ^ 2 (r mod 8): pairs stay aligned, and
 // neither a column nor an MMA fragment meets a bank conflict beyond its size.
 // Bound by the chain factor + row products + diagonal update per 16 columns.
-// Measured with its launch (one / many CTAs): 17 / 33 us at 36 unknowns, 27 / 78 at 96, 41 / 115
-// at 138, 62 / 125 at 180; from there the one SM's FP64 rate adds up: 82 / 110 at 222.
+// Measured with its launch (one / many CTAs): 17 / 30 us at 36 unknowns, 27 / 52 at 96, 39 / 63
+// at 138, 61 / 69 at 180; from there the one SM's FP64 rate adds up: 78 / 79 at 222.
 constexpr int kSmallMax = 224;
 constexpr int kSmallThreads = 512;
 __host__ __device__ constexpr size_t small_smem(int nb) {
-  return sizeof(double) * ((size_t)nb * (nb + 1) / 2 * 256 + 3 * (size_t)nb * 16 + 72);
+  return sizeof(double) * ((size_t)nb * (nb + 1) / 2 * 256 + 3 * (size_t)nb * 16 + 108);
 }
 
 __device__ __forceinline__ int small_at(int I, int J, int r, int c) {
@@ -2206,7 +2239,7 @@ ba_solve_small_kernel(int n, float lm, float ep, BaPtrs w, float* __restrict__ d
   double* bv = S + nb * (nb + 1) / 2 * 256;      // [N] right-hand side, then y, then x
   double* sv = bv + N;                           // [N] 1 / L_jj
   double* xv = sv + N;                           // [N] solution
-  double* xc = xv + N;                           // [72] column exchange of the factor
+  double* xc = xv + N;                           // [108] column exchange of the factor
   __shared__ int sfail;
   // entries (r, c) and (r, c + 1) of the damped, padded system
   auto entry2 = [&](int r, int c) {
@@ -2243,7 +2276,7 @@ ba_solve_small_kernel(int n, float lm, float ep, BaPtrs w, float* __restrict__ d
     }
   }
   auto factor = [&](int k) {
-    chol_factor_diag([&](int r, int c) -> double& { return S[small_at(k, k, r, c)]; }, bv + 16 * k, sv + 16 * k, xc, 16,
+    chol_factor_diag<false>([&](int r, int c) -> double& { return S[small_at(k, k, r, c)]; }, bv + 16 * k, sv + 16 * k, xc, 16,
                      &sfail);
   };
   // S(I, J) -= X_I X_J^T with X = column block k, by one warp
@@ -2281,7 +2314,7 @@ ba_solve_small_kernel(int n, float lm, float ep, BaPtrs w, float* __restrict__ d
       double x[4];
       chol_solve_rows([&](int r, int c) -> double& { return S[small_at(I, k, h0 + r, c)]; },
                       [&](int l, int c) -> double {
-                        return l > c ? 0.0 : l == c ? sv[16 * k + l] : S[small_at(k, k, l, c)];
+                        return l > c ? 0.0 : S[small_at(k, k, l, c)];
                       }, x);
       const double* yk = bv + 16 * k + 2 * (lane & 3);
       double acc = fma(x[0], yk[0], x[1] * yk[1]) + fma(x[2], yk[8], x[3] * yk[9]);
@@ -2323,7 +2356,7 @@ ba_solve_small_kernel(int n, float lm, float ep, BaPtrs w, float* __restrict__ d
   for (int k = nb - 1; k >= 0; --k) {
     if (tid < 256) {                                   // 16 lanes per row of L_kk^-T
       const int c = tid >> 4, r = tid & 15;
-      double v = r < c ? 0.0 : (r == c ? sv[16 * k + r] : S[small_at(k, k, c, r)]) * bv[16 * k + r];
+      double v = r < c ? 0.0 : S[small_at(k, k, c, r)] * bv[16 * k + r];
 #pragma unroll
       for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
       if (r == 0) xv[16 * k + c] = v;
@@ -2489,8 +2522,8 @@ static int run_cholesky(int n, float lm, float ep, BaPtrs w, CholBuf cb, float* 
                         cudaStream_t s) {
   if (n == 0) return HS2_OK;
   HS2_PROF("ba_cholesky", s);
-  // up to kSmallMax unknowns (the whole triangle fits one CTA's shared memory, and one CTA is still
-  // the faster: 82 us against about 110 us at 222) no other CTA takes part
+  // up to kSmallMax unknowns (the whole triangle fits one CTA's shared memory, and one CTA is no
+  // slower: 39 against 63 us at 138, 78.5 against 78.6 at 222) no other CTA takes part
   if (n <= kSmallMax) {
     static DeviceOnce small_once;
     int dev = 0;
@@ -2506,8 +2539,8 @@ static int run_cholesky(int n, float lm, float ep, BaPtrs w, CholBuf cb, float* 
     return HS2_OK;
   }
   const int nbk = (n + kNB - 1) / kNB;
-  // panel: [128][kPLD] + b, 1/L_jj, exchange; tile: [192][kPLD]; backward: 2 x 64 x 64 + 256
-  const size_t smem = sizeof(double) * std::max<size_t>(128 * kPLD + 128 + 64 + 72 + 2, 192 * kPLD);
+  // the panel's rows + b, 1/L_jj, exchange; two tile tasks; backward: 2 x 64 x 64 + 512
+  const size_t smem = sizeof(double) * std::max<size_t>(kPanelDoubles, 2 * kTileDoubles);
   static DeviceOnce once;
   static std::atomic<int> grid_cap[kMaxDevices];
   int dev = 0;
@@ -2521,7 +2554,7 @@ static int run_cholesky(int n, float lm, float ep, BaPtrs w, CholBuf cb, float* 
     return HS2_OK;
   });
   if (rc) return rc;
-  const int work = std::max(std::max(nbk, (nbk - 1) * nbk / 2), (n + kCholThreads - 1) / kCholThreads);
+  const int work = std::max(1 + kXSplit * (nbk - 1) + (nbk - 1) * (nbk - 2) / 2, (n + kCholThreads - 1) / kCholThreads);
   int G = std::max(1, std::min(grid_cap[dev].load(std::memory_order_relaxed), work));
   HS2_CUDA(cudaMemsetAsync(cb.ctl, 0, (kCtlFlags + 3 * (size_t)nbk + (size_t)nbk * nbk) * sizeof(unsigned), s));
   void* args[] = {&n, &lm, &ep, &w, &cb, &dx, &info};
