@@ -738,8 +738,8 @@ def pgba_leg(args, dev, world, rank):
 
 
 def jdsa_leg(args, dev, world, rank):
-    """The mono-prior alignment step (hislam2_b200.mono.JDSA, one hs2_jdsa call: proj_trans
-    plus the per-frame scale solve and depth update) on HI-SLAM2's frontend window, 25
+    """The mono-prior alignment step (hislam2_b200.mono.JDSA, one hs2_jdsa call:
+    its C, w, the per-frame scale solve and the depth update) on HI-SLAM2's frontend window, 25
     keyframes at 43x77 with 258 edges and its 2x2 scale grid per frame, device-timed."""
     from hislam2_b200 import _lib, mono, replicas, synth
 
@@ -770,7 +770,7 @@ def jdsa_leg(args, dev, world, rank):
     ms = max_over_ranks(e0.elapsed_time(e1), world, dev) / args.steps
     return {"value": round(world * 1e3 / ms, 2), "unit": "JDSA steps/s", "ms_per_step": round(ms, 4),
             "config": "frontend window: 25 kf, 43x77, 258 edges, 2x2 scale grid, alpha 0.01; the step's "
-                      "host sync (torch.unique, info read) included",
+                      "host sync (info read) included",
             "kernel_ms_per_step": {k: round(v[1] / args.steps, 4) for k, v in sorted(prof.items())}}
 
 

@@ -11,22 +11,38 @@
 // the two are the same frame whenever kx is contiguous, and this pairing is what the
 // reference computes when it is not.
 //
-//   proj_trans         (geometry.cu) the depth-only Schur terms C, w [M, HW];
-//   jdsa_solve         CTA per block b: per pixel, in FP32 as the reference,
+//   jdsa_keys          kx and slot of the edges from a bitmap of the frames, one CTA: a list of a
+//                      few hundred edges needs no sort, and the count stays on the device;
+//   jdsa_step          cluster of 8 CTAs per block b, pixels dealt out in runs of a CTA: per
+//                      pixel the depth-only Schur terms C, w summed over the block's edges in
+//                      their order (proj_trans's terms, geometry.cu); then, in FP32 as the
+//                      reference,
 //                        Q = 1 / (C + m alpha + (1 - m) eta),  w' = w - m alpha rd,
 //                        a = prior [> 0] of the source frame, J = -a (wa, wb, wc, wd) at the
 //                        pixel's interpolation cell,
-//                      summed in FP64 per cell over the CTA: S += alpha a^2 (1 - alpha Q) w w^T,
+//                      summed in FP64 per cell over the cluster: S += alpha a^2 (1 - alpha Q) w w^T,
 //                      diag(H) += alpha a^2 w^2, v += alpha a w (rd_src + Q w'); then
-//                      S + diag(0.1 + 1e-4 diag(H)) = L L^T in FP64 by one thread (D <= 16),
+//                      S + diag(0.1 + 1e-4 diag(H)) = L L^T in FP64 by one warp (D <= 16),
 //                      dso = S^-1 v; second pass: dz = Q (w' + alpha a (w . dso_cell)),
 //                      disps_out = clamp(where(d + dz > 10, 0, d + dz), min = 0.001) and
 //                      dzcov = (alpha a Q)^2 w^T S^-1_cell w + Q  (= |L^-1 E Q|^2 + Q).
-//                      CTAs M .. M + num_disps - 1 copy the frames that are not source frames
-//                      through the same where / clamp (the reference applies both to the
-//                      whole window).
+//                      The clusters behind the M blocks copy the frames that are not source
+//                      frames through the same where / clamp (the reference applies both to
+//                      the whole window).
 //   jdsa_scales        dscales[kx[b]] += dso[b], skipped when a block was not positive
 //                      definite or an index was bad (the reference raises before it).
+//
+// Bound by latency: 25 frames of 3311 pixels are 14 MB, 2 us of HBM.  One CTA per frame took
+// 13 pixels a thread through two passes behind a launch of atomics that summed C and w; eight
+// CTAs a frame take two pixels a thread, keep the sums of an edge list they scan themselves
+// (no zeroed buffers, no atomics, a fixed order) and meet once, in distributed shared memory.
+// 25 frames at 43x77, 258 edges, 2x2 grid: a call of mono.JDSA 183 -> 118 us (most of it the
+// keys, which torch.unique made behind two waits of the host; the kernels 61 -> 54 us), of
+// which the host's own work is half.
+#include <utility>
+
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 #include "profile.cuh"
 
@@ -36,18 +52,33 @@ namespace {
 
 constexpr int kJdThreads = 256;
 constexpr int kJdWarps = kJdThreads / 32;
+constexpr int kJdCluster = 8;      // CTAs of one block: the portable cluster size
+constexpr int kJdBatch = 64;       // edges whose relative poses are in shared memory at a time
 constexpr int kJdMaxD = 16;
+constexpr int kJdMaxCells = 9;     // (hs - 1)(ws - 1) for hs ws <= 16
 constexpr int kJdSums = 18;        // one cell: 10 Gram terms, 4 diag(H) terms, 4 rhs terms
 constexpr int kJdMaxAxis = 4096;   // ht, wd (the grid axes are staged in shared memory)
 constexpr double kJdEp = 0.1;      // schur_solve_mono_prior's ep and lm (chol.py:80)
 constexpr double kJdLm = 1e-4;
+constexpr int kJdKeyThreads = 1024;
+constexpr int kJdKeyFrames = 65536;   // frames of the bitmap (8 KB of shared memory)
+constexpr unsigned kJdCopyClusters = 1024;
 
 struct JdArgs {
+  const float* poses;
+  int64_t num_poses;
+  const float* intr;
+  const float* targets;
+  const float* weights;
+  const int64_t* ii;
+  const int64_t* jj;
+  const int64_t* slot;
+  int64_t num_edges;
   const float* disps;
   int64_t num_disps;
   int ht, wd;
-  const float* C;
-  const float* w;
+  float* C;   // a pixel's sums are written and read by one thread
+  float* w;
   const float* eta;
   const float* prior;
   int64_t num_prior;
@@ -128,18 +159,139 @@ __device__ __forceinline__ RowTerms row_terms(const JdArgs& A, int b, int64_t fr
   return t;
 }
 
+// An edge of the block as its pixels need it: Gij as a matrix and the disparities of its source frame.
+struct JdEdge {
+  float t[3], R[9];
+  int e;
+  const float* d;
+};
+
+// An edge outside the buffers marks the step as invalid and stands for frame fr, identity: nothing
+// is read out of bounds and the loop over the edges needs no test.
+__device__ __forceinline__ JdEdge load_edge(const JdArgs& A, int e, int64_t fr, int HW) {
+  JdEdge g;
+  const int64_t ix = A.ii[e], jx = A.jj[e];
+  if (ix < 0 || jx < 0 || ix >= A.num_poses || jx >= A.num_poses || ix >= A.num_disps) {
+    atomicOr(A.info, HS2_DEV_BAD_INDEX);
+    for (int i = 0; i < 3; ++i) g.t[i] = 0.f;
+    for (int i = 0; i < 9; ++i) g.R[i] = i % 4 ? 0.f : 1.f;
+    g.e = e;
+    g.d = A.disps + fr * HW;
+    return g;
+  }
+  const float* pi = A.poses + 7 * ix;
+  const float* pj = A.poses + 7 * jx;
+  float q[4];
+  relative_pose(pi, pi + 3, pj, pj + 3, g.t, q);
+  // quat_rotate's I + 2 w [v] + 2 [v]^2, one rounding an entry
+  const double x = q[0], y = q[1], z = q[2], w = q[3];
+  g.R[0] = (float)(1.0 - 2.0 * (y * y + z * z));
+  g.R[1] = (float)(2.0 * (x * y - w * z));
+  g.R[2] = (float)(2.0 * (x * z + w * y));
+  g.R[3] = (float)(2.0 * (x * y + w * z));
+  g.R[4] = (float)(1.0 - 2.0 * (x * x + z * z));
+  g.R[5] = (float)(2.0 * (y * z - w * x));
+  g.R[6] = (float)(2.0 * (x * z - w * y));
+  g.R[7] = (float)(2.0 * (y * z + w * x));
+  g.R[8] = (float)(1.0 - 2.0 * (x * x + y * y));
+  g.e = e;
+  g.d = A.disps + ix * HW;
+  return g;
+}
+
+// a / b from the correctly rounded r = 1 / b: the quotient and one Newton correction of its remainder.
+__device__ __forceinline__ float quotient(float a, float b, float r) {
+  const float q = a * r;
+  return fmaf(fmaf(-q, b, a), r, q);
+}
+
+// proj_trans's terms of NP pixels (k, k + kJdThreads) over n edges, added to C and w; the loads of four
+// edges are in flight together.  Bound by instruction issue: with a division for each of x, y and
+// the depth and the rotation by the quaternion, the 10 edges of a frame took 7 us.
+template <int NP>
+__device__ __forceinline__ void add_edges(const JdArgs& A, const JdEdge* edges, int n, int HW, int k, bool first,
+                                          float* Cm, float* wm) {
+  const float fx = A.intr[0], fy = A.intr[1], cx = A.intr[2], cy = A.intr[3];
+  float X[NP][2], C[NP], w[NP];
+#pragma unroll
+  for (int p = 0; p < NP; ++p) {
+    const int kp = k + p * kJdThreads, vi = kp / A.wd;
+    X[p][0] = ((float)(kp - vi * A.wd) - cx) / fx;
+    X[p][1] = ((float)vi - cy) / fy;
+    C[p] = first ? 0.f : Cm[kp];
+    w[p] = first ? 0.f : wm[kp];
+  }
+  for (int j0 = 0; j0 < n; j0 += 4) {
+    float h[4][NP], tu[4][NP], tv[4][NP], gu[4][NP], gv[4][NP];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const JdEdge& g = edges[min(j0 + q, n - 1)];
+      const float* trg = A.targets + (int64_t)g.e * 2 * HW;
+      const float* wgt = A.weights + (int64_t)g.e * 2 * HW;
+#pragma unroll
+      for (int p = 0; p < NP; ++p) {
+        const int kp = k + p * kJdThreads;
+        h[q][p] = g.d[kp];
+        tu[q][p] = trg[kp];
+        tv[q][p] = trg[HW + kp];
+        gu[q][p] = wgt[kp];
+        gv[q][p] = wgt[HW + kp];
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      if (j0 + q >= n) break;
+      const JdEdge& g = edges[j0 + q];
+#pragma unroll
+      for (int p = 0; p < NP; ++p) {
+        float Y[3];
+#pragma unroll
+        for (int r = 0; r < 3; ++r)
+          Y[r] = fmaf(g.R[3 * r], X[p][0], fmaf(g.R[3 * r + 1], X[p][1], fmaf(h[q][p], g.t[r], g.R[3 * r + 2])));
+        const bool bad = Y[2] < kMinDepth;
+        const float d = bad ? 0.f : 1.0f / Y[2];
+        const float xp = fx * quotient(Y[0], Y[2], d) + cx, yp = fy * quotient(Y[1], Y[2], d) + cy;
+        const float d2 = d * d;
+        const float wu = bad ? 0.f : 0.001f * gu[q][p];
+        const float wv = bad ? 0.f : 0.001f * gv[q][p];
+        const float ru = tu[q][p] - xp, rv = tv[q][p] - yp;
+        const float Jzu = fx * d * g.t[0] + fx * (-Y[0] * d2) * g.t[2];
+        const float Jzv = fy * d * g.t[1] + fy * (-Y[1] * d2) * g.t[2];
+        C[p] += wu * Jzu * Jzu + wv * Jzv * Jzv;
+        w[p] += wu * ru * Jzu + wv * rv * Jzv;
+      }
+    }
+  }
+#pragma unroll
+  for (int p = 0; p < NP; ++p) {
+    Cm[k + p * kJdThreads] = C[p];
+    wm[k + p * kJdThreads] = w[p];
+  }
+}
+
+// One exchange of block_sum over the first n of acc, and the ones after it.
+template <int n, int off, int N>
+__device__ __forceinline__ void warp_halve(double (&acc)[N], int& at, int& have) {
+  constexpr int h = (n + 1) / 2;
+  const bool up = threadIdx.x & off;
+#pragma unroll
+  for (int i = 0; i < h; ++i) {
+    const double lo = acc[i], hi = h + i < n ? acc[h + i] : 0.0;
+    acc[i] = (up ? hi : lo) + __shfl_xor_sync(0xffffffffu, up ? lo : hi, off);
+  }
+  at += up ? h : 0;
+  have = up ? have - h : min(have, h);
+  if constexpr (off > 1) warp_halve<h, off / 2>(acc, at, have);
+}
+
+// Sums of acc over the CTA into tot[0 .. N).  The warp halves the list at every exchange (a lane keeps
+// one half and sends the other), 20 exchanges of doubles for 18 sums where five rounds of all are 90.
 template <int N>
 __device__ __forceinline__ void block_sum(double (&acc)[N], double (*red)[N], double* tot) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int i = 0; i < N; ++i) {
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) acc[i] += __shfl_down_sync(0xffffffffu, acc[i], off);
-  }
-  if (lane == 0) {
-#pragma unroll
-    for (int i = 0; i < N; ++i) red[warp][i] = acc[i];
-  }
+  const int warp = threadIdx.x >> 5;
+  int at = 0, have = N;   // this lane's run of the list: start and entries that are not padding
+  warp_halve<N, 16>(acc, at, have);
+  if (have > 0) red[warp][at] = acc[0];
   __syncthreads();
   if (threadIdx.x < N) {
     double s = 0.0;
@@ -149,33 +301,75 @@ __device__ __forceinline__ void block_sum(double (&acc)[N], double (*red)[N], do
   __syncthreads();
 }
 
-__global__ void __launch_bounds__(kJdThreads)
-jdsa_solve_kernel(const JdArgs A) {
+// S + diag(ep + lm Hd) = L L^T in place and x = S^-1 v by one warp, a lane for each row and parity of the
+// column; the diagonal of S ends as 1 / L_kk, so that one reciprocal square root is all that a step
+// waits for.  Loops stay rolled: each runs once a launch, and fetching unrolled code took longer
+// than the arithmetic (4 unknowns: 14k cycles against 5.7k).  False when a pivot is not positive.
+__device__ __forceinline__ bool warp_solve(int D, double (*S)[kJdMaxD + 1], const double* Hd, double v, double& x) {
+  const int lane = threadIdx.x & 31, row = lane & 15, odd = lane >> 4;
+  if (lane < D) S[lane][lane] += kJdEp + kJdLm * Hd[lane];
+  __syncwarp();
+#pragma unroll 1
+  for (int k = 0; k < D; ++k) {
+    const double piv = S[k][k];
+    if (!(piv > 0.0)) return false;
+    const double r = rsqrt(piv);
+    const double lk = row > k && row < D ? S[row][k] * r : 0.0;
+    const double y = __shfl_sync(0xffffffffu, v, k) * r;
+    v = lane == k ? y : lane > k && lane < D ? v - lk * y : v;
+    __syncwarp();
+    if (!odd && row < D && row >= k) S[row][k] = row == k ? r : lk;
+    __syncwarp();
+#pragma unroll 1
+    for (int l = k + 1 + odd; l < D; l += 2)
+      if (row >= l && row < D) S[row][l] -= lk * S[l][k];
+    __syncwarp();
+  }
+#pragma unroll 1
+  for (int k = D - 1; k >= 0; --k) {
+    const double y = __shfl_sync(0xffffffffu, v, k) * S[k][k];
+    v = lane == k ? y : lane < k ? v - S[k][lane] * y : v;
+  }
+  x = v;
+  return true;
+}
+
+__global__ void __cluster_dims__(kJdCluster, 1, 1) __launch_bounds__(kJdThreads, 2)
+jdsa_step_kernel(const JdArgs A) {
   extern __shared__ float jd_axes[];   // gy [ht] then gx [wd]
   __shared__ double red[kJdWarps][kJdSums];
-  __shared__ double tot[kJdSums];
+  __shared__ double part[kJdMaxCells * kJdSums];   // this CTA's sums, read by the whole cluster
+  __shared__ double tot[kJdMaxCells * kJdSums];
   __shared__ double S[kJdMaxD][kJdMaxD + 1];
-  __shared__ double Lc[kJdMaxD][kJdMaxD + 1];
   __shared__ double Li[kJdMaxD][kJdMaxD + 1];
   __shared__ double Hd[kJdMaxD], v[kJdMaxD];
   __shared__ float dso[kJdMaxD];
   __shared__ float Si[kJdMaxD][kJdMaxD + 1];
   __shared__ float sc_r[kJdMaxD], sc_s[kJdMaxD];
+  __shared__ JdEdge edges[kJdBatch];
+  __shared__ int list[kJdBatch + kJdThreads];
+  __shared__ int found[kJdWarps];
   __shared__ int bad, failed;
-  const int HW = A.ht * A.wd, D = A.hs * A.ws, tid = threadIdx.x;
-  const int g = blockIdx.x;
-  if (g >= A.M) {
-    // a frame of the window that is not a source frame: the where / clamp only
-    const int64_t f = g - A.M;
-    if (find_sorted(A.kx, A.M, f) >= 0) return;
-    const float* src = A.disps + f * HW;
-    float* dst = A.out + f * HW;
-    for (int k = tid; k < HW; k += kJdThreads) dst[k] = jd_clean(src[k]);
+  const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+  const int HW = A.ht * A.wd, D = A.hs * A.ws, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int rank = (int)cluster.block_rank();
+  const int b = blockIdx.x / kJdCluster;
+  // an equal run of pixels for each CTA, in whole warps
+  const int run = (HW / kJdCluster + 32) / 32 * 32, k0 = rank * run + tid, kend = min(HW, (rank + 1) * run);
+  if (b >= A.M) {
+    // frames of the window that are not source frames: the where / clamp only
+    const int step = gridDim.x / kJdCluster - A.M;
+    for (int64_t f = b - A.M; f < A.num_disps; f += step) {
+      if (find_sorted(A.kx, A.M, f) >= 0) continue;
+      const float* src = A.disps + f * HW;
+      float* dst = A.out + f * HW;
+      for (int k = k0; k < kend; k += kJdThreads) dst[k] = jd_clean(src[k]);
+    }
     return;
   }
-  const int b = g;
-  const int64_t fr = A.kx[b];
-  const int ms = find_sorted(A.kx, A.M, A.kx[0] + b);   // source of block b's prior terms
+  // every CTA of a cluster comes to the same verdict here, so none waits for one that left
+  const int64_t fr = A.kx[b], want = A.kx[0] + b;
+  const int ms = fr == want ? b : find_sorted(A.kx, A.M, want);   // source of block b's prior terms
   const int64_t fs = ms >= 0 ? A.kx[ms] : fr;
   if (tid == 0) {
     bad = fr < 0 || fr >= A.num_disps || fr >= A.num_prior || fr >= A.num_scales || (b > 0 && A.kx[b - 1] >= fr) ||
@@ -187,8 +381,6 @@ jdsa_solve_kernel(const JdArgs A) {
   for (int i = tid; i < A.ht; i += kJdThreads) gy[i] = A.gy[i];
   for (int j = tid; j < A.wd; j += kJdThreads) gx[j] = A.gx[j];
   if (tid < D) {
-    sc_r[tid] = A.dscales[fr * D + tid];
-    sc_s[tid] = A.dscales[fs * D + tid];
     Hd[tid] = 0.0;
     v[tid] = 0.0;
   }
@@ -205,110 +397,141 @@ jdsa_solve_kernel(const JdArgs A) {
     if (tid == 0) atomicOr(A.info, HS2_DEV_BAD_INDEX);
     return;
   }
-  const bool has_src = ms >= 0;
-  const float alpha = A.alpha;
-
-  // ---- pass 1: the block's Schur complement and right-hand side, cell by cell
-  for (int cy = 0; cy < A.hs - 1; ++cy) {
-    for (int cx = 0; cx < A.ws - 1; ++cx) {
-      double acc[kJdSums];
-#pragma unroll
-      for (int i = 0; i < kJdSums; ++i) acc[i] = 0.0;
-      if (has_src) {
-        for (int k = tid; k < HW; k += kJdThreads) {
-          const int i = k / A.wd, j = k - i * A.wd;
-          if ((int)floorf(gy[i]) != cy || (int)floorf(gx[j]) != cx) continue;
-          const Cell c = make_cell(gx[j], gy[i], cx, cy, A.ws);
-          const RowTerms r = row_terms(A, b, fr, HW, k, sc_r, c);
-          const int64_t sk = fs * HW + k;
-          const float ps = A.prior[sk];
-          const float a = ps > 0.f ? ps : 0.f;
-          const float rds = A.disps[sk] - ps * interp(sc_s, c);
-          const double ca = (double)(alpha * a * a * (1.0f - alpha * r.Q));
-          const double ha = (double)(alpha * a * a);
-          const double va = (double)(alpha * a * (rds + r.Q * r.wq));
-          int q = 0;
-#pragma unroll
-          for (int kk = 0; kk < 4; ++kk) {
-#pragma unroll
-            for (int ll = kk; ll < 4; ++ll) acc[q++] += ca * c.wt[kk] * c.wt[ll];
-          }
-#pragma unroll
-          for (int kk = 0; kk < 4; ++kk) {
-            acc[10 + kk] += ha * c.wt[kk] * c.wt[kk];
-            acc[14 + kk] += va * c.wt[kk];
-          }
-        }
-      }
-      block_sum<kJdSums>(acc, red, tot);
-      if (tid < kJdSums) {
-        const int p0 = cy * A.ws + cx;
-        const int pos[4] = {p0, p0 + A.ws, p0 + 1, p0 + A.ws + 1};
-        if (tid < 10) {
-          int kk = 0, q = tid;
-          while (q >= 4 - kk) { q -= 4 - kk; ++kk; }
-          const int ll = kk + q;
-          S[pos[kk]][pos[ll]] += tot[tid];
-          if (ll != kk) S[pos[ll]][pos[kk]] += tot[tid];
-        } else if (tid < 14) {
-          Hd[pos[tid - 10]] += tot[tid];
-        } else {
-          v[pos[tid - 14]] += tot[tid];
-        }
-      }
-      __syncthreads();
-    }
+  if (tid < D) {
+    sc_r[tid] = A.dscales[fr * D + tid];
+    sc_s[tid] = A.dscales[fs * D + tid];
   }
 
-  // ---- damped D x D solve in FP64 (one thread; D <= 16)
-  if (tid == 0) {
-    bool ok = true;
-    for (int k = 0; k < D && ok; ++k) {
-      for (int l = 0; l <= k; ++l) {
-        double s = S[k][l] + (k == l ? kJdEp + kJdLm * Hd[k] : 0.0);
-        for (int m = 0; m < l; ++m) s -= Lc[k][m] * Lc[l][m];
-        if (l == k) {
-          if (!(s > 0.0)) { ok = false; break; }
-          Lc[k][k] = sqrt(s);
-        } else {
-          Lc[k][l] = s / Lc[l][l];
+  // ---- C and w of this thread's pixels: the edges of slot b in their order
+  float* Cm = A.C + (int64_t)b * HW;
+  float* wm = A.w + (int64_t)b * HW;
+  const int E = (int)A.num_edges;
+  int num = 0;         // edges in `list`
+  bool first = true;
+  for (int base = 0; base < E; base += kJdThreads) {
+    const int e = base + tid;
+    const int64_t m = e < E ? A.slot[e] : b + 1;
+    if (e < E && (m < 0 || m >= A.M)) atomicOr(A.info, HS2_DEV_BAD_INDEX);
+    const unsigned mine = __ballot_sync(0xffffffffu, m == b);
+    if (lane == 0) found[warp] = __popc(mine);
+    __syncthreads();
+    int at = num;
+    for (int q = 0; q < kJdWarps; ++q) {
+      if (q == warp && m == b) list[at + __popc(mine & ((1u << lane) - 1))] = e;
+      at += found[q];
+    }
+    num = at;
+    __syncthreads();
+    if (num <= kJdBatch && base + kJdThreads < E) continue;
+    for (int s = 0; s < num; s += kJdBatch) {
+      const int n = min(kJdBatch, num - s);
+      if (tid < n) edges[tid] = load_edge(A, list[s + tid], fr, HW);
+      __syncthreads();
+      int k = k0;
+      for (; k + kJdThreads < kend; k += 2 * kJdThreads) add_edges<2>(A, edges, n, HW, k, first, Cm, wm);
+      if (k < kend) add_edges<1>(A, edges, n, HW, k, first, Cm, wm);
+      first = false;
+      __syncthreads();
+    }
+    num = 0;
+  }
+  if (first)
+    for (int k = k0; k < kend; k += kJdThreads) Cm[k] = wm[k] = 0.f;
+  __syncthreads();   // sc_r, sc_s
+
+  const bool has_src = ms >= 0;
+  const float alpha = A.alpha;
+  // ---- pass 1: the block's Schur complement and right-hand side, cell by cell
+  const int cells = (A.hs - 1) * (A.ws - 1);
+  for (int cell = 0; cell < cells; ++cell) {
+    const int cy = cell / (A.ws - 1), cx = cell - cy * (A.ws - 1);
+    double acc[kJdSums];
+#pragma unroll
+    for (int i = 0; i < kJdSums; ++i) acc[i] = 0.0;
+    if (has_src) {
+      for (int k = k0; k < kend; k += kJdThreads) {
+        const int i = k / A.wd, j = k - i * A.wd;
+        if ((int)floorf(gy[i]) != cy || (int)floorf(gx[j]) != cx) continue;
+        const Cell c = make_cell(gx[j], gy[i], cx, cy, A.ws);
+        const RowTerms r = row_terms(A, b, fr, HW, k, sc_r, c);
+        const int64_t sk = fs * HW + k;
+        const float ps = A.prior[sk];
+        const float a = ps > 0.f ? ps : 0.f;
+        const float rds = A.disps[sk] - ps * interp(sc_s, c);
+        const double ca = (double)(alpha * a * a * (1.0f - alpha * r.Q));
+        const double ha = (double)(alpha * a * a);
+        const double va = (double)(alpha * a * (rds + r.Q * r.wq));
+        int q = 0;
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk) {
+#pragma unroll
+          for (int ll = kk; ll < 4; ++ll) acc[q++] += ca * c.wt[kk] * c.wt[ll];
+        }
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk) {
+          acc[10 + kk] += ha * c.wt[kk] * c.wt[kk];
+          acc[14 + kk] += va * c.wt[kk];
         }
       }
     }
-    double y[kJdMaxD];
-    if (ok) {
-      for (int k = 0; k < D; ++k) {
-        double s = v[k];
-        for (int m = 0; m < k; ++m) s -= Lc[k][m] * y[m];
-        y[k] = s / Lc[k][k];
+    block_sum<kJdSums>(acc, red, part + cell * kJdSums);
+  }
+  // the cluster's sums, added in the order of its CTAs by each of them
+  cluster.sync();
+  for (int i = tid; i < cells * kJdSums; i += kJdThreads) {
+    double s = 0.0;
+#pragma unroll
+    for (int q = 0; q < kJdCluster; ++q) s += cluster.map_shared_rank(part, q)[i];
+    tot[i] = s;
+  }
+  auto read = cluster.barrier_arrive();   // waited for before this CTA's shared memory goes away
+  __syncthreads();
+
+  // ---- damped D x D solve in FP64 by the first warp
+  if (warp == 0) {
+    for (int cell = 0; cell < cells; ++cell) {
+      if (lane < kJdSums) {
+        const int cy = cell / (A.ws - 1), p0 = cy * A.ws + cell - cy * (A.ws - 1);
+        const int pos[4] = {p0, p0 + A.ws, p0 + 1, p0 + A.ws + 1};
+        const double t = tot[cell * kJdSums + lane];
+        if (lane < 10) {
+          int kk = 0, q = lane;
+          while (q >= 4 - kk) { q -= 4 - kk; ++kk; }
+          const int ll = kk + q;
+          S[pos[kk]][pos[ll]] += t;
+          if (ll != kk) S[pos[ll]][pos[kk]] += t;
+        } else if (lane < 14) {
+          Hd[pos[lane - 10]] += t;
+        } else {
+          v[pos[lane - 14]] += t;
+        }
       }
-      for (int k = D - 1; k >= 0; --k) {
-        double s = y[k];
-        for (int m = k + 1; m < D; ++m) s -= Lc[m][k] * y[m];
-        y[k] = s / Lc[k][k];
-      }
+      __syncwarp();
     }
-    for (int k = 0; k < D; ++k) {
-      dso[k] = ok ? (float)y[k] : 0.f;
-      A.dso[(int64_t)b * D + k] = dso[k];
+    double x = 0.0;
+    const bool ok = warp_solve(D, S, Hd, lane < D ? v[lane] : 0.0, x);
+    if (lane < D) {
+      dso[lane] = ok ? (float)x : 0.f;
+      if (rank == 0) A.dso[(int64_t)b * D + lane] = dso[lane];
     }
-    if (!ok) {
+    if (!ok && lane == 0) {
       failed = 1;
       atomicOr(A.info, HS2_DEV_NOT_PD);
+    }
+    // columns of L^-1 by forward substitution (lane k: L x = e_k)
+    if (A.dzcov && ok && lane < D) {
+#pragma unroll 1
+      for (int i = 0; i < D; ++i) {
+        double t = i == lane ? 1.0 : 0.0;
+#pragma unroll 1
+        for (int m = lane; m < i; ++m) t -= S[i][m] * Li[m][lane];
+        Li[i][lane] = i < lane ? 0.0 : t * S[i][i];
+      }
     }
   }
   __syncthreads();
   if (A.dzcov) {
-    // columns of L^-1 by forward substitution (thread k: L x = e_k), then S^-1 = L^-T L^-1
-    if (tid < D && !failed) {
-      const int k = tid;
-      for (int i = 0; i < D; ++i) {
-        double s = i == k ? 1.0 : 0.0;
-        for (int m = k; m < i; ++m) s -= Lc[i][m] * Li[m][k];
-        Li[i][k] = i < k ? 0.0 : s / Lc[i][i];
-      }
-    }
-    __syncthreads();
+    // S^-1 = L^-T L^-1
     for (int e = tid; e < D * D; e += kJdThreads) {
       const int k = e / D, l = e - k * D;
       double s = 0.0;
@@ -319,10 +542,10 @@ jdsa_solve_kernel(const JdArgs A) {
     __syncthreads();
   }
 
-  // ---- pass 2: depth update, clean-up and covariance of every pixel of frame fr
+  // ---- pass 2: depth update, clean-up and covariance of this thread's pixels of frame fr
   float* outr = A.out + fr * HW;
   float* cov = A.dzcov ? A.dzcov + (int64_t)b * HW : nullptr;
-  for (int k = tid; k < HW; k += kJdThreads) {
+  for (int k = k0; k < kend; k += kJdThreads) {
     const int i = k / A.wd, j = k - i * A.wd;
     const int cy = (int)floorf(gy[i]), cx = (int)floorf(gx[j]);
     const Cell c = make_cell(gx[j], gy[i], cx, cy, A.ws);
@@ -347,6 +570,60 @@ jdsa_solve_kernel(const JdArgs A) {
       cov[k] = e * e * quad + r.Q;
     }
   }
+  cluster.barrier_wait(std::move(read));
+}
+
+// kx, slot and the number of distinct frames from a bitmap over the frames.
+__global__ void __launch_bounds__(kJdKeyThreads)
+jdsa_keys_kernel(const int64_t* __restrict__ ii, int E, int frames, int M, int64_t* __restrict__ kx,
+                 int64_t* __restrict__ slot, int32_t* __restrict__ count) {
+  constexpr int kWords = kJdKeyFrames / 32, kPer = kWords / kJdKeyThreads;
+  __shared__ unsigned bits[kWords];
+  __shared__ int before[kWords];   // distinct frames ahead of the word
+  __shared__ int sums[kJdKeyThreads / 32];
+  __shared__ int outside;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  for (int i = tid; i < kWords; i += kJdKeyThreads) bits[i] = 0;
+  if (tid == 0) outside = 0;
+  __syncthreads();
+  for (int e = tid; e < E; e += kJdKeyThreads) {
+    const int64_t f = ii[e];
+    if (f >= 0 && f < frames) atomicOr(&bits[f >> 5], 1u << (f & 31));
+    else outside = 1;
+  }
+  __syncthreads();
+  int n = 0;
+#pragma unroll
+  for (int i = 0; i < kPer; ++i) n += __popc(bits[tid * kPer + i]);
+  int scan = n;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const int up = __shfl_up_sync(0xffffffffu, scan, off);
+    if (lane >= off) scan += up;
+  }
+  if (lane == 31) sums[warp] = scan;
+  __syncthreads();
+  int at = scan - n, total = 0;
+  for (int q = 0; q < kJdKeyThreads / 32; ++q) {
+    if (q < warp) at += sums[q];
+    total += sums[q];
+  }
+#pragma unroll
+  for (int i = 0; i < kPer; ++i) {
+    const int word = tid * kPer + i;
+    before[word] = at;
+    for (unsigned left = bits[word]; left; left &= left - 1, ++at)
+      if (at < M) kx[at] = word * 32 + __ffs(left) - 1;
+  }
+  __syncthreads();
+  for (int i = total + tid; i < M; i += kJdKeyThreads) kx[i] = -1;
+  for (int e = tid; e < E; e += kJdKeyThreads) {
+    const int64_t f = ii[e];
+    int64_t at_f = -1;
+    if (f >= 0 && f < frames) at_f = before[f >> 5] + __popc(bits[f >> 5] & ((1u << (f & 31)) - 1));
+    slot[e] = at_f;
+  }
+  if (tid == 0) *count = outside ? -1 : total;
 }
 
 __global__ void __launch_bounds__(kJdThreads)
@@ -361,6 +638,28 @@ jdsa_scales_kernel(float* __restrict__ dscales, int D, const int64_t* __restrict
 
 }  // namespace
 }  // namespace hs2
+
+extern "C" int hs2_jdsa_keys(const int64_t* ii, int64_t num_edges, int64_t num_frames, int64_t num_kx, int64_t* kx,
+                             int64_t* slot, int32_t* count, hs2_stream_t stream) {
+  using namespace hs2;
+  if (num_edges <= 0 || num_edges > 0x7fffffff || num_frames <= 0 || num_frames > kJdKeyFrames || num_kx <= 0 ||
+      num_kx > num_edges) {
+    set_error("jdsa_keys: bad counts (edges %lld, frames %lld of at most %d, source frames %lld)",
+              (long long)num_edges, (long long)num_frames, kJdKeyFrames, (long long)num_kx);
+    return HS2_ERR_INVALID;
+  }
+  if (!ii || !kx || !slot || !count) {
+    set_error("jdsa_keys: a required pointer is null");
+    return HS2_ERR_INVALID;
+  }
+  int rc = bind_device(kx);
+  if (rc) return rc;
+  cudaStream_t s = (cudaStream_t)stream;
+  HS2_PROF("jdsa_keys", s);
+  jdsa_keys_kernel<<<1, kJdKeyThreads, 0, s>>>(ii, (int)num_edges, (int)num_frames, (int)num_kx, kx, slot, count);
+  HS2_LAUNCH_CHECK("jdsa_keys_kernel");
+  return HS2_OK;
+}
 
 extern "C" int hs2_jdsa(const float* poses, int64_t num_poses, const float* disps, int64_t num_disps, int ht, int wd,
                         const float* intrinsics, const float* targets, const float* weights, const float* eta,
@@ -391,10 +690,16 @@ extern "C" int hs2_jdsa(const float* poses, int64_t num_poses, const float* disp
   if (rc) return rc;
   cudaStream_t s = (cudaStream_t)stream;
   HS2_CUDA(cudaMemsetAsync(info, 0, sizeof(int32_t), s));
-  if ((rc = hs2_proj_trans(poses, num_poses, disps, num_disps, ht, wd, intrinsics, targets, weights, ii, jj, slot,
-                           num_edges, num_kx, C, w, info, stream)))
-    return rc;
   JdArgs A;
+  A.poses = poses;
+  A.num_poses = num_poses;
+  A.intr = intrinsics;
+  A.targets = targets;
+  A.weights = weights;
+  A.ii = ii;
+  A.jj = jj;
+  A.slot = slot;
+  A.num_edges = num_edges;
   A.disps = disps;
   A.num_disps = num_disps;
   A.ht = ht;
@@ -418,9 +723,11 @@ extern "C" int hs2_jdsa(const float* poses, int64_t num_poses, const float* disp
   A.dzcov = dzcov;
   A.info = info;
   const size_t smem = sizeof(float) * (size_t)(ht + wd);
-  HS2_PROF("jdsa_solve", s);
-  jdsa_solve_kernel<<<(unsigned)(num_kx + num_disps), kJdThreads, smem, s>>>(A);
-  HS2_LAUNCH_CHECK("jdsa_solve_kernel");
+  // every frame that is not a source frame is one of num_disps - M
+  const unsigned copies = (unsigned)std::min<int64_t>(std::max<int64_t>(num_disps - num_kx, 0), kJdCopyClusters);
+  HS2_PROF("jdsa_step", s);
+  jdsa_step_kernel<<<((unsigned)num_kx + copies) * kJdCluster, kJdThreads, smem, s>>>(A);
+  HS2_LAUNCH_CHECK("jdsa_step_kernel");
   const int D = hs * ws;
   HS2_PROF("jdsa_scales", s);
   jdsa_scales_kernel<<<(unsigned)std::min<int64_t>(64, (num_kx * D + kJdThreads - 1) / kJdThreads), kJdThreads, 0,

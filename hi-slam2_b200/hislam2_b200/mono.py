@@ -16,6 +16,7 @@ from . import _lib
 from .backends import _contig, _cuda, _dtype, _ptr, _stream
 
 _GRIDS = {}
+_KEY_FRAMES = 65536    # hs2_jdsa_keys' limit
 
 
 def grid_axes(ht, wd, hs, ws, device):
@@ -29,6 +30,11 @@ def grid_axes(ht, wd, hs, ws, device):
         gx = torch.linspace(0, ws - 1 - 1e-6, wd)
         _GRIDS[key] = (gy.to(device), gx.to(device))
     return _GRIDS[key]
+
+
+def _check_eta(eta, M, H, W):
+    if eta.numel() != M * H * W:
+        raise RuntimeError("JDSA: eta needs M*H*W values (M = %d distinct source frames)" % M)
 
 
 def JDSA(target, weight, eta, poses, disps, intrinsics, disps_prior, dscales, ii, jj, alpha, with_dzcov=True):
@@ -72,26 +78,36 @@ def JDSA(target, weight, eta, poses, disps, intrinsics, disps_prior, dscales, ii
         raise RuntimeError("JDSA: target/weight must be [E,2,H,W] and jj as long as ii")
     if disps_prior.shape[1:] != (H, W):
         raise RuntimeError("JDSA: disps_prior must have the disparities' H, W")
-    kx, slot = torch.unique(ii, sorted=True, return_inverse=True)
-    M = kx.numel()
-    if eta.numel() != M * H * W:
-        raise RuntimeError("JDSA: eta needs M*H*W values (M = %d distinct source frames)" % M)
+    M, rest = divmod(eta.numel(), H * W) if H * W else (0, 1)
+    on_device = rest == 0 and 1 <= M <= E and P <= _KEY_FRAMES
+    lib = _lib.load()
+    info = torch.empty(2, dtype=torch.int32, device=dev)
+    if on_device:
+        # eta says how many source frames there are, so their keys need no answer from the device
+        # (torch.unique sorts, and waits for the count: 183 us a call with it, 118 without)
+        keys = torch.empty(M + E, dtype=torch.int64, device=dev)
+        kx, slot = keys[:M], keys[M:]
+        _lib.check(lib.hs2_jdsa_keys(_ptr(ii), E, P, M, _ptr(kx), _ptr(slot), _ptr(info[1:]), _stream(dev)),
+                   "jdsa_keys")
+    else:
+        kx, slot = torch.unique(ii, sorted=True, return_inverse=True)
+        slot = slot.contiguous()
+        M = kx.numel()
+        _check_eta(eta, M, H, W)
     hs, ws = dscales.shape[1:]
     D = hs * ws
     gy, gx = grid_axes(H, W, hs, ws, dev)
-    C = torch.empty((M, H * W), dtype=torch.float32, device=dev)
-    w = torch.empty_like(C)
+    C, w = torch.empty((2, M, H * W), dtype=torch.float32, device=dev)
     dso = torch.empty((M, D), dtype=torch.float32, device=dev)
     out = torch.empty_like(d3)
     dzcov = torch.empty((M, H * W), dtype=torch.float32, device=dev) if with_dzcov else None
-    info = torch.empty(1, dtype=torch.int32, device=dev)
-    slot = slot.contiguous()
-    _lib.check(_lib.load().hs2_jdsa(_ptr(pdata), pdata.shape[0], _ptr(d3), P, H, W, _ptr(intr), _ptr(target),
-                                    _ptr(weight), _ptr(eta), _ptr(disps_prior), disps_prior.shape[0],
-                                    _ptr(dscales), dscales.shape[0], hs, ws, _ptr(gy), _ptr(gx), _ptr(ii),
-                                    _ptr(jj), _ptr(slot), E, _ptr(kx), M, float(alpha), _ptr(C), _ptr(w),
-                                    _ptr(dso), _ptr(out), _ptr(dzcov), _ptr(info), _stream(dev)), "jdsa")
-    bits = int(info.item())
+    _lib.check(lib.hs2_jdsa(_ptr(pdata), pdata.shape[0], _ptr(d3), P, H, W, _ptr(intr), _ptr(target), _ptr(weight),
+                            _ptr(eta), _ptr(disps_prior), disps_prior.shape[0], _ptr(dscales), dscales.shape[0], hs,
+                            ws, _ptr(gy), _ptr(gx), _ptr(ii), _ptr(jj), _ptr(slot), E, _ptr(kx), M, float(alpha),
+                            _ptr(C), _ptr(w), _ptr(dso), _ptr(out), _ptr(dzcov), _ptr(info), _stream(dev)), "jdsa")
+    bits, count = info.tolist()
+    if on_device and count != M:
+        _check_eta(eta, torch.unique(ii).numel(), H, W)
     if bits & _lib.HS2_DEV_BAD_INDEX:
         raise RuntimeError("JDSA: an edge or source frame lies outside the pose / disparity / prior / scale "
                            "buffers")

@@ -432,6 +432,17 @@ int hs2_proj_trans(const float* poses, int64_t num_poses, const float* disps, in
 int hs2_bi_inter(const float* scales, int64_t num, int hs, int ws, const float* grids, int ht, int wd,
                  float* outputs, float* jacobians, int32_t* info, hs2_stream_t stream);
 
+/* jdsa_keys: kx and slot of hs2_jdsa from the edges' source frames ii [num_edges] in [0, num_frames),
+ * for a caller that knows their number num_kx (the rows of eta) and would otherwise wait for
+ * the device to learn it.  kx [num_kx]: the sorted distinct frames, filled up with -1 when there
+ * are fewer; slot [num_edges]: the position of ii[e] among the distinct frames, -1 for a frame out
+ * of range.  count: int32[1] = the number of distinct frames, or -1 when a frame was out of range;
+ * unless it equals num_kx, hs2_jdsa on these keys sets HS2_DEV_BAD_INDEX.
+ * Limits: 1 <= num_kx <= num_edges, 1 <= num_frames <= 65536.
+ */
+int hs2_jdsa_keys(const int64_t* ii, int64_t num_edges, int64_t num_frames, int64_t num_kx, int64_t* kx,
+                  int64_t* slot, int32_t* count, hs2_stream_t stream);
+
 /* jdsa  (reference: hislam2/geom/ba.py:170-219 JDSA, :159-167 get_prior_depth_aligned,
  *        hislam2/geom/chol.py:80-107 schur_solve_mono_prior; the caller is
  *        hislam2/depth_video.py:234-240)
