@@ -20,9 +20,11 @@
 //
 // Bound by shared-memory wavefronts and FMA issue together: a union position costs 5
 // wavefronts and 16 FMAs (4 cycles of issue) per group.  Measured (84 edges, 48x64, radius
-// 4, four levels, B200): 2.61 ms for the tiles plus 0.58 / 0.30 ms to pack / unpack,
+// 4, four levels, B200): 2.50 ms for the tiles plus 0.16 / 0.12 ms to pack (and pool) / unpack,
 // against 27.3 ms for the pixel-by-pixel kernel (altcorr_bwd_kernel, kept for other
-// channel counts and radius > 6).
+// channel counts and radius > 6).  Packing and unpacking move 530 and 400 MB there (81 and
+// 61 us at the copy rate); with index arithmetic and one load in flight per element they took
+// 192 and 343 us, by warp-owned rows with eight to sixteen loads in flight 102 and 124.
 #include "common.cuh"
 #include "profile.cuh"
 #include "corr_backward.cuh"
@@ -33,7 +35,8 @@ namespace {
 
 constexpr int kCbC = 128;
 constexpr int kCbThreads = 512;      // 16 warps = 16 groups of 2x2 pixels
-constexpr int kCbPackPix = 64;
+constexpr int kCbPackPix = 64;       // pixels of a transposed block
+constexpr int kCbPackCh = 256 / kCbPackPix;   // channels that its 256 threads hold at once
 
 struct CbArgs {
   const float* f1;                   // [B*N1][H*W][128]
@@ -338,22 +341,35 @@ corr_bwd_pack_kernel(const T* __restrict__ src, float* __restrict__ dst, float* 
   if (flags && !flags[n]) return;
   const int p0 = blockIdx.x * kCbPackPix, np = min(kCbPackPix, HW - p0);
   const int64_t frame = (int64_t)blockIdx.z * N + n;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const T* s = src + frame * kCbC * HW + p0;
+  const int q = threadIdx.x & (kCbPackPix - 1), cq = threadIdx.x / kCbPackPix;
   bool bad = false;
-  for (int idx = threadIdx.x; idx < kCbC * kCbPackPix; idx += 256) {
-    const int c = idx / kCbPackPix, q = idx % kCbPackPix;
-    if (q < np) {
-      const float v = to_f(s[(int64_t)c * HW + q]);
-      bad |= !isfinite(v);
-      tile[q][c] = v;
+  if (q < np) {
+#pragma unroll 2
+    for (int c0 = cq; c0 < kCbC; c0 += 8 * kCbPackCh) {       // eight loads in flight, twice
+      T v[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[i] = s[(int64_t)(c0 + i * kCbPackCh) * HW + q];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const float f = to_f(v[i]);
+        bad |= !isfinite(f);
+        tile[q][c0 + i * kCbPackCh] = f;
+      }
     }
   }
   if (bad) atomicOr(nonfinite, 1);
   __syncthreads();
-  const int64_t at = (frame * HW + p0) * kCbC;
-  for (int idx = threadIdx.x; idx < np * kCbC; idx += 256) {
-    dst[at + idx] = tile[idx / kCbC][idx % kCbC];
-    if (acc) acc[at + idx] = 0.f;
+  float* d = dst + (frame * HW + p0) * kCbC + lane;
+#pragma unroll 4
+  for (int p = warp; p < np; p += 8) {                        // a pixel's row by one warp
+#pragma unroll
+    for (int k = 0; k < kCbC; k += 32) d[p * kCbC + k] = tile[p][lane + k];
+  }
+  if (acc) {
+    float4* a = reinterpret_cast<float4*>(acc + (frame * HW + p0) * kCbC);
+    for (int i = threadIdx.x; i < np * (kCbC / 4); i += 256) a[i] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
 }
 
@@ -391,26 +407,40 @@ corr_bwd_unpack_kernel(const __grid_constant__ CbUnpack U, T* __restrict__ dst,
   const int p0 = blockIdx.x * kCbPackPix, np = min(kCbPackPix, HW - p0);
   const int64_t frame = (int64_t)blockIdx.z * N + n;
   const bool live = !flags || flags[n];
-  for (int idx = threadIdx.x; idx < np * kCbC; idx += 256) {
-    const int q = idx / kCbC, c = idx % kCbC;
-    float v = 0.f;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll 2
+  for (int q = warp; q < np; q += 8) {                        // a pixel's row by one warp, all levels' loads together
+    float v[4] = {0.f, 0.f, 0.f, 0.f};
     if (live) {
       const int y = (p0 + q) / W, x = (p0 + q) - y * W;
-      for (int l = U.levels - 1; l > 0; --l) {
-        const int yl = y >> l, xl = x >> l;
-        if (yl < U.H[l] && xl < U.W[l])
-          v += U.acc[l][((frame * U.H[l] + yl) * U.W[l] + xl) * kCbC + c];
-        v *= 0.25f;
+      float a[4][4];
+#pragma unroll
+      for (int l = 0; l < 4; ++l) {
+        if (l < U.levels) {
+          const int yl = y >> l, xl = x >> l;
+          const bool in = yl < U.H[l] && xl < U.W[l];
+          const float* row = U.acc[l] + ((frame * U.H[l] + yl) * U.W[l] + xl) * kCbC + lane;
+#pragma unroll
+          for (int k = 0; k < 4; ++k) a[l][k] = in ? row[32 * k] : 0.f;
+        }
       }
-      v += U.acc[0][(frame * HW + p0 + q) * kCbC + c];
+#pragma unroll
+      for (int l = 3; l >= 0; --l) {
+        if (l < U.levels) {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) v[k] = (v[k] + a[l][k]) * (l > 0 ? 0.25f : 1.f);
+        }
+      }
     }
-    tile[q][c] = v;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) tile[q][lane + 32 * k] = v[k];
   }
   __syncthreads();
   T* d = dst + frame * kCbC * HW + p0;
-  for (int idx = threadIdx.x; idx < kCbC * kCbPackPix; idx += 256) {
-    const int c = idx / kCbPackPix, q = idx % kCbPackPix;
-    if (q < np) d[(int64_t)c * HW + q] = from_f<T>(tile[q][c]);
+  const int q = threadIdx.x & (kCbPackPix - 1), cq = threadIdx.x / kCbPackPix;
+  if (q < np) {
+#pragma unroll 8
+    for (int c = cq; c < kCbC; c += kCbPackCh) d[(int64_t)c * HW + q] = from_f<T>(tile[q][c]);
   }
 }
 
