@@ -262,7 +262,9 @@ struct CvAppend {
 }  // namespace
 
 // ----------------------------------------------------------------- pack ---
-// fmaps [K, 128, HW] (T) -> rows [K, HW, 128] of the operand type; 64 pixels per CTA.
+// fmaps [K, 128, HW] (T) -> rows [K, HW, 128] of the operand type; 64 pixels per CTA.  A thread's 32
+// loads go out eight at a time: one by one, behind a bounds test each, they took 64 us for the
+// 2 x 48 frames of 43x77 in float16 (81 MB each way, 25 us at the copy rate), now 55.
 template <typename T, int P>
 __global__ void __launch_bounds__(256) corr_pack_kernel(const T* __restrict__ f, int HW, void* __restrict__ rows,
                                                         float* __restrict__ scale) {
@@ -271,9 +273,16 @@ __global__ void __launch_bounds__(256) corr_pack_kernel(const T* __restrict__ f,
   const int k = blockIdx.y;
   const int p0 = blockIdx.x * 64;
   const T* src = f + (int64_t)k * kCvC * HW;
-  for (int i = threadIdx.x; i < kCvC * 64; i += 256) {
-    const int c = i >> 6, p = i & 63;
-    tile[c][p] = (p0 + p < HW) ? to_f<T>(src[(int64_t)c * HW + p0 + p]) * 0.25f : 0.f;
+  {
+    const int p = threadIdx.x & 63, at = min(p0 + p, HW - 1);   // pixels past the frame are not stored
+#pragma unroll
+    for (int c0 = threadIdx.x >> 6; c0 < kCvC; c0 += 32) {
+      T v[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[i] = src[(int64_t)(c0 + 4 * i) * HW + at];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) tile[c0 + 4 * i][p] = to_f<T>(v[i]) * 0.25f;
+    }
   }
   __syncthreads();
   if (P == kE4M3) {
@@ -301,9 +310,10 @@ __global__ void __launch_bounds__(256) corr_pack_kernel(const T* __restrict__ f,
   } else {
     using OpT = typename std::conditional<P == kBF16, __nv_bfloat16, __half>::type;
     OpT* out = static_cast<OpT*>(rows) + ((int64_t)k * HW + p0) * kCvC;
-    for (int i = threadIdx.x; i < 64 * kCvC / 2; i += 256) {
+    const int end = min(64, HW - p0) * (kCvC / 2);
+#pragma unroll 4
+    for (int i = threadIdx.x; i < end; i += 256) {
       const int p = i / (kCvC / 2), c = (i - p * (kCvC / 2)) * 2;
-      if (p0 + p >= HW) continue;
       const uint32_t lo = bits16<OpT>(from_f<OpT>(tile[c][p])), hi = bits16<OpT>(from_f<OpT>(tile[c + 1][p]));
       *reinterpret_cast<uint32_t*>(out + (int64_t)p * kCvC + c) = lo | (hi << 16);
     }
