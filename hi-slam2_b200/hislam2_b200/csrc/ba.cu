@@ -7,7 +7,7 @@
 //               ii (stable), per-frame row lists of E (reference :1841-1849,
 //               :1712-1740, :1413-1439, all host code in the reference)
 //   per iteration
-//   edge_setup  Gij = Gj Gi^-1 and the 6x6 map L with Ji = L Jj for every edge
+//   edge_setup  Gij = Gj Gi^-1 and the 6x6 map L with Ji = L Jj for every edge; the sums zeroed
 //   linearize   per (depth frame, pixel chunk): residuals and Jacobians of all
 //               edges leaving that frame; writes the E rows, Q = 1/(C+eta) and w,
 //               accumulates each edge's Hjj / vj (reference :364-606, :1901-1906)
@@ -20,7 +20,7 @@
 //               (reference SparseBlock::solve :1660-1680)
 //   backsub     dz = Q (w - sum_rows E.dx), rows with pose index <= 0 skipped as in
 //               the reference (EvT6x1_kernel :1562-1582, :1920), disps += dz
-//   pose_retr   poses[t0:t1] <- exp(dx) * poses (FP64 math, reference :1363-1396)
+//   pose_retr   poses[t0:t1] <- exp(dx) * poses (FP64 math, reference :1363-1396), in backsub's launch
 //
 // Only the (tiny) key generation is serial; everything else is sized by the
 // static problem dimensions, so a whole call is graph-capturable.
@@ -271,10 +271,18 @@ __device__ __forceinline__ void ba_edge_setup_body(int gid, const float* __restr
   }
 }
 
+// The edges' tables by the first blocks, and the sums of the step zeroed by all of them: hedge
+// [27 E], A [n n], b [n].  One launch in the place of a kernel and three memsets, which were 3 us
+// each however small.  With the poses moved by the back-substitution's launch: a call of 8 keyframes and 2
+// iterations 235 -> 216 us, of 25 and 4 612 -> 584, of 300 and 8 9.05 -> 8.92 ms.
 __global__ void ba_edge_setup_kernel(const float* __restrict__ poses, const int64_t* __restrict__ ii,
-                                     const int64_t* __restrict__ jj, int E, float* __restrict__ etab,
-                                     double* __restrict__ etab64, const int32_t* __restrict__ info) {
-  ba_edge_setup_body(blockIdx.x * blockDim.x + threadIdx.x, poses, ii, jj, E, etab, etab64, info);
+                                     const int64_t* __restrict__ jj, int E, int n, BaPtrs w,
+                                     const int32_t* __restrict__ info) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
+  for (int64_t i = t; i < 27 * (int64_t)E; i += step) w.hedge[i] = 0.0;
+  for (int64_t i = t; i < (int64_t)n * n / 2; i += step) reinterpret_cast<double2*>(w.A)[i] = make_double2(0.0, 0.0);
+  for (int i = t; i < n; i += step) w.b[i] = 0.0;
+  ba_edge_setup_body(t, poses, ii, jj, E, w.etab, w.etab64, info);
 }
 
 // ------------------------------------------------------------ linearize ---
@@ -2456,17 +2464,6 @@ __device__ __forceinline__ void ba_backsub_body(int s, int chunk, float* __restr
   }
 }
 
-// 256 threads x 2 pixels over the linearisation's 512-pixel chunks
-constexpr int kBsThreads = 2 * kLinThreads;
-constexpr int kBsPPT = kLinPPT / 2;
-static_assert(kBsThreads * kBsPPT == kLinChunk, "back-substitution covers the linearisation's chunks");
-
-__global__ void __launch_bounds__(kBsThreads)
-ba_backsub_kernel(float* __restrict__ disps, int HW, int P, BaPtrs w, const float* __restrict__ dx,
-                  float* __restrict__ dz, int64_t dz_rows, const int32_t* __restrict__ info) {
-  ba_backsub_body<kBsThreads, kBsPPT>(blockIdx.x, blockIdx.y, disps, HW, P, w, dx, dz, dz_rows, info);
-}
-
 // ------------------------------------------------------------ pose retr ---
 __device__ __forceinline__ void ba_pose_retr_body(int k, float* __restrict__ poses, int t0, int P, const BaPtrs w,
                                                   const int32_t* __restrict__ info) {
@@ -2480,6 +2477,24 @@ __device__ __forceinline__ void ba_pose_retr_body(int k, float* __restrict__ pos
   retract_left(xi, t, q);
   for (int c = 0; c < 3; ++c) p[c] = (float)t[c];
   for (int c = 0; c < 4; ++c) p[3 + c] = (float)q[c];
+}
+
+// 256 threads x 2 pixels over the linearisation's 512-pixel chunks
+constexpr int kBsThreads = 2 * kLinThreads;
+constexpr int kBsPPT = kLinPPT / 2;
+static_assert(kBsThreads * kBsPPT == kLinChunk, "back-substitution covers the linearisation's chunks");
+
+__global__ void __launch_bounds__(kBsThreads)
+ba_backsub_kernel(float* __restrict__ poses, int t0, float* __restrict__ disps, int HW, int P, BaPtrs w,
+                  const float* __restrict__ dx, float* __restrict__ dz, int64_t dz_rows,
+                  const int32_t* __restrict__ info) {
+  if (blockIdx.x == 0) {
+    // the poses: a launch of their own took 3 us more per iteration
+    if (blockIdx.y == 0)
+      for (int k = threadIdx.x; k < P; k += kBsThreads) ba_pose_retr_body(k, poses, t0, P, w, info);
+    return;
+  }
+  ba_backsub_body<kBsThreads, kBsPPT>(blockIdx.x - 1, blockIdx.y, disps, HW, P, w, dx, dz, dz_rows, info);
 }
 
 __global__ void ba_pose_retr_kernel(float* __restrict__ poses, int t0, int P, const BaPtrs w,
@@ -2641,16 +2656,13 @@ static int build_system(const BaProblem& p, const BaLaunch& l, const float* pose
   const int P = p.P;
   const int n = 6 * P;
   const int64_t S = std::min<int64_t>(p.K, (int64_t)P + E);
-  if (E > 0) {
+  if (E > 0 || n > 0) {
+    // blocks for the edges' threads, or for 32 bytes a thread of A (n = 6 P: whole pairs), up to 16 an SM
+    const int64_t zero = ((int64_t)n * n / 4 + 127) / 128 + 1;
+    const int64_t blocks = std::max<int64_t>((6 * (int64_t)E + 127) / 128, std::min<int64_t>(zero, 16 * kNumSMs));
     HS2_PROF("ba_edge_setup", s);
-    ba_edge_setup_kernel<<<(6 * E + 127) / 128, 128, 0, s>>>(poses, ii, jj, E, w.etab, w.etab64, info);
+    ba_edge_setup_kernel<<<(unsigned)blocks, 128, 0, s>>>(poses, ii, jj, E, n, w, info);
     HS2_LAUNCH_CHECK("ba_edge_setup_kernel");
-    HS2_CUDA(cudaMemsetAsync(w.hedge, 0, sizeof(double) * 27 * (size_t)E, s));
-  }
-  if (n > 0) {
-    HS2_PROF("ba_zero_system", s);
-    HS2_CUDA(cudaMemsetAsync(w.A, 0, sizeof(double) * (size_t)n * n, s));
-    HS2_CUDA(cudaMemsetAsync(w.b, 0, sizeof(double) * (size_t)n, s));
   }
   const int path = g_schur_path.load();
   const bool fused = !p.motion_only && path == 2;
@@ -2794,6 +2806,7 @@ extern "C" int hs2_ba(float* poses, int64_t num_poses, float* disps, int64_t num
     if ((rc = build_system(p, l, poses, disps, intrinsics, targets, weights, eta, eta_rows, ii, jj, w, info, s)))
       return rc;
     if ((rc = run_cholesky(n, lm, ep, w, cb, dx, info, s))) return rc;
+    bool moved = false;                       // the back-substitution's launch moves the poses too
     if (!p.motion_only && S > 0) {
       dim3 grid((unsigned)S, nchunk);
       HS2_PROF("ba_backsub", s);
@@ -2802,11 +2815,13 @@ extern "C" int hs2_ba(float* poses, int64_t num_poses, float* disps, int64_t num
                                                              dx, dz, dz_rows, info);
         HS2_LAUNCH_CHECK("ba_backsub_frame_kernel");
       } else {
-        ba_backsub_kernel<<<grid, kBsThreads, 0, s>>>(disps, p.HW, P, w, dx, dz, dz_rows, info);
+        ba_backsub_kernel<<<dim3((unsigned)S + 1, nchunk), kBsThreads, 0, s>>>(poses, t0, disps, p.HW, P, w, dx, dz,
+                                                                               dz_rows, info);
         HS2_LAUNCH_CHECK("ba_backsub_kernel");
+        moved = true;
       }
     }
-    if (P > 0) {
+    if (P > 0 && !moved) {
       HS2_PROF("ba_pose_retr", s);
       ba_pose_retr_kernel<<<(P + 127) / 128, 128, 0, s>>>(poses, t0, P, w, info);
       HS2_LAUNCH_CHECK("ba_pose_retr_kernel");
