@@ -29,7 +29,8 @@
 // appends its new elements, 16 accumulator columns at a time, to its row of a per-warp
 // staging buffer at the run's 16-byte phase in global memory; the warp then writes all
 // full 16-byte chunks (neighbouring lanes, neighbouring chunks) and each lane keeps its
-// partial chunk in registers for the next append.  Level 1 reads the two image rows'
+// partial chunk in registers for the next append.  A level may start at any element: the chunks
+// are those of its address, not of its element indices.  Level 1 reads the two image rows'
 // accumulators again from TMEM and pools the rounded values; the rows above of levels 1
 // and 2 wait in shared memory.  No barrier spans the epilogue warps, single elements are
 // written only at the ends of a unit's runs, and everything runs in short loops: the
@@ -181,8 +182,8 @@ struct CvShare {
 };
 
 // Writes the warp's full chunks after an append of n elements.  Row r of the warp holds the
-// run of source pixel r; its new elements start at out[g0 + r * plane], `since` elements after
-// the unit's part of the run began.  rows: live rows of the warp; done: the unit's last append.
+// run of source pixel r; its new elements start at out[g0 + r * plane] (out on a 16-byte boundary),
+// `since` elements after the unit's part of the run began.  rows: live rows of the warp; done: the unit's last append.
 // Returns the lane's partial chunk.
 // One copy for all levels: inlined everywhere, the epilogue's loops outgrow the instruction cache.
 __device__ __noinline__ uint4 run_flush(const CvShare sh, uint16_t* __restrict__ out, int64_t g0, int plane, int n,
@@ -321,8 +322,11 @@ __global__ void __launch_bounds__(256) corr_pack_kernel(const T* __restrict__ f,
 }
 
 // --------------------------------------------------------------- volume ---
+// A level's output: the 16-byte boundary at or before its first element, and how many elements before
+// it that boundary lies.  Run positions count from the boundary, so a multiple of 8 is aligned.
 struct CvOut {
   uint16_t* lvl[4];
+  int skew[4];
 };
 
 template <int P, typename T>
@@ -523,7 +527,7 @@ corr_volume_kernel(const __grid_constant__ CUtensorMap amap, const __grid_consta
         uint4 tail = make_uint4(0, 0, 0, 0);
         for (int i = i0; i < i1; ++i) {
           if (!(ok = wait_row(reg, par))) break;
-          const int64_t g0 = px0 * g.HW + (int64_t)i * g.W;
+          const int64_t g0 = px0 * g.HW + (int64_t)i * g.W + out.skew[0];
           CvAppend ap(row, tail, ((int)(g0 & 7) + lane * g.HW) & 7, g.W);
           uint32_t v[2][16], w[8];
           load(reg, 0, v[0]);
@@ -575,7 +579,7 @@ corr_volume_kernel(const __grid_constant__ CUtensorMap amap, const __grid_consta
             next_row();
           }
           const bool live = two && g.levels > 1 && g.W1 > 0;
-          int64_t g0 = px0 * HW1 + (int64_t)j * g.W1;
+          int64_t g0 = px0 * HW1 + (int64_t)j * g.W1 + out.skew[1];
           if (live) {
             CvAppend ap(row, tail1, ((int)(g0 & 7) + lane * HW1) & 7, g.W1);
             for (int pc = 0; pc < np; ++pc) {
@@ -607,7 +611,7 @@ corr_volume_kernel(const __grid_constant__ CUtensorMap amap, const __grid_consta
           if (!live) continue;
           tail1 = run_flush(sh1, out.lvl[1], g0, HW1, g.W1, (j - (i0 >> 1)) * g.W1, j == (i1 >> 1) - 1, rows, chunks, stg);
           if (!(j & 1) || g.levels < 3 || g.W2 == 0) continue;
-          g0 = px0 * HW2 + (int64_t)j2 * g.W2;
+          g0 = px0 * HW2 + (int64_t)j2 * g.W2 + out.skew[2];
           {
             CvAppend ap(row, tail2, ((int)(g0 & 7) + lane * HW2) & 7, g.W2);
             for (int pc = 0; pc < np; ++pc) {
@@ -626,7 +630,7 @@ corr_volume_kernel(const __grid_constant__ CUtensorMap amap, const __grid_consta
           }
           tail2 = run_flush(sh2, out.lvl[2], g0, HW2, g.W2, (j2 - (i0 >> 2)) * g.W2, j2 == (i1 >> 2) - 1, rows, chunks, stg);
           if (!(j2 & 1) || g.levels < 4 || g.W3 == 0) continue;
-          g0 = px0 * HW3 + (int64_t)j3 * g.W3;
+          g0 = px0 * HW3 + (int64_t)j3 * g.W3 + out.skew[3];
           {
             CvAppend ap(row, tail3, ((int)(g0 & 7) + lane * HW3) & 7, g.W3);
             for (int pc = 0; pc < np; ++pc) {
@@ -799,7 +803,11 @@ extern "C" int hs2_corr_volume(const void* fmap1, int64_t k1, const void* fmap2,
     sc2 = sc1 + (size_t)k1 * HW;
   }
   CvOut out;
-  for (int l = 0; l < 4; ++l) out.lvl[l] = l < levels ? static_cast<uint16_t*>(pyramid[l]) : nullptr;
+  for (int l = 0; l < 4; ++l) {
+    const uintptr_t at = l < levels ? reinterpret_cast<uintptr_t>(pyramid[l]) : 0;
+    out.lvl[l] = reinterpret_cast<uint16_t*>(at & ~(uintptr_t)15);
+    out.skew[l] = (int)(at & 15) / 2;
+  }
   const CvGeom g = cv_geom(ht, wd, num_pairs, levels, precision == HS2_CV_E4M3 ? 1 : 2);
   if (dtype == HS2_F16) {
     if (precision == HS2_CV_E4M3) {

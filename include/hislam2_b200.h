@@ -166,6 +166,8 @@ int hs2_ba_adjoint(const float* poses, int64_t num_poses, const float* disps, in
  *   level 0 = sum_c (fmap1[ii,c]/4)(fmap2[jj,c]/4) accumulated in F32 on the tensor
  *   cores, level l = 2x2 average of level l-1 (floor sizes), each level rounded to
  *   `dtype` and pooled from the rounded level above (avg_pool2d's arithmetic).
+ *   A level needs the alignment of its elements (2 bytes), so the levels may lie one after
+ *   the other in one buffer.
  *   precision HS2_CV_NATIVE contracts the 16-bit values as given; HS2_CV_E4M3
  *   quantises each pixel's feature vector to FP8 e4m3 with its own scale
  *   (max |f/4| / 448) and rescales the F32 sums.  channels must be 128, wd <= 96.
