@@ -52,7 +52,9 @@ class PyramidSampler(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, coords, radius, *volumes):
-        ctx.save_for_backward(coords, *volumes)
+        # a copy: the caller may move its coordinates on before the backward
+        kept = coords.clone() if any(ctx.needs_input_grad[2:]) else None
+        ctx.save_for_backward(kept, *volumes)
         ctx.radius = radius
         return backends.corr_pyramid_forward(volumes, coords, radius)
 
@@ -61,7 +63,7 @@ class PyramidSampler(torch.autograd.Function):
         coords, *volumes = ctx.saved_tensors
         rd = 2 * ctx.radius + 1
         n, _, ht, wd = grad_output.shape
-        planar = coords.permute(0, 3, 1, 2).contiguous()
+        planar = None if coords is None else coords.permute(0, 3, 1, 2).contiguous()
         grads = []
         for i, volume in enumerate(volumes):
             if not ctx.needs_input_grad[2 + i]:
