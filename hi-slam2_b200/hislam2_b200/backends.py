@@ -573,13 +573,14 @@ def corr_pyramid_fits(volumes, coords, radius):
 def corr_pyramid_forward(volumes, coords, radius):
     """``corr_index_forward`` of every pyramid level at ``coords / 2^level``, concatenated.
 
-    ``volumes[l]`` [N,H,W,H>>l,W>>l], ``coords`` [N,H,W,2] contiguous; returns [N, L*(2r+1)^2, H, W].
-    For inputs that pass :func:`corr_pyramid_fits`.
+    ``volumes[l]`` [N,H,W,H>>l,W>>l], ``coords`` [...,H,W,2] contiguous, of N frames in all; returns
+    [..., L*(2r+1)^2, H, W] (not a view: a caller may go on in place).  For inputs that pass
+    :func:`corr_pyramid_fits` as [N,H,W,2].
     """
     _contig("coords", coords)
-    n, h, w, _ = coords.shape
-    L, r, dev = len(volumes), int(radius), coords.device
-    corr = torch.empty(n, L * (2 * r + 1) ** 2, h, w, dtype=volumes[0].dtype, device=dev)
+    *lead, h, w, _ = coords.shape
+    n, L, r, dev = volumes[0].shape[0], len(volumes), int(radius), coords.device
+    corr = torch.empty(*lead, L * (2 * r + 1) ** 2, h, w, dtype=volumes[0].dtype, device=dev)
     ptrs = (ctypes.c_void_p * 4)(*[v.data_ptr() for v in volumes])
     _lib.check(_lib.load().hs2_corr_pyramid_forward(ptrs, L, _DTYPES[volumes[0].dtype], n, h, w, _ptr(coords), r,
                                                     _ptr(corr), _stream(dev)), "corr_pyramid_forward")

@@ -48,7 +48,7 @@ class CorrSampler(torch.autograd.Function):
 
 class PyramidSampler(torch.autograd.Function):
     """:class:`CorrSampler` of every pyramid level at coords / 2^level in one launch, concatenated;
-    coords [N, H, W, 2]; gradients w.r.t. the volumes."""
+    coords [..., H, W, 2] for volumes of as many pixels; gradients w.r.t. the volumes."""
 
     @staticmethod
     def forward(ctx, coords, radius, *volumes):
@@ -62,8 +62,10 @@ class PyramidSampler(torch.autograd.Function):
     def backward(ctx, grad_output):
         coords, *volumes = ctx.saved_tensors
         rd = 2 * ctx.radius + 1
-        n, _, ht, wd = grad_output.shape
-        planar = None if coords is None else coords.permute(0, 3, 1, 2).contiguous()
+        ht, wd = grad_output.shape[-2:]
+        grad_output = grad_output.flatten(0, -4)
+        n = grad_output.shape[0]
+        planar = None if coords is None else coords.reshape(n, ht, wd, 2).permute(0, 3, 1, 2).contiguous()
         grads = []
         for i, volume in enumerate(volumes):
             if not ctx.needs_input_grad[2 + i]:
@@ -91,7 +93,7 @@ class CorrBlock:
         levels = self.corr_pyramid[:self.num_levels]
         pixels = coords.reshape(batch * num, ht, wd, -1)
         if len(levels) == self.num_levels and backends.corr_pyramid_fits(levels, pixels, self.radius):
-            return PyramidSampler.apply(pixels.contiguous(), self.radius, *levels).view(batch, num, -1, ht, wd)
+            return PyramidSampler.apply(coords.contiguous(), self.radius, *levels)
         out_pyramid = []
         coords = coords.permute(0, 1, 4, 2, 3).contiguous().view(batch * num, 2, ht, wd)
         for i in range(self.num_levels):

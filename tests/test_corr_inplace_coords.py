@@ -24,8 +24,10 @@ def sample(volume, planar, r):
 
 
 def plain_forward(volumes, coords, radius):
-    planar = coords.permute(0, 3, 1, 2)
-    return torch.cat([sample(v, planar / 2 ** i, radius).flatten(1, 2) for i, v in enumerate(volumes)], 1)
+    h, w = coords.shape[-3:-1]
+    planar = coords.reshape(-1, h, w, 2).permute(0, 3, 1, 2)
+    out = torch.cat([sample(v, planar / 2 ** i, radius).flatten(1, 2) for i, v in enumerate(volumes)], 1)
+    return torch.empty(*coords.shape[:-3], *out.shape[1:], dtype=out.dtype).copy_(out.reshape(*coords.shape[:-3], *out.shape[1:]))
 
 
 def plain_backward(volume, planar, grad, radius):
