@@ -40,9 +40,9 @@ def outputs(dev, dtype):
 def check(dev, dtype, differentiate):
     for (_, plain), (leaf, out) in zip(outputs(dev, dtype), outputs(dev, dtype)):
         assert not out._is_view()
-        want = 0.5 * plain.relu()
-        out.relu_()
+        want = (0.5 * plain).relu()
         out *= 0.5
+        out.relu_()
         assert torch.equal(out, want) and tuple(out.shape) == (1, 2, 2 * 49, 8, 9)
         if differentiate:
             assert torch.autograd.grad(out.float().sum(), leaf)[0].abs().max() > 0
