@@ -155,8 +155,9 @@ corr_index_fwd_r_kernel(const __grid_constant__ CiLevels lv, const float* __rest
     const float cx = s * coords[at], cy = s * coords[at + (interleaved ? 1 : HW1)];
     const float fx = floorf(cx), fy = floorf(cy);
     frac[tid] = make_float2(cx - fx, cy - fy);
-    // a window further out than this has no taps; the clamp keeps the sums in range
-    org[tid] = make_int2(min(max((int)fx, -(1 << 20)), 1 << 20) - R, min(max((int)fy, -(1 << 20)), 1 << 20) - R);
+    // a window that ends before 0 or starts at w2 has no taps; the clamp, which follows the level's own
+    // size, keeps the sums in range: |o.y| w2 + 64 planes stay below 2^31
+    org[tid] = make_int2(min(max((int)fx, -2 * D), w2 + 2 * D) - R, min(max((int)fy, -2 * D), h2 + 2 * D) - R);
   }
   __syncthreads();
   const T* vol = static_cast<const T*>(lv.vol[lvl]) + ((int64_t)n * HW1 + pix0) * (int64_t)HW2;
