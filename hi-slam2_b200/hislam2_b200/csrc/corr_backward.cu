@@ -661,6 +661,10 @@ extern "C" int hs2_corr_lookup_backward(const void* fmap1, const void* fmap2, in
     set_error("corr_lookup_backward: workspace of %zu bytes required", need);
     return HS2_ERR_WORKSPACE;
   }
+  if (reinterpret_cast<uintptr_t>(workspace) & 15) {
+    set_error("corr_lookup_backward: the workspace must start on a 16-byte boundary");
+    return HS2_ERR_WORKSPACE;
+  }
   if ((rc = bind_device(fmap1_grad))) return rc;
   cudaStream_t s = (cudaStream_t)stream;
   char* ws = static_cast<char*>(workspace);

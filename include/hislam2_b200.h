@@ -267,7 +267,8 @@ int hs2_altcorr_levels_packed(const void* packed1, const void* const* packed_lev
  *   leaves out the forward's 1/16), 1/16 gives the exact adjoint of the forward.
  *   workspace: hs2_altcorr_backward_workspace_size() bytes (channel-last f32 features and
  *   accumulators of the tiled kernel for c == 128).  With fewer bytes, down to the f32
- *   accumulators alone (none when dtype is f32), the pixel-by-pixel kernel runs instead.
+ *   accumulators alone (none when dtype is f32), or when it does not start on a 16-byte
+ *   boundary, the pixel-by-pixel kernel runs instead.
  */
 int hs2_altcorr_backward_workspace_size(int dtype, int b, int n1, int n2, int c, int h, int w, int h2,
                                         int w2, size_t* bytes);
@@ -284,6 +285,7 @@ int hs2_altcorr_backward(const void* fmap1, const void* fmap2, int dtype, int b,
  *   fmap2[k]; coords [n,h,w,2] f32; grad [n, levels*(2r+1)^2, h, w] of `dtype`; scale multiplies every
  *   product (1/16 for the lookup's own scaling); 1 to 4 levels, radius <= 6
  *   -> fmap1_grad, fmap2_grad [n,c,h,w] of `dtype`, fully written; accumulated in f32.
+ *   workspace: on a 16-byte boundary, else HS2_ERR_WORKSPACE.
  */
 int hs2_corr_lookup_backward_workspace_size(int dtype, int n, int c, int h, int w, int levels, int radius,
                                             size_t* bytes);
