@@ -656,6 +656,13 @@ static int batch_plan(const hs2_ba_window* in, int nwin, int gsplit, BatchPlanHo
   return HS2_OK;
 }
 
+// The plan's base inside the caller's workspace, which may start anywhere: the units read the E rows by
+// 16-byte vectors.
+constexpr size_t kBatchAlign = 256;
+static char* batch_base(void* workspace) {
+  return reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(workspace) + kBatchAlign - 1) & ~(uintptr_t)(kBatchAlign - 1));
+}
+
 }  // namespace hs2
 
 extern "C" int hs2_ba_batch_workspace_size(const hs2_ba_window* windows, int num_windows, size_t* bytes) {
@@ -667,7 +674,7 @@ extern "C" int hs2_ba_batch_workspace_size(const hs2_ba_window* windows, int num
   BatchPlanHost pl;
   int rc = batch_plan(windows, num_windows, 1, pl);
   if (rc) return rc;
-  *bytes = pl.total;
+  *bytes = pl.total + kBatchAlign - 1;
   return HS2_OK;
 }
 
@@ -677,8 +684,10 @@ extern "C" int hs2_ba_batch_prepare(const hs2_ba_window* windows, int num_window
   BatchPlanHost pl;
   int rc = batch_plan(windows, num_windows, gram_split, pl);
   if (rc) return rc;
-  if (!workspace || workspace_bytes < pl.total) {
-    set_error("ba_batch_prepare: workspace of %zu bytes required", pl.total);
+  char* base = batch_base(workspace);
+  const size_t need = pl.total + (size_t)(base - static_cast<char*>(workspace));
+  if (!workspace || workspace_bytes < need) {
+    set_error("ba_batch_prepare: workspace of %zu bytes required", need);
     return HS2_ERR_WORKSPACE;
   }
   if (!grid) {
@@ -687,7 +696,6 @@ extern "C" int hs2_ba_batch_prepare(const hs2_ba_window* windows, int num_window
   }
   if ((rc = bind_device(workspace))) return rc;
   cudaStream_t s = (cudaStream_t)stream;
-  char* base = static_cast<char*>(workspace);
   int dev = 0, sms = 0, occ = 0;
   HS2_CUDA(cudaGetDevice(&dev));
   HS2_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -730,7 +738,7 @@ extern "C" int hs2_ba_batch_run(void* workspace, int num_windows, int grid, int 
   int rc;
   if ((rc = bind_device(workspace))) return rc;
   cudaStream_t s = (cudaStream_t)stream;
-  char* base = static_cast<char*>(workspace);
+  char* base = batch_base(workspace);
   const int nwin = num_windows;
   size_t o = 0;
   auto take = [&](size_t bytes) { size_t at = o; o = align256(o + bytes); return at; };

@@ -100,6 +100,7 @@ int hs2_corr_index_backward(const float* coords, const void* corr_grad, int dtyp
  *   gram_split: pixel splits per depth frame of the Schur Gram (tuning knob, >= 1);
  *   ctas_per_sm: CTAs per SM of the persistent grid (0 = as many as fit).
  *   Each window's info [4] is as for hs2_ba.
+ *   workspace: hs2_ba_batch_workspace_size() bytes, at any address (the same one for both).
  */
 typedef struct hs2_ba_window {
   float* poses;
