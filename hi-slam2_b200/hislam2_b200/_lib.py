@@ -46,6 +46,8 @@ SIGNATURES = {
                                   _p, _p],
     "hs2_altcorr_backward_workspace_size": [_i32, _i32, _i32, _i32, _i32, _i32, _i32, _i32, _i32,
                                             ctypes.POINTER(_sz)],
+    "hs2_altcorr_backward_call_workspace_size": [_i32, _i32, _i32, _i32, _i32, _i32, _i32, _i32, _i32, _i32, _i32,
+                                                 ctypes.POINTER(_sz)],
     "hs2_altcorr_backward": [_p, _p, _i32, _i32, _i32, _i32, _i32, _i32, _i32, _i32, _i32, _p, _p, _p,
                              _i32, _p, _i32, _f32, _p, _p, _p, _p, _sz, _p],
     "hs2_corr_lookup_backward_workspace_size": [_i32, _i32, _i32, _i32, _i32, _i32, _i32, ctypes.POINTER(_sz)],

@@ -888,12 +888,17 @@ def altcorr_backward(fmap1, fmap2, coords, ii, jj, grad, radius, scale=1.0):
         raise RuntimeError("altcorr_backward: grad must be %s" % ((B, M, 2 * r + 1, 2 * r + 1, H, W),))
     lib = _lib.load()
     nbytes = ctypes.c_size_t(0)
-    _lib.check(lib.hs2_altcorr_backward_workspace_size(dt, B, N1, N2, C, H, W, H2, W2, ctypes.byref(nbytes)),
-               "altcorr_backward_workspace_size")
-    ws = torch.empty(max(1, nbytes.value), dtype=torch.uint8, device=fmap1.device)
+    _lib.check(lib.hs2_altcorr_backward_call_workspace_size(dt, B, N1, N2, C, H, W, H2, W2, M, r, ctypes.byref(nbytes)),
+               "altcorr_backward_call_workspace_size")
     g1 = torch.empty_like(fmap1)
     g2 = torch.empty_like(fmap2)
     info = torch.zeros(1, dtype=torch.int32, device=fmap1.device)
+    try:
+        ws = torch.empty(max(1, nbytes.value), dtype=torch.uint8, device=fmap1.device)
+    except torch.cuda.OutOfMemoryError:
+        # no room for the tiles' FP32 copies of the frames in use: the accumulators alone
+        nbytes.value = 0 if dt == _lib.HS2_F32 else 4 * (fmap1.numel() + fmap2.numel())
+        ws = torch.empty(max(1, nbytes.value), dtype=torch.uint8, device=fmap1.device)
     _lib.check(lib.hs2_altcorr_backward(_ptr(fmap1), _ptr(fmap2), dt, B, N1, N2, C, H, W, H2, W2, _ptr(coords),
                                         _ptr(ii), _ptr(jj), M, _ptr(grad), r, float(scale), _ptr(g1), _ptr(g2),
                                         _ptr(info), _ptr(ws), nbytes.value, _stream(fmap1.device)),

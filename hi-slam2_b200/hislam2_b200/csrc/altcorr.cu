@@ -932,14 +932,20 @@ extern "C" int hs2_altcorr_forward(const void* fmap1, const void* fmap2, int dty
   return HS2_ERR_DTYPE;
 }
 
-extern "C" int hs2_altcorr_backward_workspace_size(int dtype, int b, int n1, int n2, int c, int h, int w,
-                                                   int h2, int w2, size_t* bytes) {
+extern "C" int hs2_altcorr_backward_call_workspace_size(int dtype, int b, int n1, int n2, int c, int h, int w, int h2,
+                                                        int w2, int m, int radius, size_t* bytes) {
   using namespace hs2;
   if (!bytes) return HS2_ERR_INVALID;
   *bytes = ac_bwd_bytes(dtype, b, n1, n2, c, h, w, h2, w2);
-  if (c == 128 && b > 0 && n1 > 0 && n2 > 0 && h > 0 && w > 0 && h2 > 0 && w2 > 0)
-    *bytes = std::max(*bytes, altcorr_bwd_tiled_bytes(b, n1, n2, h, w, h2, w2));
+  if (h > 0 && w > 0 && h2 > 0 && w2 > 0 && altcorr_bwd_tiled_ok(b, n1, n2, c, m, radius))
+    *bytes = std::max(*bytes, altcorr_bwd_tiled_bytes(b, n1, n2, h, w, h2, w2, m));
   return HS2_OK;
+}
+
+extern "C" int hs2_altcorr_backward_workspace_size(int dtype, int b, int n1, int n2, int c, int h, int w,
+                                                   int h2, int w2, size_t* bytes) {
+  // for any number of edges and any radius
+  return hs2_altcorr_backward_call_workspace_size(dtype, b, n1, n2, c, h, w, h2, w2, 0x7fffffff, 0, bytes);
 }
 
 extern "C" int hs2_altcorr_backward(const void* fmap1, const void* fmap2, int dtype, int b, int n1, int n2,
@@ -963,7 +969,7 @@ extern "C" int hs2_altcorr_backward(const void* fmap1, const void* fmap2, int dt
   // levels: 3.5 ms (2.6 tiles, 0.9 packing, since then less than half) against 27.3 ms pixel by pixel.
   if ((dtype == HS2_F32 || dtype == HS2_F16 || dtype == HS2_BF16) && altcorr_bwd_tiled_ok(b, n1, n2, c, m, radius) &&
       workspace && !(reinterpret_cast<uintptr_t>(workspace) & 15) &&
-      workspace_bytes >= altcorr_bwd_tiled_bytes(b, n1, n2, h, w, h2, w2))
+      workspace_bytes >= altcorr_bwd_tiled_bytes(b, n1, n2, h, w, h2, w2, m))
     return altcorr_bwd_tiled(dtype, fmap1, fmap2, b, n1, n2, h, w, h2, w2, coords, ii, jj, m, grad, radius, scale,
                              fmap1_grad, fmap2_grad, info, workspace, s);
   switch (dtype) {

@@ -25,6 +25,8 @@
 // channel counts and radius > 6).  Packing and unpacking move 530 and 400 MB there (81 and
 // 61 us at the copy rate); with index arithmetic and one load in flight per element they took
 // 192 and 343 us, by warp-owned rows with eight to sixteen loads in flight 102 and 124.
+#include <algorithm>
+
 #include "common.cuh"
 #include "profile.cuh"
 #include "corr_backward.cuh"
@@ -39,15 +41,18 @@ constexpr int kCbPackPix = 64;       // pixels of a transposed block
 constexpr int kCbPackCh = 256 / kCbPackPix;   // channels that its 256 threads hold at once
 
 struct CbArgs {
-  const float* f1;                   // [B*N1][H*W][128]
-  const float* f2[4];                // [B*N2][H2*W2][128] per level
+  const float* f1;                   // [B*S1][H*W][128]
+  const float* f2[4];                // [B*S2][H2*W2][128] per level
   float* o1;
   float* o2[4];
   const float* coords;               // [B][M][2][H][W], or [B][M][H][W][2] when interleaved
   const void* grad;                  // [B][M][levels][2r+1 (x)][2r+1 (y)][H][W]
   const int64_t* ii;                 // null: frame m on both sides
   const int64_t* jj;
-  int N1, N2, M, H, W, r, levels, cap, interleaved;
+  const int* slot1;                  // with ii: where a frame's packed features and accumulator are
+  const int* slot2;
+  int N1, N2, S1, S2;                // frames, and packed frames a batch entry
+  int M, H, W, r, levels, cap, interleaved;
   int H2[4], W2[4];
   float scale;
   const int32_t* nonfinite;
@@ -111,13 +116,14 @@ __global__ void __launch_bounds__(kCbThreads, 2) corr_bwd_tile_kernel(const __gr
   const int64_t bm = (int64_t)b * A.M + m;
   const bool separate = *A.nonfinite != 0;
   const int gx = 2 * (warp & 3), gy = 2 * (warp >> 2);             // the warp's group inside the tile
-  const float4* f1 = reinterpret_cast<const float4*>(A.f1) + ((int64_t)b * A.N1 + ix) * HW * 32;
-  float4* o1 = reinterpret_cast<float4*>(A.o1) + ((int64_t)b * A.N1 + ix) * HW * 32;
+  const int64_t fr1 = (int64_t)b * A.S1 + (A.ii ? A.slot1[ix] : m), fr2 = (int64_t)b * A.S2 + (A.ii ? A.slot2[jx] : m);
+  const float4* f1 = reinterpret_cast<const float4*>(A.f1) + fr1 * HW * 32;
+  float4* o1 = reinterpret_cast<float4*>(A.o1) + fr1 * HW * 32;
 
   for (int lvl = 0; lvl < A.levels; ++lvl) {
     const int H2 = A.H2[lvl], W2 = A.W2[lvl];
-    const float4* f2 = reinterpret_cast<const float4*>(A.f2[lvl]) + ((int64_t)b * A.N2 + jx) * (int64_t)H2 * W2 * 32;
-    float* o2 = A.o2[lvl] + ((int64_t)b * A.N2 + jx) * (int64_t)H2 * W2 * kCbC;
+    const float4* f2 = reinterpret_cast<const float4*>(A.f2[lvl]) + fr2 * H2 * W2 * 32;
+    float* o2 = A.o2[lvl] + fr2 * H2 * W2 * kCbC;
     __syncthreads();                                               // the previous level's F1 / Gu readers
     if (tid < 64) {
       const int px = tx0 + (tid & 7), py = ty0 + (tid >> 3);
@@ -323,10 +329,36 @@ __global__ void __launch_bounds__(kCbThreads, 2) corr_bwd_tile_kernel(const __gr
   }
 }
 
-__global__ void corr_bwd_flag_kernel(const int64_t* __restrict__ idx, int m, int n, unsigned char* __restrict__ flags) {
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < m; e += gridDim.x * blockDim.x) {
+// Where the frames that the edges use are packed: slot[f] = their number below f, -1 for a frame that
+// no edge uses; CTA 0 for the edges' ii, CTA 1 for jj.  At most m slots a side.
+__global__ void __launch_bounds__(1024)
+corr_bwd_slots_kernel(const int64_t* __restrict__ ii, const int64_t* __restrict__ jj, int m, int n1, int n2,
+                      int* __restrict__ slot1, int* __restrict__ slot2) {
+  const int64_t* idx = blockIdx.x ? jj : ii;
+  const int n = blockIdx.x ? n2 : n1, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  int* slot = blockIdx.x ? slot2 : slot1;
+  __shared__ int counts[32];
+  for (int f = tid; f < n; f += 1024) slot[f] = 0;
+  __syncthreads();
+  for (int e = tid; e < m; e += 1024) {
     const int64_t f = idx[e];
-    if (f >= 0 && f < n) flags[f] = 1;
+    if (f >= 0 && f < n) slot[f] = 1;
+  }
+  __syncthreads();
+  int base = 0;
+  for (int f0 = 0; f0 < n; f0 += 1024) {
+    const int f = f0 + tid;
+    const bool used = f < n && slot[f];
+    const unsigned mask = __ballot_sync(0xffffffffu, used);
+    if (lane == 0) counts[warp] = __popc(mask);
+    __syncthreads();
+    int at = base;
+    for (int q = 0; q < 32; ++q) {
+      if (q < warp) at += counts[q];
+      base += counts[q];
+    }
+    if (f < n) slot[f] = used ? at + __popc(mask & ((1u << lane) - 1)) : -1;
+    __syncthreads();
   }
 }
 
@@ -335,14 +367,14 @@ __global__ void corr_bwd_flag_kernel(const int64_t* __restrict__ idx, int m, int
 template <typename T>
 __global__ void __launch_bounds__(256)
 corr_bwd_pack_kernel(const T* __restrict__ src, float* __restrict__ dst, float* __restrict__ acc,
-                     const unsigned char* __restrict__ flags, int N, int HW, int32_t* __restrict__ nonfinite) {
+                     const int* __restrict__ slots, int N, int S, int HW, int32_t* __restrict__ nonfinite) {
   __shared__ float tile[kCbPackPix][kCbC + 1];
-  const int n = blockIdx.y;
-  if (flags && !flags[n]) return;
+  const int n = blockIdx.y, slot = slots ? slots[n] : n;
+  if (slot < 0) return;
   const int p0 = blockIdx.x * kCbPackPix, np = min(kCbPackPix, HW - p0);
-  const int64_t frame = (int64_t)blockIdx.z * N + n;
+  const int64_t frame = (int64_t)blockIdx.z * S + slot;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const T* s = src + frame * kCbC * HW + p0;
+  const T* s = src + ((int64_t)blockIdx.z * N + n) * kCbC * HW + p0;
   const int q = threadIdx.x & (kCbPackPix - 1), cq = threadIdx.x / kCbPackPix;
   bool bad = false;
   if (q < np) {
@@ -401,12 +433,12 @@ struct CbUnpack {
 template <typename T>
 __global__ void __launch_bounds__(256)
 corr_bwd_unpack_kernel(const __grid_constant__ CbUnpack U, T* __restrict__ dst,
-                       const unsigned char* __restrict__ flags, int N) {
+                       const int* __restrict__ slots, int N, int S) {
   __shared__ float tile[kCbPackPix][kCbC + 1];
-  const int n = blockIdx.y, W = U.W[0], HW = U.H[0] * W;
+  const int n = blockIdx.y, slot = slots ? slots[n] : n, W = U.W[0], HW = U.H[0] * W;
   const int p0 = blockIdx.x * kCbPackPix, np = min(kCbPackPix, HW - p0);
-  const int64_t frame = (int64_t)blockIdx.z * N + n;
-  const bool live = !flags || flags[n];
+  const int64_t frame = (int64_t)blockIdx.z * S + slot;
+  const bool live = slot >= 0;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll 2
   for (int q = warp; q < np; q += 8) {                        // a pixel's row by one warp, all levels' loads together
@@ -436,7 +468,7 @@ corr_bwd_unpack_kernel(const __grid_constant__ CbUnpack U, T* __restrict__ dst,
     for (int k = 0; k < 4; ++k) tile[q][lane + 32 * k] = v[k];
   }
   __syncthreads();
-  T* d = dst + frame * kCbC * HW + p0;
+  T* d = dst + ((int64_t)blockIdx.z * N + n) * kCbC * HW + p0;
   const int q = threadIdx.x & (kCbPackPix - 1), cq = threadIdx.x / kCbPackPix;
   if (q < np) {
 #pragma unroll 8
@@ -465,20 +497,20 @@ int cb_tile(const CbArgs& a, int b, cudaStream_t s) {
 size_t up256(size_t n) { return (n + 255) & ~(size_t)255; }
 
 template <typename T>
-int cb_pack(const void* src, float* dst, float* acc, const unsigned char* flags, int b, int n, int hw, int32_t* bad,
+int cb_pack(const void* src, float* dst, float* acc, const int* slots, int b, int n, int cap, int hw, int32_t* bad,
             cudaStream_t s) {
   HS2_PROF("corr_bwd_pack", s);
   corr_bwd_pack_kernel<T><<<dim3((hw + kCbPackPix - 1) / kCbPackPix, n, b), 256, 0, s>>>(static_cast<const T*>(src), dst,
-                                                                                       acc, flags, n, hw, bad);
+                                                                                       acc, slots, n, cap, hw, bad);
   HS2_LAUNCH_CHECK("corr_bwd_pack_kernel");
   return HS2_OK;
 }
 
 template <typename T>
-int cb_unpack(const CbUnpack& u, void* dst, const unsigned char* flags, int b, int n, cudaStream_t s) {
+int cb_unpack(const CbUnpack& u, void* dst, const int* slots, int b, int n, int cap, cudaStream_t s) {
   HS2_PROF("corr_bwd_unpack", s);
   corr_bwd_unpack_kernel<T><<<dim3((u.H[0] * u.W[0] + kCbPackPix - 1) / kCbPackPix, n, b), 256, 0, s>>>(
-      u, static_cast<T*>(dst), flags, n);
+      u, static_cast<T*>(dst), slots, n, cap);
   HS2_LAUNCH_CHECK("corr_bwd_unpack_kernel");
   return HS2_OK;
 }
@@ -487,21 +519,19 @@ template <typename T>
 int altcorr_bwd_tiled_t(const void* fmap1, const void* fmap2, int b, int n1, int n2, int h, int w, int h2, int w2,
                         const float* coords, const int64_t* ii, const int64_t* jj, int m, const float* grad,
                         int radius, float scale, void* g1, void* g2, int32_t* info, void* ws, cudaStream_t s) {
-  const size_t e1 = up256((size_t)b * n1 * h * w * kCbC * 4), e2 = up256((size_t)b * n2 * h2 * w2 * kCbC * 4);
+  const int s1 = std::min(n1, m), s2 = std::min(n2, m);
+  const size_t e1 = up256((size_t)b * s1 * h * w * kCbC * 4), e2 = up256((size_t)b * s2 * h2 * w2 * kCbC * 4);
   char* p = static_cast<char*>(ws);
   float *f1 = reinterpret_cast<float*>(p), *f2 = reinterpret_cast<float*>(p + e1);
   float *o1 = reinterpret_cast<float*>(p + e1 + e2), *o2 = reinterpret_cast<float*>(p + 2 * e1 + e2);
-  unsigned char* flags = reinterpret_cast<unsigned char*>(p + 2 * (e1 + e2));
-  const size_t nf = up256((size_t)n1 + n2) + 256;
-  int32_t* bad = reinterpret_cast<int32_t*>(flags + nf - 256);
-  HS2_CUDA(cudaMemsetAsync(flags, 0, nf, s));
-  corr_bwd_flag_kernel<<<(m + 255) / 256, 256, 0, s>>>(ii, m, n1, flags);
-  HS2_LAUNCH_CHECK("corr_bwd_flag_kernel");
-  corr_bwd_flag_kernel<<<(m + 255) / 256, 256, 0, s>>>(jj, m, n2, flags + n1);
-  HS2_LAUNCH_CHECK("corr_bwd_flag_kernel");
+  int32_t* bad = reinterpret_cast<int32_t*>(p + 2 * (e1 + e2));
+  int *slot1 = bad + 1, *slot2 = slot1 + n1;
+  HS2_CUDA(cudaMemsetAsync(bad, 0, sizeof(int32_t), s));
+  corr_bwd_slots_kernel<<<2, 1024, 0, s>>>(ii, jj, m, n1, n2, slot1, slot2);
+  HS2_LAUNCH_CHECK("corr_bwd_slots_kernel");
   int rc;
-  if ((rc = cb_pack<T>(fmap1, f1, o1, flags, b, n1, h * w, bad, s))) return rc;
-  if ((rc = cb_pack<T>(fmap2, f2, o2, flags + n1, b, n2, h2 * w2, bad, s))) return rc;
+  if ((rc = cb_pack<T>(fmap1, f1, o1, slot1, b, n1, s1, h * w, bad, s))) return rc;
+  if ((rc = cb_pack<T>(fmap2, f2, o2, slot2, b, n2, s2, h2 * w2, bad, s))) return rc;
   CbArgs a{};
   a.f1 = f1;
   a.f2[0] = f2;
@@ -511,6 +541,7 @@ int altcorr_bwd_tiled_t(const void* fmap1, const void* fmap2, int b, int n1, int
   a.grad = grad;
   a.ii = ii;
   a.jj = jj;
+  a.slot1 = slot1, a.slot2 = slot2, a.S1 = s1, a.S2 = s2;
   a.N1 = n1, a.N2 = n2, a.M = m, a.H = h, a.W = w, a.r = radius, a.levels = 1, a.cap = cb_cap(radius);
   a.H2[0] = h2, a.W2[0] = w2;
   a.scale = scale;
@@ -520,9 +551,9 @@ int altcorr_bwd_tiled_t(const void* fmap1, const void* fmap2, int b, int n1, int
   CbUnpack u{};
   u.levels = 1;
   u.acc[0] = o1, u.H[0] = h, u.W[0] = w;
-  if ((rc = cb_unpack<T>(u, g1, flags, b, n1, s))) return rc;
+  if ((rc = cb_unpack<T>(u, g1, slot1, b, n1, s1, s))) return rc;
   u.acc[0] = o2, u.H[0] = h2, u.W[0] = w2;
-  return cb_unpack<T>(u, g2, flags + n1, b, n2, s);
+  return cb_unpack<T>(u, g2, slot2, b, n2, s2, s);
 }
 
 // Workspace of the lookup's backward: packed fmap1 and its accumulator, then per level the packed
@@ -554,8 +585,8 @@ int corr_lookup_bwd_t(const void* fmap1, const void* fmap2, int n, int h, int w,
   int32_t* bad = reinterpret_cast<int32_t*>(ws + L.flag);
   HS2_CUDA(cudaMemsetAsync(bad, 0, sizeof(int32_t), s));
   int rc;
-  if ((rc = cb_pack<T>(fmap1, at(L.f1), nullptr, nullptr, 1, n, h * w, bad, s))) return rc;
-  if ((rc = cb_pack<T>(fmap2, at(L.f2[0]), at(L.o2[0]), nullptr, 1, n, h * w, bad, s))) return rc;
+  if ((rc = cb_pack<T>(fmap1, at(L.f1), nullptr, nullptr, 1, n, n, h * w, bad, s))) return rc;
+  if ((rc = cb_pack<T>(fmap2, at(L.f2[0]), at(L.o2[0]), nullptr, 1, n, n, h * w, bad, s))) return rc;
   for (int l = 1; l < levels; ++l) {
     const int64_t total = (int64_t)n * (h >> l) * (w >> l);
     HS2_PROF("corr_bwd_pool", s);
@@ -569,7 +600,7 @@ int corr_lookup_bwd_t(const void* fmap1, const void* fmap2, int n, int h, int w,
   a.coords = coords;
   a.interleaved = 1;
   a.grad = grad;
-  a.N1 = a.N2 = a.M = n, a.H = h, a.W = w, a.r = radius, a.levels = levels, a.cap = cb_cap(radius);
+  a.N1 = a.N2 = a.S1 = a.S2 = a.M = n, a.H = h, a.W = w, a.r = radius, a.levels = levels, a.cap = cb_cap(radius);
   a.scale = scale;
   a.nonfinite = bad;
   CbUnpack u{};
@@ -582,10 +613,10 @@ int corr_lookup_bwd_t(const void* fmap1, const void* fmap2, int n, int h, int w,
     u.acc[l] = at(L.o2[l]);
   }
   if ((rc = cb_tile<T, false>(a, 1, s))) return rc;
-  if ((rc = cb_unpack<T>(u, g2, nullptr, 1, n, s))) return rc;
+  if ((rc = cb_unpack<T>(u, g2, nullptr, 1, n, n, s))) return rc;
   u.levels = 1;
   u.acc[0] = at(L.o1);
-  return cb_unpack<T>(u, g1, nullptr, 1, n, s);
+  return cb_unpack<T>(u, g1, nullptr, 1, n, n, s);
 }
 
 int cl_check(int dtype, int n, int c, int h, int w, int levels, int radius) {
@@ -608,9 +639,10 @@ bool altcorr_bwd_tiled_ok(int b, int n1, int n2, int c, int m, int radius) {
   return c == kCbC && radius <= kCbMaxRadius && b > 0 && n1 > 0 && n2 > 0 && n1 <= 65535 && n2 <= 65535 && m > 0;
 }
 
-size_t altcorr_bwd_tiled_bytes(int b, int n1, int n2, int h, int w, int h2, int w2) {
-  return 2 * (up256((size_t)b * n1 * h * w * kCbC * 4) + up256((size_t)b * n2 * h2 * w2 * kCbC * 4)) +
-         up256((size_t)n1 + n2) + 256;
+size_t altcorr_bwd_tiled_bytes(int b, int n1, int n2, int h, int w, int h2, int w2, int m) {
+  return 2 * (up256((size_t)b * std::min(n1, m) * h * w * kCbC * 4) +
+              up256((size_t)b * std::min(n2, m) * h2 * w2 * kCbC * 4)) +
+         up256(((size_t)n1 + n2 + 1) * sizeof(int32_t));
 }
 
 int altcorr_bwd_tiled(int dtype, const void* fmap1, const void* fmap2, int b, int n1, int n2, int h, int w, int h2,

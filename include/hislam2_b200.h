@@ -266,8 +266,9 @@ int hs2_altcorr_levels_packed(const void* packed1, const void* const* packed_lev
  *   -> fmap1_grad [b,n1,c,h,w], fmap2_grad [b,n2,c,h2,w2] of `dtype`, fully written.
  *   `scale` multiplies every product: 1 reproduces the reference operator (which
  *   leaves out the forward's 1/16), 1/16 gives the exact adjoint of the forward.
- *   workspace: hs2_altcorr_backward_workspace_size() bytes (channel-last f32 features and
- *   accumulators of the tiled kernel for c == 128).  With fewer bytes, down to the f32
+ *   workspace: hs2_altcorr_backward_call_workspace_size() bytes for a call of m edges at a
+ *   radius, hs2_altcorr_backward_workspace_size() for any (channel-last f32 features and
+ *   accumulators of the tiled kernel for c == 128, radius <= 6).  With fewer bytes, down to the f32
  *   accumulators alone (none when dtype is f32), or when it does not start on a 16-byte
  *   boundary, the pixel-by-pixel kernel runs instead.
  */
