@@ -274,6 +274,8 @@ int hs2_altcorr_levels_packed(const void* packed1, const void* const* packed_lev
  */
 int hs2_altcorr_backward_workspace_size(int dtype, int b, int n1, int n2, int c, int h, int w, int h2,
                                         int w2, size_t* bytes);
+int hs2_altcorr_backward_call_workspace_size(int dtype, int b, int n1, int n2, int c, int h, int w, int h2,
+                                             int w2, int m, int radius, size_t* bytes);
 int hs2_altcorr_backward(const void* fmap1, const void* fmap2, int dtype, int b, int n1, int n2, int c,
                          int h, int w, int h2, int w2, const float* coords, const int64_t* ii,
                          const int64_t* jj, int m, const float* grad, int radius, float scale,
