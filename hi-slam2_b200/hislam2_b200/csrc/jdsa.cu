@@ -13,7 +13,9 @@
 //
 //   jdsa_keys          kx and slot of the edges from a bitmap of the frames, one CTA: a list of a
 //                      few hundred edges needs no sort, and the count stays on the device;
-//   jdsa_step          cluster of 8 CTAs per block b, pixels dealt out in runs of a CTA: per
+//   proj_trans         (geometry.cu) windows of more than kJdFusedBlocks source frames: the depth-only
+//                      Schur terms C, w, edge by edge with atomics, ahead of a jdsa_step that reads them;
+//   jdsa_step          cluster of 8 (after proj_trans: 2) CTAs per block b, pixels dealt out in runs of a CTA: per
 //                      pixel the depth-only Schur terms C, w summed over the block's edges in
 //                      their order (proj_trans's terms, geometry.cu); then, in FP32 as the
 //                      reference,
@@ -52,7 +54,14 @@ namespace {
 
 constexpr int kJdThreads = 256;
 constexpr int kJdWarps = kJdThreads / 32;
-constexpr int kJdCluster = 8;      // CTAs of one block: the portable cluster size
+// Up to kJdFusedBlocks source frames (two waves of their CTAs) a cluster of eight CTAs sums its block's
+// edges itself.  Each of its CTAs looks through the whole edge list, so beyond that proj_trans
+// sums them, a CTA per edge, and two CTAs a block have work enough for the GPU.  A call, the edges summed
+// by the cluster / ahead: 60 frames of 43x77 with 700 edges 140 / 146 us, 100 with 2000 234 / 181, 300
+// with 6000 546 / 333, 1000 of 24x32 with 20000 2030 / 335; 150 of 120x160 with 2000 575 / 504.
+constexpr int kJdCluster = 8;      // the portable cluster size
+constexpr int kJdPlainCluster = 2;
+constexpr int kJdFusedBlocks = 2 * 2 * kNumSMs / kJdCluster;
 constexpr int kJdBatch = 64;       // edges whose relative poses are in shared memory at a time
 constexpr int kJdMaxD = 16;
 constexpr int kJdMaxCells = 9;     // (hs - 1)(ws - 1) for hs ws <= 16
@@ -328,7 +337,9 @@ __device__ __forceinline__ bool warp_solve(int D, double (*S)[kJdMaxD + 1], cons
   return true;
 }
 
-__global__ void __cluster_dims__(kJdCluster, 1, 1) __launch_bounds__(kJdThreads, 2)
+// kRanks: CTAs of a block; kEdges: C and w are summed here, else they are read
+template <int kRanks, bool kEdges>
+__global__ void __cluster_dims__(kRanks, 1, 1) __launch_bounds__(kJdThreads, 2)
 jdsa_step_kernel(const JdArgs A) {
   extern __shared__ float jd_axes[];   // gy [ht] then gx [wd]
   __shared__ double red[kJdWarps][kJdSums];
@@ -340,19 +351,19 @@ jdsa_step_kernel(const JdArgs A) {
   __shared__ float dso[kJdMaxD];
   __shared__ float Si[kJdMaxD][kJdMaxD + 1];
   __shared__ float sc_r[kJdMaxD], sc_s[kJdMaxD];
-  __shared__ JdEdge edges[kJdBatch];
-  __shared__ int list[kJdBatch + kJdThreads];
+  __shared__ JdEdge edges[kEdges ? kJdBatch : 1];
+  __shared__ int list[kEdges ? kJdBatch + kJdThreads : 1];
   __shared__ int found[kJdWarps];
   __shared__ int bad, failed;
   const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
   const int HW = A.ht * A.wd, D = A.hs * A.ws, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int rank = (int)cluster.block_rank();
-  const int b = blockIdx.x / kJdCluster;
+  const int b = blockIdx.x / kRanks;
   // an equal run of pixels for each CTA, in whole warps
-  const int run = (HW / kJdCluster + 32) / 32 * 32, k0 = rank * run + tid, kend = min(HW, (rank + 1) * run);
+  const int run = (HW / kRanks + 32) / 32 * 32, k0 = rank * run + tid, kend = min(HW, (rank + 1) * run);
   if (b >= A.M) {
     // frames of the window that are not source frames: the where / clamp only
-    const int step = gridDim.x / kJdCluster - A.M;
+    const int step = gridDim.x / kRanks - A.M;
     for (int64_t f = b - A.M; f < A.num_disps; f += step) {
       if (find_sorted(A.kx, A.M, f) >= 0) continue;
       const float* src = A.disps + f * HW;
@@ -399,7 +410,7 @@ jdsa_step_kernel(const JdArgs A) {
   // ---- C and w of this thread's pixels: the edges of slot b in their order
   float* Cm = A.C + (int64_t)b * HW;
   float* wm = A.w + (int64_t)b * HW;
-  const int E = (int)A.num_edges;
+  const int E = kEdges ? (int)A.num_edges : 0;
   int num = 0;         // edges in `list`
   bool first = true;
   for (int base = 0; base < E; base += kJdThreads) {
@@ -429,7 +440,7 @@ jdsa_step_kernel(const JdArgs A) {
     }
     num = 0;
   }
-  if (first)
+  if (kEdges && first)
     for (int k = k0; k < kend; k += kJdThreads) Cm[k] = wm[k] = 0.f;
   __syncthreads();   // sc_r, sc_s
 
@@ -475,7 +486,7 @@ jdsa_step_kernel(const JdArgs A) {
   for (int i = tid; i < cells * kJdSums; i += kJdThreads) {
     double s = 0.0;
 #pragma unroll
-    for (int q = 0; q < kJdCluster; ++q) s += cluster.map_shared_rank(part, q)[i];
+    for (int q = 0; q < kRanks; ++q) s += cluster.map_shared_rank(part, q)[i];
     tot[i] = s;
   }
   auto read = cluster.barrier_arrive();   // waited for before this CTA's shared memory goes away
@@ -717,10 +728,18 @@ extern "C" int hs2_jdsa(const float* poses, int64_t num_poses, const float* disp
   A.dzcov = dzcov;
   A.info = info;
   const size_t smem = sizeof(float) * (size_t)(ht + wd);
+  const bool fused = num_kx <= kJdFusedBlocks;
+  if (!fused && (rc = hs2_proj_trans(poses, num_poses, disps, num_disps, ht, wd, intrinsics, targets, weights, ii, jj,
+                                     slot, num_edges, num_kx, C, w, info, stream)))
+    return rc;
   // every frame that is not a source frame is one of num_disps - M
   const unsigned copies = (unsigned)std::min<int64_t>(std::max<int64_t>(num_disps - num_kx, 0), kJdCopyClusters);
   HS2_PROF("jdsa_step", s);
-  jdsa_step_kernel<<<((unsigned)num_kx + copies) * kJdCluster, kJdThreads, smem, s>>>(A);
+  const unsigned clusters = (unsigned)num_kx + copies;
+  if (fused)
+    jdsa_step_kernel<kJdCluster, true><<<clusters * kJdCluster, kJdThreads, smem, s>>>(A);
+  else
+    jdsa_step_kernel<kJdPlainCluster, false><<<clusters * kJdPlainCluster, kJdThreads, smem, s>>>(A);
   HS2_LAUNCH_CHECK("jdsa_step_kernel");
   const int D = hs * ws;
   HS2_PROF("jdsa_scales", s);
