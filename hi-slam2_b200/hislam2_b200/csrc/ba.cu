@@ -915,6 +915,10 @@ ba_schur_tc_kernel(const __grid_constant__ CUtensorMap emap, int HW, int chunk, 
       pn = c0 + (c + kTcGroups) * kTcK + lane;
       qn = pn < c1 ? Q[pn] : 0.f;
       wn = pn < c1 ? Wv[pn] : 0.f;
+      // With an odd number of stages the groups take turns on a stage.  A barrier tells only the parity of
+      // its phase, so a group that came round before the other group's copy had landed would take the
+      // phase before that for its own: it first waits until the stage's last use has been multiplied.
+      if (nst % kTcGroups && use > 0 && !mbar_wait(bar_empty + 8 * st, (use - 1) & 1, abort_flag)) break;
       if (!mbar_wait(bar_tma + 8 * st, use & 1, abort_flag)) break;
       uint8_t* hi = gbase + st * stage_bytes;
       uint8_t* lo = hi + tile_bytes;
