@@ -438,30 +438,39 @@ corr_bwd_unpack_kernel(const __grid_constant__ CbUnpack U, T* __restrict__ dst,
   const int n = blockIdx.y, slot = slots ? slots[n] : n, W = U.W[0], HW = U.H[0] * W;
   const int p0 = blockIdx.x * kCbPackPix, np = min(kCbPackPix, HW - p0);
   const int64_t frame = (int64_t)blockIdx.z * S + slot;
-  const bool live = slot >= 0;
+  if (slot < 0) {
+    // no edge uses the frame: its share of the frame's zeros, by 16-byte stores where they are aligned
+    T* f = dst + ((int64_t)blockIdx.z * N + n) * kCbC * HW + (int64_t)blockIdx.x * kCbPackPix * kCbC;
+    const int count = np * kCbC;              // of 128 HW elements: the blocks' runs are equal but for the last
+    constexpr int kVec = 16 / sizeof(T);
+    if (reinterpret_cast<uintptr_t>(f) & 15) {
+      for (int i = threadIdx.x; i < count; i += 256) f[i] = from_f<T>(0.f);
+    } else {
+      for (int i = threadIdx.x; i < count / kVec; i += 256) reinterpret_cast<uint4*>(f)[i] = make_uint4(0, 0, 0, 0);
+    }
+    return;
+  }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll 2
   for (int q = warp; q < np; q += 8) {                        // a pixel's row by one warp, all levels' loads together
     float v[4] = {0.f, 0.f, 0.f, 0.f};
-    if (live) {
-      const int y = (p0 + q) / W, x = (p0 + q) - y * W;
-      float a[4][4];
+    const int y = (p0 + q) / W, x = (p0 + q) - y * W;
+    float a[4][4];
 #pragma unroll
-      for (int l = 0; l < 4; ++l) {
-        if (l < U.levels) {
-          const int yl = y >> l, xl = x >> l;
-          const bool in = yl < U.H[l] && xl < U.W[l];
-          const float* row = U.acc[l] + ((frame * U.H[l] + yl) * U.W[l] + xl) * kCbC + lane;
+    for (int l = 0; l < 4; ++l) {
+      if (l < U.levels) {
+        const int yl = y >> l, xl = x >> l;
+        const bool in = yl < U.H[l] && xl < U.W[l];
+        const float* row = U.acc[l] + ((frame * U.H[l] + yl) * U.W[l] + xl) * kCbC + lane;
 #pragma unroll
-          for (int k = 0; k < 4; ++k) a[l][k] = in ? row[32 * k] : 0.f;
-        }
+        for (int k = 0; k < 4; ++k) a[l][k] = in ? row[32 * k] : 0.f;
       }
+    }
 #pragma unroll
-      for (int l = 3; l >= 0; --l) {
-        if (l < U.levels) {
+    for (int l = 3; l >= 0; --l) {
+      if (l < U.levels) {
 #pragma unroll
-          for (int k = 0; k < 4; ++k) v[k] = (v[k] + a[l][k]) * (l > 0 ? 0.25f : 1.f);
-        }
+        for (int k = 0; k < 4; ++k) v[k] = (v[k] + a[l][k]) * (l > 0 ? 0.25f : 1.f);
       }
     }
 #pragma unroll
