@@ -3225,10 +3225,6 @@ extern "C" int hs2_ba_adjoint(const float* poses, int64_t num_poses, const float
   return HS2_OK;
 }
 
-namespace hs2 {
-
-}  // namespace hs2
-
 // ================================================================= pgba ===
 // Sim3 pose-graph bundle adjustment (reference operator: src/droid.cpp:171-196 ->
 // src/droid_kernels.cu:1940-2044): ONE damped Gauss-Newton step over Sim3 poses

@@ -1,5 +1,5 @@
 // Workspace layout of the dense BA (one window) and the per-pixel linearisation,
-// shared by the single-window kernels (ba.cu) and the batched ones (ba_batch.cu).
+// shared by the single-window kernels (ba.cu) and the batched ones (ba_batch.cuh).
 #pragma once
 
 #include <algorithm>
@@ -159,14 +159,5 @@ __device__ __forceinline__ void lin_pixel(const float* __restrict__ tab, float f
 #pragma unroll
   for (int r = 2; r < 6; ++r) Ej[r] = fmaf(zu, Ju[r], zv * Jv[r]);
 }
-
-
-// Keys of one window (ba.cu): depth slots, edge groups by source frame, E-row lists.
-__global__ void ba_keys_kernel(const int64_t* __restrict__ ii, const int64_t* __restrict__ jj, int E, int K, int t0,
-                               int t1, int64_t eta_rows, BaPtrs w, int32_t* __restrict__ info);
-// Per-edge table of one window (ba.cu): Gij, its rotation matrix, the map L (Ji = L Jj).
-__global__ void ba_edge_setup_kernel(const float* __restrict__ poses, const int64_t* __restrict__ ii,
-                                     const int64_t* __restrict__ jj, int E, float* __restrict__ etab,
-                                     double* __restrict__ etab64, const int32_t* __restrict__ info);
 
 }  // namespace hs2
