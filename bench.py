@@ -1047,7 +1047,7 @@ def profile_batch(args, dev):
 
 def profile_altcorr(args, dev):
     """AltCorrBlock (float16, radius 3, 4 levels, pyramid packed channel-last) on the
-    first --profile-edges edges of the 300-keyframe window: 4 altcorr_fwd_packed launches."""
+    first --profile-edges edges of the 300-keyframe window: one altcorr_fwd_tile launch."""
     from hislam2_b200 import synth
     from hislam2_b200.corr import AltCorrBlock
     p = synth.make_ba_problem(WORKLOAD, seed=0)

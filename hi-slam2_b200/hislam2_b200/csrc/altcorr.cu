@@ -965,8 +965,9 @@ extern "C" int hs2_altcorr_backward(const void* fmap1, const void* fmap2, int dt
   if ((rc = bind_device(fmap1_grad))) return rc;
   cudaStream_t s = (cudaStream_t)stream;
   // 128 channels: gradients by tiles (corr_backward.cu), unless the caller brought only the
-  // accumulators' workspace or one that does not start on 16 bytes (the tiles' vectors).  84 edges at 48x64, radius 4, four FP32
-  // levels: 3.5 ms (2.6 tiles, 0.9 packing, since then less than half) against 27.3 ms pixel by pixel.
+  // accumulators' workspace or one that does not start on 16 bytes (the tiles' vectors).  84 edges at
+  // 48x64, radius 4, four FP32 levels, a call each: 3.4 ms (2.6 tiles, 0.4 packing, 0.4 unpacking)
+  // against 25.8 ms pixel by pixel.
   if ((dtype == HS2_F32 || dtype == HS2_F16 || dtype == HS2_BF16) && altcorr_bwd_tiled_ok(b, n1, n2, c, m, radius) &&
       workspace && !(reinterpret_cast<uintptr_t>(workspace) & 15) &&
       workspace_bytes >= altcorr_bwd_tiled_bytes(b, n1, n2, h, w, h2, w2, m))

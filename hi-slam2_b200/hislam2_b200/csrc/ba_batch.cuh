@@ -275,9 +275,9 @@ __device__ void batch_cholesky_blocked(int n, float lm, float ep, BaPtrs w, floa
 // entry leaves the CTA.
 // The general ba_schur body (22-block tiles, one thread per 6x6 block) leaves two thirds
 // of a CTA idle on frames of 5 to 14 blocks, stages 132 rows whatever the frame holds and
-// waits for every stage: 420 us per unit against 55 to 70 us here (64 windows of 8 to 40
-// keyframes, two units per frame, two CTAs per SM; one LM iteration 6.4 ms against 2.26 ms, 1.90 since
-// the back-substitution's rows are listed and read as vectors).
+// waits for every stage: 420 us per unit against 74 here (64 windows of 8 to 40 keyframes, two units
+// per frame, two CTAs per SM: 0.83 ms of Gram in a CTA's 11 units of an LM iteration, which
+// takes 1.95 ms, 6.4 with the general body).
 constexpr int kGramRows = 256;        // rows with w's: 42 blocks
 constexpr int kGramTiles = (kGramRows / 8) * (kGramRows / 8 + 1) / 2;
 constexpr int kGramStages = 4;

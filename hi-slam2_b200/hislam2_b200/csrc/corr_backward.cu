@@ -6,8 +6,9 @@
 // Both are 128-long axpys; a pixel-by-pixel kernel re-reads f2 for every pixel and sends
 // every (pixel, tap) product to memory as an atomic.  Here a CTA owns an 8x8 tile, as 16
 // groups of 2x2 pixels:
-//   * features and gradients are channel-last in FP32 (corr_bwd_pack), so one position is
-//     one 512-byte row and a warp holds it as one float4 per lane;
+//   * features and gradients are channel-last in FP32 (corr_bwd_pack; only frames that an edge
+//     uses have a place, so the workspace follows the edges), so one position is one 512-byte row
+//     and a warp holds it as one float4 per lane;
 //   * the window gradients of a group are laid out over the union of its four windows, one
 //     float4 (four pixels) per position, so one shared-memory broadcast feeds 16 FMAs;
 //   * g1: one warp per group walks the union, reading each f2 row once for four pixels;

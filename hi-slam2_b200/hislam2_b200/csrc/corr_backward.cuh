@@ -6,7 +6,7 @@
 
 namespace hs2 {
 
-// The tile kernel covers 128 channels and radius <= 6 (177 KB of shared memory at 6).
+// The tile kernel covers 128 channels and radius <= 6 (142 KB of shared memory at 6).
 constexpr int kCbMaxRadius = 6;
 
 bool altcorr_bwd_tiled_ok(int b, int n1, int n2, int c, int m, int radius);

@@ -15,10 +15,9 @@
 //                      few hundred edges needs no sort, and the count stays on the device;
 //   proj_trans         (geometry.cu) windows of more than kJdFusedBlocks source frames: the depth-only
 //                      Schur terms C, w, edge by edge with atomics, ahead of a jdsa_step that reads them;
-//   jdsa_step          cluster of 8 (after proj_trans: 2) CTAs per block b, pixels dealt out in runs of a CTA: per
-//                      pixel the depth-only Schur terms C, w summed over the block's edges in
-//                      their order (proj_trans's terms, geometry.cu); then, in FP32 as the
-//                      reference,
+//   jdsa_step          cluster of 8 (after proj_trans: 2) CTAs per block b, pixels dealt out in runs of
+//                      a CTA: per pixel the depth-only Schur terms C, w summed over the block's
+//                      edges in their order (proj_trans's terms); then, in FP32 as the reference,
 //                        Q = 1 / (C + m alpha + (1 - m) eta),  w' = w - m alpha rd,
 //                        a = prior [> 0] of the source frame, J = -a (wa, wb, wc, wd) at the
 //                        pixel's interpolation cell,
@@ -38,8 +37,8 @@
 // 13 pixels a thread through two passes behind a launch of atomics that summed C and w; eight
 // CTAs a frame take two pixels a thread, keep the sums of an edge list they scan themselves
 // (no zeroed buffers, no atomics, a fixed order) and meet once, in distributed shared memory.
-// 25 frames at 43x77, 258 edges, 2x2 grid: a call of mono.JDSA 183 -> 118 us (most of it the
-// keys, which torch.unique made behind two waits of the host; the kernels 61 -> 54 us), of
+// 25 frames at 43x77, 258 edges, 2x2 grid: a call of mono.JDSA 183 -> 121 us (most of it the
+// keys, which torch.unique made behind two waits of the host; the kernels 61 -> 53 us), of
 // which the host's own work is half.
 #include <utility>
 

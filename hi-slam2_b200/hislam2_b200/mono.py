@@ -84,7 +84,7 @@ def JDSA(target, weight, eta, poses, disps, intrinsics, disps_prior, dscales, ii
     info = torch.empty(2, dtype=torch.int32, device=dev)
     if on_device:
         # eta says how many source frames there are, so their keys need no answer from the device
-        # (torch.unique sorts, and waits for the count: 183 us a call with it, 118 without)
+        # (torch.unique sorts, and waits for the count: 183 us a call with it, 121 without)
         keys = torch.empty(M + E, dtype=torch.int64, device=dev)
         kx, slot = keys[:M], keys[M:]
         _lib.check(lib.hs2_jdsa_keys(_ptr(ii), E, P, M, _ptr(kx), _ptr(slot), _ptr(info[1:]), _stream(dev)),
