@@ -72,7 +72,7 @@ int hs2_corr_index_forward(const void* volume, int dtype, int64_t n, int h1, int
 /* corr_pyramid_forward  (reference: hislam2/modules/corr.py:40-51, CorrBlock's lookup)
  *   corr_index_forward of every pyramid level at coords / 2^level in one launch:
  *   volumes[l] [n,h1,w1,h1>>l,w1>>l] of `dtype` (f32, f16, bf16) for 1 to 4 levels,
- *   coords [n,h1,w1,2] f32 (x, y), radius 3 or 4
+ *   coords [n,h1,w1,2] f32 (x, y), radius 3 or 4, n <= 65535, h1*w1 <= 2^24
  *   -> corr [n, levels*(2r+1)^2, h1, w1], the levels' channels one after the other.
  */
 int hs2_corr_pyramid_forward(const void* const* volumes, int levels, int dtype, int64_t n, int h1, int w1,
@@ -146,7 +146,7 @@ int hs2_ba_batch_set_wait_test(unsigned spin_limit, int unsatisfiable);
  *   [t1-t0,6] receives the adjoint pose solution.  All outputs are fully written.
  *   info as for hs2_ba, plus HS2_DEV_LIMIT when a depth frame has more than 256
  *   optimised rows or an edge pose more than 8 duplicate rows in one frame.
- *   Workspace: hs2_ba_adjoint_workspace_size() bytes.
+ *   Workspace: hs2_ba_adjoint_workspace_size() bytes, 256-byte aligned.
  */
 int hs2_ba_adjoint_workspace_size(int64_t num_poses, int64_t num_disps, int ht, int wd, int64_t num_edges, int t0,
                                   int t1, size_t* bytes);
@@ -175,7 +175,8 @@ int hs2_ba_adjoint(const float* poses, int64_t num_poses, const float* disps, in
  *   info: int32[1] on the device; info[0] |= HS2_DEV_BAD_INDEX for a pair whose frame
  *   index is outside [0, k1) / [0, k2) (its outputs are left unwritten),
  *   HS2_DEV_TIMEOUT if a bounded wait gave up.
- *   Workspace: hs2_corr_volume_workspace_size() bytes (the packed operands).
+ *   Workspace: hs2_corr_volume_workspace_size() bytes (the packed operands), on a 16-byte
+ *   boundary.
  */
 enum hs2_corr_precision { HS2_CV_NATIVE = 0, HS2_CV_E4M3 = 1 };
 int hs2_corr_volume_workspace_size(int64_t k1, int64_t k2, int channels, int ht, int wd, int dtype, int precision,
@@ -233,8 +234,8 @@ int hs2_altcorr_forward(const void* fmap1, const void* fmap2, int dtype, int b, 
 
 /* altcorr_forward on channel-last features (same reference op; float16 / bfloat16 with
  * c in {32, 64, 128, 256}).  hs2_altcorr_pack writes fmap [b,n,c,h,w] channel-last,
- * [b,n,h*w,c], into the start of `workspace` (hs2_altcorr_pack_workspace_size() bytes,
- * a frame-flag array at its end): only the frames listed in `frames[num_frames]` (the
+ * [b,n,h*w,c], into the start of `workspace` (hs2_altcorr_pack_workspace_size() bytes on a
+ * 16-byte boundary, a frame-flag array at its end): only the frames listed in `frames[num_frames]` (the
  * ii or jj of a call), or all n frames when `frames` is null.  hs2_altcorr_forward_packed
  * then takes two such buffers in place of fmap1 / fmap2 and writes the same corr as
  * hs2_altcorr_forward: products of the 16-bit features formed exactly and summed in
